@@ -1,5 +1,5 @@
-"""The workloads this library is timed on, each a call (or a frame of calls)
-a user's program makes through a public entry point.
+"""The workloads this library is timed on, each a call a user's program makes
+through a public entry point.
 
 * ``apply``   esf_pressure_apply: the pressure operator alone, as a caller
               that runs its own Krylov loop uses it, one product a pass.
@@ -8,10 +8,9 @@ a user's program makes through a public entry point.
               solver benchmark sets it) or to the 1e-8 residual.
 * ``static``  esf_pressure_solve_static: the allocation-free FP64 solve.
 * ``batch``   esf_pressure_solve_batch: many independent systems at once.
-* ``frame``   a frame of coupled steps (1/60 s at dt = 1/240) of the rubber
-              ball at the reference's shipped solver settings (tolerance
-              0.02, at most 500 iterations), and the fields a program reads
-              after it.
+* ``step``    one coupled step (dt = 1/240) of the rubber ball at the
+              reference's shipped solver settings (tolerance 0.02, at most
+              500 iterations), and the fields a program reads after it.
 * ``bake``    esf_rasterize_solid: a solid's rest mass from its mesh.
 
 Sizes are cells per axis. Inputs come from the seed alone.
@@ -56,9 +55,9 @@ def listed():
         # small independent systems in one call
         {"name": "batch_32x64", "kind": "batch", "nx": 32, "ny": 32, "nz": 32, "systems": 64, "iters": 100,
          "eps": 1e-30},
-        # frames of the coupled step, in each precision
-        {"name": "frame_fp64_64", "kind": "frame", "n": 64, "precision": "fp64"},
-        {"name": "frame_mixed_128", "kind": "frame", "n": 128, "precision": "mixed"},
+        # the coupled step, in each precision
+        {"name": "step_fp64_64", "kind": "step", "n": 64, "precision": "fp64"},
+        {"name": "step_mixed_128", "kind": "step", "n": 128, "precision": "mixed"},
         # the shipped sphere's resolution: a spacing of a hundredth of the radius
         {"name": "bake_100", "kind": "bake", "level": 3, "per_radius": 100},
     ]
@@ -69,8 +68,8 @@ def _log_int(rng, lo, hi):
 
 
 def draw(rng):
-    kind = rng.choice(["apply", "apply", "solve", "solve", "solve", "static", "batch", "frame", "bake"])
-    if kind == "frame":
+    kind = rng.choice(["apply", "apply", "solve", "solve", "solve", "static", "batch", "step", "bake"])
+    if kind == "step":
         return {"kind": kind, "n": _log_int(rng, 24, 96), "precision": rng.choice(["fp64", "mixed", "x64"])}
     if kind == "bake":
         return {"kind": kind, "level": rng.choice([2, 3]), "per_radius": _log_int(rng, 20, 80)}
@@ -168,7 +167,7 @@ def _scene(case, seed):
 def prepare(case, seed):
     kind = case["kind"]
     lib = E.load(build_if_missing=True)
-    if kind == "frame":
+    if kind == "step":
         return {"case": case, "integrator": E.make_scene(_scene(case, seed), precision=PRECISION[case["precision"]])}
     if kind == "bake":
         verts, faces = _mesh(case, seed)
@@ -206,12 +205,12 @@ def _check(status, what):
 
 def run(state):
     case, kind = state["case"], state["case"]["kind"]
-    if kind == "frame":
+    if kind == "step":
         scene = state["integrator"]
-        reports = E.run_frames(scene, 1, 1.0 / 60.0)
+        report = scene.stepImplicit()
         return {"velocity": scene.get("velocity"), "pressure": scene.get("lambda1"),
                 "mesh": scene.get("solid.meshVertices"),
-                "iterations": [i for r in reports for i in r["iterations"]][:12]}
+                "iterations": report["iterations"]}
     if kind == "bake":
         res, dh, origin, mass, total = rasterize_solid(state["verts"], state["faces"],
                                                        0.1 / case["per_radius"], 1000.0)
@@ -246,14 +245,14 @@ def run(state):
 # vector is read and written once: r, t, q, d and x in and out, 1/diag and 1/m
 # in; and the arithmetic of one operator product with the vector updates.
 ITERATION_WORDS, ITERATION_FLOPS, PRODUCT_FLOPS = 12, 54, 36
-FRAME_WORDS = 60  # node fields the step reads and writes once each (FP64)
+STEP_WORDS = 60  # node fields the step reads and writes once each (FP64)
 
 
 def work(case):
     kind = case["kind"]
-    if kind == "frame":
+    if kind == "step":
         nodes = (case["n"] + 1) ** 3
-        return {"bytes": 4 * FRAME_WORDS * 8 * nodes, "flops": 4 * 400 * nodes}
+        return {"bytes": STEP_WORDS * 8 * nodes, "flops": 400 * nodes}
     if kind == "bake":
         nodes = (2.0 * case["per_radius"] + 20) ** 3
         return {"bytes": 8 * nodes, "flops": 0}
@@ -339,7 +338,7 @@ def _bake_mass(case, seed):
 
 def exact(case, seed):
     kind = case["kind"]
-    if kind == "frame":  # a whole engine: no 64-bit value apart from its own
+    if kind == "step":  # a whole engine: no 64-bit value apart from its own
         return None
     if kind == "bake":
         return _bake_mass(case, seed)
