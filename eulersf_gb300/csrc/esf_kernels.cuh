@@ -339,295 +339,7 @@ __global__ void __launch_bounds__(256) k_phi_init(GridDev g, SolidDev s, double 
   }
 }
 
-// solveDistance (DEFOR_SOLID_3D.cpp:369-394)
-__device__ __forceinline__ void solve_distance(double p, double q, double r, double* v) {
-  // std::min / std::max semantics: (b < a) ? b : a
-  double ds[3];
-  double mqr = (r < q) ? r : q, Mqr = (q < r) ? r : q;
-  ds[0] = (mqr < p) ? mqr : p;
-  ds[2] = (p < Mqr) ? Mqr : p;
-  ds[1] = p + q + r - ds[0] - ds[2];
-  double b[3], c[3];
-  b[0] = ds[0];
-  c[0] = ds[0] * ds[0] - 1.0f;
-  for (int x = 1; x < 3; x++) {
-    b[x] = ds[x] + b[x - 1];
-    c[x] = ds[x] * ds[x] + c[x - 1];
-  }
-  int i = 2;
-  double discrim = b[i] * b[i] - (double)(i + 1) * c[i];
-  double nd = (b[i] + sqrt(discrim)) / (double)(i + 1);
-  while ((discrim < 0.0f || nd < ds[i]) && i != -1) {
-    i--;
-    if (i < 0) break;
-    discrim = b[i] * b[i] - (double)(i + 1) * c[i];
-    if (discrim > 0.0f) nd = (b[i] + sqrt(discrim)) / (double)(i + 1);
-  }
-  if (nd < *v) *v = nd;
-}
-
-// A Gauss-Seidel sweep pass (sweepPhi, sweepOnePass): node (i,j,k) reads
-// its three upwind neighbours as updated in the same pass, so every order in
-// which each node comes after its three upwind neighbours gives the
-// sequential loop's result bit for bit. The pass runs as a wavefront of
-// tiles (k_sweep_tile below).
-struct Sweep {
-  int i0, j0, k0;   // first index in sweep order
-  int di, dj, dk;   // +1 / -1
-  int ni, nj, nk;   // counts
-};
-
-// ---------------------------------------------- velocity extension (a19)
-// DEFOR_SOLID_3D::sweepOnePass (DEFOR_SOLID_3D.cpp:457-519). Its
-// solvableX/Y/Z flags live for the whole pass and, once cleared, stay
-// cleared: a node sees a flag cleared iff some node at or before it in loop
-// order triggered it. Triggers depend on phi and mass only (constant during
-// the pass), so the first trigger rank of each flag is found by a min
-// reduction before the wavefront runs.
-
-// First trigger rank of the three pass-long flags of sweepOnePass, by
-// atomicMin over all nodes of the pass (ranks: long long loop order).
-__global__ void k_sweep_vec_ranks(GridDev g, const double* ph, const double* ms, Sweep w,
-                                  unsigned long long* ranks) {
-  __shared__ unsigned long long sm[3];
-  if (threadIdx.x < 3) sm[threadIdx.x] = ~0ull;
-  __syncthreads();
-  unsigned long long r0 = ~0ull, r1 = ~0ull, r2 = ~0ull;
-  const long long nij = (long long)w.ni * w.nj, total = nij * w.nk;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    int a = (int)(t % w.ni), b = (int)((t / w.ni) % w.nj), c = (int)(t / nij);
-    int i = w.i0 + a * w.di, j = w.j0 + b * w.dj, k = w.k0 + c * w.dk;
-    long long n = nidx(g, i, j, k);
-    if (ms[n] != 0) continue;
-    double pn = ph[n];
-    double dp = pn - ph[nidx(g, i - w.di, j, k)], dpn = pn - ph[nidx(g, i + w.di, j, k)];
-    if (dp < 0 && dpn >= 0) continue;
-    if (dp < 0 && dpn < 0 && (unsigned long long)t < r0) r0 = t;
-    double dq = pn - ph[nidx(g, i, j - w.dj, k)], dqn = pn - ph[nidx(g, i, j + w.dj, k)];
-    if (dq < 0 && dqn >= 0) continue;
-    if (dq < 0 && dqn < 0 && (unsigned long long)t < r1) r1 = t;
-    double dr = pn - ph[nidx(g, i, j, k - w.dk)], drn = pn - ph[nidx(g, i, j, k + w.dk)];
-    if (dr < 0 && drn >= 0) continue;
-    if (dr < 0 && drn < 0 && (unsigned long long)t < r2) r2 = t;
-  }
-  // one shared-memory and one global atomic per block and flag
-  if (r0 != ~0ull) atomicMin(&sm[0], r0);
-  if (r1 != ~0ull) atomicMin(&sm[1], r1);
-  if (r2 != ~0ull) atomicMin(&sm[2], r2);
-  __syncthreads();
-  if (threadIdx.x < 3 && sm[threadIdx.x] != ~0ull) atomicMin(&ranks[threadIdx.x], sm[threadIdx.x]);
-}
-// One launch of a sweep pass as a tile wavefront: the pass's nodes in
-// sweep coordinates (a, b, c) are cut into ST^3 tiles, and launch P runs
-// every tile (I, J, K) with I + J + K = P, whose three upwind tiles ran in
-// launch P - 1. A block copies its tile and the upwind layer of each axis
-// into shared memory, settles for each of its nodes what does not change
-// during the pass (all nodes at once), sweeps the tile's sub-planes
-// a'+b'+c' = q in order in shared memory (a barrier between sub-planes), and
-// writes the tile back. PHI: the distance update of sweepPhi
-// (DEFOR_SOLID_3D.cpp:397-455) on phi, for nodes without solid mass. VEC:
-// the sweepOnePass update (DEFOR_SOLID_3D.cpp:457-519) of the three velocity
-// components; its skip tests and blend weights depend on phi, the mass and
-// the pass-long flags (resolved from the ranks of k_sweep_vec_ranks) only,
-// none of which change during the pass, so they are formed up front.
-constexpr int ST = 8;           // tile edge
-constexpr int SP = ST + 1;      // tile plus the upwind layer
-constexpr int SWEEP_THREADS = 128;  // blocks of the wave kernel
-constexpr int TILE_THREADS = ST * ST * ST;  // one thread per node of a tile
-static_assert(ST * ST <= TILE_THREADS, "one thread per (a', b') of a tile");
-template <bool VEC>
-__global__ void __launch_bounds__(TILE_THREADS) k_sweep_tile(GridDev g, double* f, double* ph,
-                                                              const double* ms, Sweep w, int P,
-                                                              const unsigned long long* ranks) {
-  constexpr int NC = VEC ? 3 : 1;
-  __shared__ double sv[NC * SP * SP * SP];
-  __shared__ double sAlpha[VEC ? ST * ST * ST : 1], sBeta[VEC ? ST * ST * ST : 1];
-  __shared__ unsigned char sUpd[ST * ST * ST];
-  const int nti = (w.ni + ST - 1) / ST, ntj = (w.nj + ST - 1) / ST, ntk = (w.nk + ST - 1) / ST;
-  const int I = blockIdx.x % nti, J = blockIdx.x / nti, K = P - I - J;
-  if (J >= ntj || K < 0 || K >= ntk) return;
-  const int a0 = I * ST, b0 = J * ST, c0 = K * ST;
-  const int na = min(ST, w.ni - a0), nb = min(ST, w.nj - b0), nc = min(ST, w.nk - c0);
-  double* const src = VEC ? f : ph;
-  // tile and upwind layers: local -1 .. n-1 on each axis (local -1 of the
-  // first tile is the node before the pass's first, inside the box)
-  for (int t = threadIdx.x; t < SP * SP * SP; t += TILE_THREADS) {
-    const int la = t % SP - 1, lb = (t / SP) % SP - 1, lc = t / (SP * SP) - 1;
-    if (la >= na || lb >= nb || lc >= nc) continue;
-    const long long n = nidx(g, w.i0 + (a0 + la) * w.di, w.j0 + (b0 + lb) * w.dj, w.k0 + (c0 + lc) * w.dk);
-#pragma unroll
-    for (int q = 0; q < NC; q++) sv[NC * t + q] = src[NC * n + q];
-  }
-  // per node of the tile: update or not, and (VEC) the blend weights
-  const long long nij = (long long)w.ni * w.nj;
-  for (int t = threadIdx.x; t < ST * ST * ST; t += TILE_THREADS) {
-    const int la = t % ST, lb = (t / ST) % ST, lc = t / (ST * ST);
-    unsigned char upd = 0;
-    if (la < na && lb < nb && lc < nc) {
-      const int a = a0 + la, b = b0 + lb, c = c0 + lc;
-      const int i = w.i0 + a * w.di, j = w.j0 + b * w.dj, k = w.k0 + c * w.dk;
-      const long long n = nidx(g, i, j, k);
-      if (ms[n] == 0) {
-        if (!VEC) {
-          upd = 1;
-        } else {
-          const unsigned long long rank = (unsigned long long)(a + (long long)b * w.ni + (long long)c * nij);
-          const double pn = ph[n];
-          double dp = pn - ph[nidx(g, i - w.di, j, k)], dpn = pn - ph[nidx(g, i + w.di, j, k)];
-          bool skip = dp < 0 && dpn >= 0;
-          double dq = 0, dqn = 0, dr = 0, drn = 0;
-          if (!skip) {
-            dq = pn - ph[nidx(g, i, j - w.dj, k)];
-            dqn = pn - ph[nidx(g, i, j + w.dj, k)];
-            skip = dq < 0 && dqn >= 0;
-          }
-          if (!skip) {
-            dr = pn - ph[nidx(g, i, j, k - w.dk)];
-            drn = pn - ph[nidx(g, i, j, k + w.dk)];
-            skip = dr < 0 && drn >= 0;
-          }
-          if (!skip) {
-            if (rank >= ranks[0]) dp = 0;
-            if (rank >= ranks[1]) dq = 0;
-            if (rank >= ranks[2]) dr = 0;
-            double alpha, beta;
-            if (dp + dq + dr < 1e-3) {
-              alpha = 0.333;
-              beta = 0.333;
-            } else {
-              alpha = dp / (dp + dq + dr);
-              beta = dq / (dp + dq + dr);
-            }
-            sAlpha[t] = alpha;
-            sBeta[t] = beta;
-            upd = 1;
-          }
-        }
-      }
-    }
-    sUpd[t] = upd;
-  }
-  __syncthreads();
-  const int la = threadIdx.x % ST, lb = threadIdx.x / ST;
-  const bool mine = threadIdx.x < ST * ST && la < na && lb < nb;
-  for (int q = 0; q <= (na - 1) + (nb - 1) + (nc - 1); q++) {
-    const int lc = q - la - lb;
-    if (mine && lc >= 0 && lc < nc) {
-      const int u = la + lb * ST + lc * ST * ST;
-      if (sUpd[u]) {
-        const int s = (la + 1) + (lb + 1) * SP + (lc + 1) * SP * SP;
-        const int sa = s - 1, sb = s - SP, sc = s - SP * SP;  // upwind in a, b, c
-        if (!VEC) {
-          solve_distance(sv[sa], sv[sb], sv[sc], &sv[s]);
-        } else {
-          const double alpha = sAlpha[u], beta = sBeta[u];
-#pragma unroll
-          for (int e = 0; e < 3; e++)
-            sv[3 * s + e] = (alpha * sv[3 * sa + e] + beta * sv[3 * sb + e]) + (1 - alpha - beta) * sv[3 * sc + e];
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < SP * SP * SP; t += TILE_THREADS) {
-    const int ta = t % SP - 1, tb = (t / SP) % SP - 1, tc = t / (SP * SP) - 1;
-    if (ta < 0 || tb < 0 || tc < 0 || ta >= na || tb >= nb || tc >= nc) continue;
-    const long long n = nidx(g, w.i0 + (a0 + ta) * w.di, w.j0 + (b0 + tb) * w.dj, w.k0 + (c0 + tc) * w.dk);
-#pragma unroll
-    for (int e = 0; e < NC; e++) src[NC * n + e] = sv[NC * t + e];
-  }
-}
-// A whole sweep pass in one cooperative launch: the blocks walk the pass's
-// hyperplanes a + b + c = p in order, each plane split over all threads, with
-// a grid-wide barrier between planes. Values written in this pass by other
-// blocks are read through L2 (ld.cg); the barrier is one growing counter in
-// global memory, its wait bounded (a block that gives up sets *err and
-// carries on, so the launch always ends; the host reports it).
-// Same per-node operations as k_sweep_tile, each node after its three
-// upwind neighbours, so the same bits; the critical path is the 3n planes
-// rather than the tile wavefront's ~9n sub-planes.
-constexpr unsigned WAVE_WAIT_LIMIT = 1u << 22;
-// Arrival p of every block: a release add on a counter that only grows (the
-// host zeroes it before the launch), then acquire loads until it reaches
-// (p + 1) x blocks.
-__device__ __forceinline__ void wave_barrier(unsigned* count, unsigned target, int* err) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned cur;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(cur) : "l"(count) : "memory");
-    cur += 1;
-    unsigned it = 0;
-    while (cur < target && ++it < WAVE_WAIT_LIMIT)
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(count) : "memory");
-    if (cur < target) *err = 1;
-  }
-  __syncthreads();
-}
-template <bool VEC>
-__global__ void __launch_bounds__(SWEEP_THREADS) k_sweep_wave(GridDev g, double* f, double* ph,
-                                                              const double* ms, Sweep w,
-                                                              const unsigned long long* ranks,
-                                                              unsigned* bar, int* err) {
-  const long long nij = (long long)w.ni * w.nj;
-  const int planes = w.ni + w.nj + w.nk - 2;
-  unsigned long long rx = 0, ry = 0, rz = 0;
-  if (VEC) {
-    rx = ranks[0];
-    ry = ranks[1];
-    rz = ranks[2];
-  }
-  for (int p = 0; p < planes; p++) {
-    for (long long t = blockIdx.x * (long long)SWEEP_THREADS + threadIdx.x; t < nij;
-         t += (long long)gridDim.x * SWEEP_THREADS) {
-      const int a = (int)(t % w.ni), b = (int)(t / w.ni);
-      const int c = p - a - b;
-      if (c < 0 || c >= w.nk) continue;
-      const int i = w.i0 + a * w.di, j = w.j0 + b * w.dj, k = w.k0 + c * w.dk;
-      const long long n = nidx(g, i, j, k);
-      if (ms[n] != 0) continue;
-      const long long ea = nidx(g, i - w.di, j, k), eb = nidx(g, i, j - w.dj, k), ec = nidx(g, i, j, k - w.dk);
-      if (!VEC) {
-        double v = __ldcg(ph + n);
-        solve_distance(__ldcg(ph + ea), __ldcg(ph + eb), __ldcg(ph + ec), &v);
-        ph[n] = v;
-        continue;
-      }
-      const unsigned long long rank = (unsigned long long)(a + (long long)b * w.ni + (long long)c * nij);
-      const double pn = ph[n];
-      double dp = pn - ph[ea], dpn = pn - ph[nidx(g, i + w.di, j, k)];
-      if (dp < 0 && dpn >= 0) continue;
-      double dq = pn - ph[eb], dqn = pn - ph[nidx(g, i, j + w.dj, k)];
-      if (dq < 0 && dqn >= 0) continue;
-      double dr = pn - ph[ec], drn = pn - ph[nidx(g, i, j, k + w.dk)];
-      if (dr < 0 && drn >= 0) continue;
-      if (rank >= rx) dp = 0;
-      if (rank >= ry) dq = 0;
-      if (rank >= rz) dr = 0;
-      double alpha, beta;
-      if (dp + dq + dr < 1e-3) {
-        alpha = 0.333;
-        beta = 0.333;
-      } else {
-        alpha = dp / (dp + dq + dr);
-        beta = dq / (dp + dq + dr);
-      }
-#pragma unroll
-      for (int e = 0; e < 3; e++)
-        f[3 * n + e] = (alpha * __ldcg(f + 3 * ea + e) + beta * __ldcg(f + 3 * eb + e)) +
-                       (1 - alpha - beta) * __ldcg(f + 3 * ec + e);
-    }
-    wave_barrier(bar, (unsigned)(p + 1) * gridDim.x, err);
-  }
-}
-
-// Launches of one sweep pass as a tile wavefront.
-inline int sweep_tile_launches(const Sweep& w) {
-  return (w.ni + ST - 1) / ST + (w.nj + ST - 1) / ST + (w.nk + ST - 1) / ST - 2;
-}
-inline int sweep_tile_blocks(const Sweep& w) {
-  return ((w.ni + ST - 1) / ST) * ((w.nj + ST - 1) / ST);
-}
+#include "esf_sweep.cuh"
 
 // Face copies of sweepVectorField (DEFOR_SOLID_3D.cpp:544-563), one axis
 // per launch, in the order z, y, x.

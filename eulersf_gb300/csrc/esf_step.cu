@@ -165,8 +165,9 @@ struct esf_scene {
   esf::DBuf contactCount;  // particles that took a solid-solid impulse this step
   // scratch
   esf::DBuf cubTmp, keys, vals, skeys, svals, bstart, bend, mt, pweights;
+  esf::DBuf sweepMail, sweepDims, sweepList;  // sweepPhi's mailboxes and ticket; velocity passes' bounds and lists
   long long mtLen = 0;
-  int *dInts = nullptr, *hInts = nullptr;
+  int *dInts = nullptr, *hInts = nullptr;  // 64 words; pinned copies, and 64 more of the velocity extension
   unsigned long long* dU64 = nullptr;
   unsigned long long* hU64 = nullptr;
   esf::PressureWork* pw = nullptr;
@@ -309,7 +310,7 @@ extern "C" esf_status esf_create(const esf_grid* g, const esf_params* p, void* s
   A(dInts, 64 * 4);
   A(dU64, 16 * 8);
 #undef A
-  if (!e && cudaMallocHost(&s->hInts, 64 * 4) != cudaSuccess) e = ESF_ERR_OOM;
+  if (!e && cudaMallocHost(&s->hInts, 128 * 4) != cudaSuccess) e = ESF_ERR_OOM;
   if (!e && cudaMallocHost(&s->hU64, 16 * 8) != cudaSuccess) e = ESF_ERR_OOM;
   if (!e) {
     // zero-initialised like the reference's Eigen/vector fields
@@ -374,7 +375,7 @@ extern "C" esf_status esf_destroy(esf_scene* s) {
   DBuf* bufs[] = {&s->sNode, &s->solidF, &s->solidMv, &s->damped, &s->solidV0, &s->solidPC,
                   &s->solidB1, &s->sysDiag, &s->blocks, &s->nbr, &s->mask, &s->Ke, &s->nf, &s->fbCells, &s->fbSlot, &s->mfCell, &s->mfCorner,
                   &s->energy, &s->cubTmp, &s->keys, &s->vals, &s->skeys, &s->svals, &s->bstart,
-                  &s->bend, &s->mt, &s->pweights, &s->contactCount};
+                  &s->bend, &s->mt, &s->pweights, &s->contactCount, &s->sweepMail, &s->sweepDims, &s->sweepList};
   for (DBuf* b : bufs) b->release();
   pressure_work_free(s->pw);
   solid_work_free(s->sw);
@@ -665,19 +666,36 @@ static esf_status compute_solid_mass(esf_scene* sc, Solid* d, int usesdf) {
   return ESF_OK;
 }
 
-// One Gauss-Seidel sweep pass (sweepPhi when !VEC, sweepOnePass of the
-// velocity when VEC): the cooperative hyperplane wave (k_sweep_wave, one
-// launch per pass, sweepPhi) or the tile wavefront (k_sweep_tile, ~3n/8
-// launches, the velocity passes, and sweepPhi where the device has no
-// cooperative launch); ESF_SWEEP=wave or =tiles forces one for both. Both
-// give the bits of the sequential loop. A wave whose
-// grid barrier timed out raises the scene's sweep error word (dInts[42]),
-// checked when the step or init ends.
+// The Gauss-Seidel sweeps: sweepPhi as a systolic march of warps
+// (k_sweep_march), the velocity extension over level lists (k_extend_field);
+// ESF_SWEEP=wave runs both as cooperative hyperplane waves (k_sweep_wave)
+// instead, for comparison. Either gives the bits of the sequential loops. A
+// wait that ran out raises the scene's sweep error word (dInts[42]), checked
+// when the step or init ends.
 constexpr int kSweepBar = 40, kSweepErr = 42;
 constexpr int kFallbackCount = 44;  // mixed: cells of the FP32 stiffness evaluated again in FP64 (one per solid)
 constexpr int kOverlap = 52;        // broad phase: two solids' meshes overlap
+static bool sweep_wave_asked() {
+  const char* pick = getenv("ESF_SWEEP");
+  return pick && strcmp(pick, "wave") == 0;
+}
+// direction `dir` of the reference's eight loops over the box, which leave
+// out `margin` nodes of each axis
+static Sweep sweep_of(const Box& ex, int dir, int margin) {
+  Sweep w;
+  w.dj = (dir & 1) ? -1 : 1;
+  w.di = (dir & 2) ? -1 : 1;
+  w.dk = (dir & 4) ? -1 : 1;
+  w.i0 = w.di > 0 ? ex.lo[0] + 1 : ex.hi[0] - 2;
+  w.j0 = w.dj > 0 ? ex.lo[1] + 1 : ex.hi[1] - 2;
+  w.k0 = w.dk > 0 ? ex.lo[2] + 1 : ex.hi[2] - 2;
+  w.ni = ex.hi[0] - ex.lo[0] - margin;
+  w.nj = ex.hi[1] - ex.lo[1] - margin;
+  w.nk = ex.hi[2] - ex.lo[2] - margin;
+  return w;
+}
 template <bool VEC>
-static esf_status sweep_pass(esf_scene* sc, Solid* d, const Sweep& w, const unsigned long long* ranks) {
+static esf_status sweep_wave(esf_scene* sc, Solid* d, const Sweep& w, const unsigned long long* ranks) {
   cudaStream_t st = sc->stream;
   static const int coopBlocks = [] {
     int dev = 0, coop = 0, sms = 0, per = 0;
@@ -689,37 +707,125 @@ static esf_status sweep_pass(esf_scene* sc, Solid* d, const Sweep& w, const unsi
       return 0;
     return sms * per;
   }();
-  // sweepPhi's per-node work (FP64 square roots and divisions) makes its
-  // critical path the cost: the wave (3n steps) beats the tiles (~9n
-  // sub-plane steps), 23.3 against 37.6 ms for 2 x 8 passes per 256^3 step
-  // (blocks of 32, 64 or 128 threads: the same). The velocity pass is a
-  // blend of three values: there the wave's ~5 us per plane (grid barrier,
-  // L2 round trips) costs more than the tiles' extra sub-planes in shared
-  // memory, 37.6 against 21.1 ms for 4 x 8 passes. One cluster of 8 blocks
-  // of 1024 threads with the hardware cluster barrier measured 82 ms for
-  // sweepPhi: FP64 work of a plane on 8 SMs.
-  const char* pick = getenv("ESF_SWEEP");
-  const bool wave = pick ? strcmp(pick, "wave") == 0 : !VEC;
+  if (coopBlocks <= 0) {
+    set_error("ESF_SWEEP=wave: the device has no cooperative launch");
+    return ESF_ERR_UNSUPPORTED;
+  }
+  const long long nij = (long long)w.ni * w.nj;
+  const int blocks = (int)std::min<long long>(coopBlocks, (nij + SWEEP_THREADS - 1) / SWEEP_THREADS);
+  unsigned* bar = reinterpret_cast<unsigned*>(sc->dInts + kSweepBar);
+  int* err = sc->dInts + kSweepErr;
+  ESF_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), st));
+  GridDev g = sc->g;
   double* f = VEC ? d->d.vel : nullptr;
   double* ph = d->d.phi;
   const double* ms = d->d.mass;
-  if (coopBlocks > 0 && wave) {
-    const long long nij = (long long)w.ni * w.nj;
-    const int blocks = (int)std::min<long long>(coopBlocks, (nij + SWEEP_THREADS - 1) / SWEEP_THREADS);
-    unsigned* bar = reinterpret_cast<unsigned*>(sc->dInts + kSweepBar);
-    int* err = sc->dInts + kSweepErr;
-    ESF_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), st));
-    GridDev g = sc->g;
-    Sweep ww = w;
-    void* args[] = {&g, &f, &ph, (void*)&ms, &ww, (void*)&ranks, &bar, &err};
-    note_launch();
-    ESF_CUDA(cudaLaunchCooperativeKernel((const void*)k_sweep_wave<VEC>, dim3(blocks), dim3(SWEEP_THREADS),
-                                         args, 0, st));
+  Sweep ww = w;
+  void* args[] = {&g, &f, &ph, (void*)&ms, &ww, (void*)&ranks, &bar, &err};
+  note_launch();
+  ESF_CUDA(cudaLaunchCooperativeKernel((const void*)k_sweep_wave<VEC>, dim3(blocks), dim3(SWEEP_THREADS), args, 0,
+                                       st));
+  return ESF_OK;
+}
+// 2 x sweepPhi (DEFOR_SOLID_3D.cpp:397-455), eight passes each
+static esf_status sweep_phi(esf_scene* sc, Solid* d, const Box& ex) {
+  const Sweep shape = sweep_of(ex, 0, 1);
+  if (shape.ni <= 0 || shape.nj <= 0 || shape.nk <= 0) return ESF_OK;
+  if (sweep_wave_asked()) {
+    for (int pass = 0; pass < 16; pass++) TRY(sweep_wave<false>(sc, d, sweep_of(ex, pass % 8, 1), nullptr));
     return ESF_OK;
   }
-  const int launches = sweep_tile_launches(w), blocks = sweep_tile_blocks(w);
-  for (int P = 0; P < launches; P++)
-    ESF_COUNTED k_sweep_tile<VEC><<<blocks, TILE_THREADS, 0, st>>>(sc->g, f, ph, ms, w, P, ranks);
+  const GridDev& G = sc->g;
+  cudaStream_t st = sc->stream;
+  // distances reach X + Y + Z + 2 nodes; beyond 4096 FP32 no longer decides
+  // which square roots matter (solve_distance_fast)
+  const float skipBelow = G.X + G.Y + G.Z + 2 <= 4096 ? 0.99f : 0.0f;
+  // the passes' seed bounds and tickets (PHI_PASS_WORDS words each), then the
+  // mailboxes, emptied before each pass
+  const size_t head = (size_t)16 * PHI_PASS_WORDS * sizeof(int), mail = march_mail(shape) * sizeof(double);
+  TRY(sc->sweepMail.ensure(head + mail));
+  int* state = sc->sweepMail.as<int>();
+  double* box = reinterpret_cast<double*>(sc->sweepMail.as<char>() + head);
+  ESF_CUDA(cudaMemsetAsync(state, 0x7f, head, st));
+  const long long total = (long long)shape.ni * shape.nj * shape.nk;
+  for (int pass = 0; pass < 16; pass++, state += PHI_PASS_WORDS) {
+    const Sweep w = sweep_of(ex, pass % 8, 1);
+    if (mail) ESF_CUDA(cudaMemsetAsync(box, 0xff, mail, st));
+    ESF_COUNTED k_sweep_seeds<<<kblocks(total), KT, 0, st>>>(G, d->d.phi, d->d.mass, w, state, skipBelow);
+    ESF_COUNTED k_sweep_march<<<march_patches(w), 32, 0, st>>>(G, d->d.phi, d->d.mass, w, state, box,
+                                                               sc->dInts + kSweepErr, skipBelow);
+  }
+  ESF_LAUNCH_CHECK();
+  return ESF_OK;
+}
+// extendVectorField (DEFOR_SOLID_3D.cpp:566-574): 4 x (eight passes of
+// sweepOnePass, then the face copies)
+static esf_status extend_velocity(esf_scene* sc, Solid* d) {
+  const GridDev& G = sc->g;
+  cudaStream_t st = sc->stream;
+  const Box ex = mkbox(d->ex[0], d->ex[1], d->ex[2], d->ex[3], d->ex[4], d->ex[5]);
+  if (ex.hi[0] - ex.lo[0] < 3 || ex.hi[1] - ex.lo[1] < 3 || ex.hi[2] - ex.lo[2] < 3) return ESF_OK;
+  Sweep8 all;
+  for (int dir = 0; dir < 8; dir++) all.d[dir] = sweep_of(ex, dir, 2);
+  const Sweep& shape = all.d[0];
+  const long long total = (long long)shape.ni * shape.nj * shape.nk;  // each at least 1
+  // the weights lie in the particle weights' buffer, which the gather before
+  // was the last to read; the flags' ranks, the octants' bounds, the levels and
+  // the lists in buffers of their own
+  SweepLists L;
+  L.levels = shape.ni + shape.nj + shape.nk - 1;
+  const size_t words = 48 + 8 + 8 * (size_t)(L.levels + 1) + 8 * (size_t)L.levels;
+  TRY(sc->sweepDims.ensure(24 * sizeof(unsigned long long) + words * sizeof(int)));
+  unsigned long long* ranks = sc->sweepDims.as<unsigned long long>();
+  int* dims = reinterpret_cast<int*>(ranks + 24);
+  L.count = dims + 48;
+  L.off = L.count + 8;
+  L.cur = L.off + 8 * (L.levels + 1);
+  TRY(sc->pweights.ensure((size_t)8 * total * sizeof(double2)));
+  double2* wt = sc->pweights.as<double2>();
+  L.entry = nullptr;
+  int* const h = sc->hInts + 64;
+  for (int q = 0; q < 48; q++) h[q] = q % 2 ? -1 : INT_MAX;
+  ESF_CUDA(cudaMemsetAsync(ranks, 0xff, 24 * sizeof(unsigned long long), st));
+  ESF_CUDA(cudaMemcpyAsync(dims, h, 48 * sizeof(int), cudaMemcpyHostToDevice, st));
+  ESF_CUDA(cudaMemsetAsync(L.off, 0, 8 * (size_t)(L.levels + 1) * sizeof(int), st));
+  const dim3 grid(std::min(kblocks(total), 152 * 4), 8);
+  ESF_COUNTED k_sweep_vec_ranks<<<grid, KT, 0, st>>>(G, d->d.phi, d->d.mass, all, ranks);
+  ESF_COUNTED k_sweep_vec_weights<<<grid, KT, 0, st>>>(G, d->d.phi, d->d.mass, all, ranks, wt, dims);
+  ESF_COUNTED k_sweep_vec_list<true><<<grid, KT, 0, st>>>(G, all, wt, dims, L);
+  ESF_COUNTED k_sweep_vec_scan<<<8, KT, 0, st>>>(L);
+  ESF_LAUNCH_CHECK();
+  ESF_CUDA(cudaMemcpyAsync(h, dims, 56 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  ESF_CUDA(cudaStreamSynchronize(st));
+  // columns of the largest octant's plane, and all entries
+  long long cols = 1, entries = 0;
+  for (int dir = 0; dir < 8; dir++) {
+    const int* q = h + 6 * dir;
+    if (q[1] < 0) continue;
+    cols = std::max(cols, (long long)(q[3] - q[2] + 2) * (q[5] - q[4] + 2));
+    entries += h[48 + dir];
+  }
+  // two planes and the levels in shared memory: octants up to 115 x 115
+  // columns (a solid that spans more than 200 nodes); beyond that the wave
+  const long long smem = 16 * cols + 32LL * (L.levels + 1);
+  if (!sweep_wave_asked() && smem <= 220 * 1024) {
+    TRY(sc->sweepList.ensure((size_t)entries * sizeof(SweepEntry)));
+    L.entry = sc->sweepList.as<SweepEntry>();
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_extend_field, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    ESF_CUDA(attr);
+    ESF_COUNTED k_sweep_vec_list<false><<<grid, KT, 0, st>>>(G, all, wt, dims, L);
+    ESF_COUNTED k_extend_field<<<3, EXTEND_THREADS, (size_t)smem, st>>>(G, d->d.vel, d->d.mass, ex, all, dims, L,
+                                                                        (int)cols);
+    ESF_LAUNCH_CHECK();
+    return ESF_OK;
+  }
+  for (int round = 0; round < 4; round++) {
+    for (int dir = 0; dir < 8; dir++) TRY(sweep_wave<true>(sc, d, all.d[dir], ranks + 3 * dir));
+    for (int axis = 2; axis >= 0; axis--)
+      ESF_COUNTED k_extend_faces<<<kblocks(boxn(ex) / (ex.hi[axis] - ex.lo[axis])), KT, 0, st>>>(
+          G, d->d.vel, d->d.mass, ex, axis);
+  }
   ESF_LAUNCH_CHECK();
   return ESF_OK;
 }
@@ -764,23 +870,7 @@ static esf_status compute_sdf(esf_scene* sc, Solid* d) {
   d->ex[4] = std::min(ymax + exn, G.Y);
   d->ex[5] = std::min(zmax + exn, G.Z);
   Box ex = mkbox(d->ex[0], d->ex[1], d->ex[2], d->ex[3], d->ex[4], d->ex[5]);
-  // 2 x sweepPhi: 8 passes each, every pass a wavefront of 8^3 tiles
-  for (int rep = 0; rep < 2; rep++)
-    for (int dir = 0; dir < 8; dir++) {
-      Sweep w;
-      w.dj = (dir & 1) ? -1 : 1;
-      w.di = (dir & 2) ? -1 : 1;
-      w.dk = (dir & 4) ? -1 : 1;
-      w.i0 = w.di > 0 ? ex.lo[0] + 1 : ex.hi[0] - 2;
-      w.j0 = w.dj > 0 ? ex.lo[1] + 1 : ex.hi[1] - 2;
-      w.k0 = w.dk > 0 ? ex.lo[2] + 1 : ex.hi[2] - 2;
-      w.ni = ex.hi[0] - ex.lo[0] - 1;
-      w.nj = ex.hi[1] - ex.lo[1] - 1;
-      w.nk = ex.hi[2] - ex.lo[2] - 1;
-      if (w.ni <= 0 || w.nj <= 0 || w.nk <= 0) continue;
-      TRY(sweep_pass<false>(sc, d, w, nullptr));
-    }
-  ESF_LAUNCH_CHECK();
+  TRY(sweep_phi(sc, d, ex));
   tm.mark("sdf: 2 x sweepPhi");
   return ESF_OK;
 }
@@ -1350,36 +1440,7 @@ extern "C" esf_status esf_step(esf_scene* sc, esf_step_report* rep) {
     tm.mark("p2g: gather");
   }
   ESF_CUDA(cudaEventRecord(sc->ph[8], st));
-  for (int i = 0; i < sc->ns; i++) {  // extendVectorField = 4 x sweepVectorField
-    Solid* d = sc->s[i];
-    Box ex = mkbox(d->ex[0], d->ex[1], d->ex[2], d->ex[3], d->ex[4], d->ex[5]);
-    if (ex.hi[0] - ex.lo[0] < 3 || ex.hi[1] - ex.lo[1] < 3 || ex.hi[2] - ex.lo[2] < 3) continue;
-    unsigned long long* ranks = sc->dU64 + 8;
-    for (int rep = 0; rep < 4; rep++) {
-      for (int dir = 0; dir < 8; dir++) {
-        Sweep w;
-        w.dj = (dir & 1) ? -1 : 1;
-        w.di = (dir & 2) ? -1 : 1;
-        w.dk = (dir & 4) ? -1 : 1;
-        w.i0 = w.di > 0 ? ex.lo[0] + 1 : ex.hi[0] - 2;
-        w.j0 = w.dj > 0 ? ex.lo[1] + 1 : ex.hi[1] - 2;
-        w.k0 = w.dk > 0 ? ex.lo[2] + 1 : ex.hi[2] - 2;
-        w.ni = ex.hi[0] - ex.lo[0] - 2;
-        w.nj = ex.hi[1] - ex.lo[1] - 2;
-        w.nk = ex.hi[2] - ex.lo[2] - 2;
-        if (w.ni <= 0 || w.nj <= 0 || w.nk <= 0) continue;
-        ESF_CUDA(cudaMemsetAsync(ranks, 0xff, 3 * 8, st));
-        const long long total = (long long)w.ni * w.nj * w.nk;
-        ESF_COUNTED k_sweep_vec_ranks<<<kblocks(total), KT, 0, st>>>(G, d->d.phi, d->d.mass, w, ranks);
-        TRY(sweep_pass<true>(sc, d, w, ranks));
-      }
-      for (int axis = 2; axis >= 0; axis--) {
-        const long long nf = boxn(ex) / (ex.hi[axis] - ex.lo[axis]);
-        ESF_COUNTED k_extend_faces<<<kblocks(nf), KT, 0, st>>>(G, d->d.vel, d->d.mass, ex, axis);
-      }
-    }
-    ESF_LAUNCH_CHECK();
-  }
+  for (int i = 0; i < sc->ns; i++) TRY(extend_velocity(sc, sc->s[i]));
   ESF_CUDA(cudaEventRecord(sc->ph[9], st));
   for (int i = 0; i < sc->ns; i++) {  // DEFOR_SOLID_3D::finalizeSolution() (:1198-1233)
     Solid* d = sc->s[i];
