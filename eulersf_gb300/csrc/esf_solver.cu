@@ -1662,93 +1662,112 @@ struct SolidMF {
 };
 constexpr int MF_CELL_PLANES = 43;
 
+// valid cell t's 24 shares of K x (x: the solid vector, as a function of its index)
+template <typename X>
+__device__ __forceinline__ void mf_cell(const SolidMF& m, long long t, const X& x, float* share) {
+  const long long nc = m.nc;
+  const float* q = m.cell + t;
+  float GF[8][3], dF[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    // (loads without a branch: the eight corners' are in flight together)
+    const int j = m.corner[i * nc + t];
+    const long long k = 3 * (long long)max(j, 0);
+    float xi[3] = {x(k), x(k + 1), x(k + 2)};
+#pragma unroll
+    for (int a = 0; a < 3; a++) xi[a] = j >= 0 ? xi[a] : 0.0f;
+#pragma unroll
+    for (int b = 0; b < 3; b++) GF[i][b] = q[(18 + 3 * i + b) * nc];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+      for (int b = 0; b < 3; b++) dF[a][b] += xi[a] * GF[i][b];
+  }
+  float R[3][3], L[3][3];
+#pragma unroll
+  for (int i = 0; i < 9; i++) {
+    R[i / 3][i % 3] = q[i * nc];
+    L[i / 3][i % 3] = q[(9 + i) * nc];
+  }
+  // dPK(dF) = R (2 mu sym + lambda tr(sym) I + lambda tr(R^T dF) I + [L f]x),
+  // R^T dF = dFh, sym/skew of dFh, f the axial vector of the skew part
+  float h[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int b = 0; b < 3; b++) h[a][b] = (R[0][a] * dF[0][b] + R[1][a] * dF[1][b]) + R[2][a] * dF[2][b];
+  const float trh = h[0][0] + (h[1][1] + h[2][2]);
+  float P[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int b = 0; b < 3; b++) P[a][b] = m.mu * (h[a][b] + h[b][a]) + (a == b ? 2.0f * m.lambda * trh : 0.0f);
+  const float f[3] = {-0.5f * (h[1][2] - h[2][1]) + 0.5f * (h[2][1] - h[1][2]),
+                      -0.5f * (h[2][0] - h[0][2]) + 0.5f * (h[0][2] - h[2][0]),
+                      -0.5f * (h[0][1] - h[1][0]) + 0.5f * (h[1][0] - h[0][1])};
+  float Lf[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) Lf[a] = (L[a][0] * f[0] + L[a][1] * f[1]) + L[a][2] * f[2];
+  P[0][1] -= Lf[2];
+  P[0][2] += Lf[1];
+  P[1][0] += Lf[2];
+  P[1][2] -= Lf[0];
+  P[2][0] -= Lf[1];
+  P[2][1] += Lf[0];
+  float D[3][3];  // R P
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int b = 0; b < 3; b++) D[a][b] = (R[a][0] * P[0][b] + R[a][1] * P[1][b]) + R[a][2] * P[2][b];
+  const float w = q[42 * nc] * m.scale;
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+      share[(3 * i + r) * nc + t] = w * ((D[r][0] * GF[i][0] + D[r][1] * GF[i][1]) + D[r][2] * GF[i][2]);
+}
 __global__ void __launch_bounds__(VT) k_mf_cell(SolidMF m, const float* __restrict__ x,
                                                  float* __restrict__ share, const PcrState* st) {
   if (st->done) return;
-  const long long nc = m.nc;
-  for (long long t = blockIdx.x * (long long)VT + threadIdx.x; t < nc; t += (long long)gridDim.x * VT) {
-    const float* q = m.cell + t;
-    float GF[8][3], dF[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int j = m.corner[i * nc + t];
-      float xi[3] = {0.0f, 0.0f, 0.0f};
-      if (j >= 0) {
-        xi[0] = x[3 * (long long)j];
-        xi[1] = x[3 * (long long)j + 1];
-        xi[2] = x[3 * (long long)j + 2];
-      }
-#pragma unroll
-      for (int b = 0; b < 3; b++) GF[i][b] = q[(18 + 3 * i + b) * nc];
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) dF[a][b] += xi[a] * GF[i][b];
-    }
-    float R[3][3], L[3][3];
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-      R[i / 3][i % 3] = q[i * nc];
-      L[i / 3][i % 3] = q[(9 + i) * nc];
-    }
-    // dPK(dF) = R (2 mu sym + lambda tr(sym) I + lambda tr(R^T dF) I + [L f]x),
-    // R^T dF = dFh, sym/skew of dFh, f the axial vector of the skew part
-    float h[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int b = 0; b < 3; b++) h[a][b] = (R[0][a] * dF[0][b] + R[1][a] * dF[1][b]) + R[2][a] * dF[2][b];
-    const float trh = h[0][0] + (h[1][1] + h[2][2]);
-    float P[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int b = 0; b < 3; b++) P[a][b] = m.mu * (h[a][b] + h[b][a]) + (a == b ? 2.0f * m.lambda * trh : 0.0f);
-    const float f[3] = {-0.5f * (h[1][2] - h[2][1]) + 0.5f * (h[2][1] - h[1][2]),
-                        -0.5f * (h[2][0] - h[0][2]) + 0.5f * (h[0][2] - h[2][0]),
-                        -0.5f * (h[0][1] - h[1][0]) + 0.5f * (h[1][0] - h[0][1])};
-    float Lf[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) Lf[a] = (L[a][0] * f[0] + L[a][1] * f[1]) + L[a][2] * f[2];
-    P[0][1] -= Lf[2];
-    P[0][2] += Lf[1];
-    P[1][0] += Lf[2];
-    P[1][2] -= Lf[0];
-    P[2][0] -= Lf[1];
-    P[2][1] += Lf[0];
-    float D[3][3];  // R P
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int b = 0; b < 3; b++) D[a][b] = (R[a][0] * P[0][b] + R[a][1] * P[1][b]) + R[a][2] * P[2][b];
-    const float w = q[42 * nc] * m.scale;
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-        share[(3 * i + r) * nc + t] = w * ((D[r][0] * GF[i][0] + D[r][1] * GF[i][1]) + D[r][2] * GF[i][2]);
-  }
+  for (long long t = blockIdx.x * (long long)VT + threadIdx.x; t < m.nc; t += (long long)gridDim.x * VT)
+    mf_cell(m, t, [&](long long i) { return x[i]; }, share);
 }
 
+// solid node a's sum of the shares of the (up to 8) cells around it
+__device__ __forceinline__ void mf_node(const SolidMF& m, long long a, const float* share, float y[3]) {
+  const GridDev& g = m.g;
+  const long long n = m.sNode[a];
+  const int nx = (int)(n % g.X), ny = (int)((n / g.X) % g.Y), nz = (int)(n / g.slab);
+  y[0] = y[1] = y[2] = 0.0f;
+  // the cells around the node, corner ia of each; loads without branches, so
+  // that the eight cells' are in flight together
+  int ord[8];
+  float sh[8][3];
+#pragma unroll
+  for (int ia = 7; ia >= 0; ia--) {
+    const int cx = nx - (ia & 1), cy = ny - ((ia >> 1) & 1), cz = nz - ((ia >> 2) & 1);
+    const bool in = cx >= 0 && cy >= 0 && cz >= 0 && cx <= g.X - 2 && cy <= g.Y - 2 && cz <= g.Z - 2;
+    const int o = m.cellOrd[in ? cx + (long long)cy * g.cX + (long long)cz * g.cslab : 0];
+    ord[ia] = in ? o : -1;
+  }
+#pragma unroll
+  for (int ia = 7; ia >= 0; ia--)
+#pragma unroll
+    for (int r = 0; r < 3; r++) sh[ia][r] = share[(3 * ia + r) * m.nc + max(ord[ia], 0)];
+#pragma unroll
+  for (int ia = 7; ia >= 0; ia--)
+#pragma unroll
+    for (int r = 0; r < 3; r++) y[r] = ord[ia] >= 0 ? y[r] + sh[ia][r] : y[r];
+}
 __global__ void __launch_bounds__(VT) k_mf_gather(SolidMF m, long long S, const float* __restrict__ share,
                                                    const float* __restrict__ damped, const float* in, float* out,
                                                    double* partial, PcrState* st) {
   __shared__ double sred[32];
   if (st->done) return;
-  const GridDev& g = m.g;
   float accT = 0;
   for (long long a = blockIdx.x * (long long)VT + threadIdx.x; a < S; a += (long long)gridDim.x * VT) {
-    const long long n = m.sNode[a];
-    const int nx = (int)(n % g.X), ny = (int)((n / g.X) % g.Y), nz = (int)(n / g.slab);
-    float y[3] = {0.0f, 0.0f, 0.0f};
-    for (int ia = 7; ia >= 0; ia--) {  // the cells around the node, corner ia of each
-      const int cx = nx - (ia & 1), cy = ny - ((ia >> 1) & 1), cz = nz - ((ia >> 2) & 1);
-      if (cx < 0 || cy < 0 || cz < 0 || cx > g.X - 2 || cy > g.Y - 2 || cz > g.Z - 2) continue;
-      const int ord = m.cellOrd[cx + (long long)cy * g.cX + (long long)cz * g.cslab];
-      if (ord < 0) continue;
-#pragma unroll
-      for (int r = 0; r < 3; r++) y[r] += share[(3 * ia + r) * m.nc + ord];
-    }
+    float y[3];
+    mf_node(m, a, share, y);
 #pragma unroll
     for (int r = 0; r < 3; r++) {
       const long long i = 3 * a + r;
@@ -1793,6 +1812,7 @@ struct SolidWork {
   long long mfShareCap;
   float* damped32;      // damped mass (the assembled diagonal's mass part), FP32
   double *r, *d, *Ap, *s, *invd, *partial;
+  unsigned* bar;      // grid barrier of the persistent solve: arrivals, error
   float *blocks32, *x32, *r32, *d32, *Ap32, *s32, *invd32, *b32;
   PcrState *st, *st32;
   long long cap;
@@ -1813,6 +1833,7 @@ esf_status solid_work_alloc(SolidWork** out, long long S, int mixed) {
   ESF_CUDA(cudaMalloc(&w->partial, ESF_MAX_PARTIALS * 8));
   ESF_CUDA(cudaMalloc(&w->st, sizeof(PcrState)));
   ESF_CUDA(cudaMalloc(&w->st32, sizeof(PcrState)));
+  ESF_CUDA(cudaMalloc(&w->bar, 2 * sizeof(unsigned)));
   ESF_CUDA(cudaMallocHost(&w->hst, 4 * sizeof(PcrState)));
   for (int i = 0; i < 4; i++) ESF_CUDA(cudaEventCreateWithFlags(&w->ev[i], cudaEventDisableTiming));
   ESF_CUDA(cudaStreamCreateWithFlags(&w->capStream, cudaStreamNonBlocking));
@@ -1836,7 +1857,7 @@ long long solid_work_capacity(const SolidWork* w) { return w ? w->cap : 0; }
 void solid_work_free(SolidWork* w) {
   if (!w) return;
   cudaFree(w->r); cudaFree(w->d); cudaFree(w->Ap); cudaFree(w->s); cudaFree(w->invd);
-  cudaFree(w->partial); cudaFree(w->st); cudaFree(w->st32);
+  cudaFree(w->partial); cudaFree(w->st); cudaFree(w->st32); cudaFree(w->bar);
   vec_free(&w->mapped, w->blocks32);
   cudaFree(w->x32); cudaFree(w->r32); cudaFree(w->d32); cudaFree(w->Ap32); cudaFree(w->s32);
   cudaFree(w->invd32); cudaFree(w->b32);
@@ -1953,14 +1974,27 @@ static esf_status capture_solid(cudaStream_t cs, const SolidKernels<T>& k, bool 
   return ESF_OK;
 }
 
+#include "esf_solid_persist.cuh"
+
 // One solid PCR solve from graphs, set-up and iterations as the reference's.
 template <typename T>
 static esf_status solid_pcr_graph(SolidWork* w, int slot, long long S, const T* blocks, const int* nbr,
                                   const T* invd, const T* b, T* x, T* r, T* d, T* Ap, T* s,
                                   PcrState* dst, double eps, int maxIt, cudaStream_t st, PcrState* out,
                                   int inner) {
-  SolidKernels<T> k{S, blocks, invd, b, nbr, x, r, d, Ap, s, w->partial, dst};
   const bool mf = std::is_same<T, float>::value && w->mfOn;
+  if (S <= persist_rows()) {
+    SolidPersist<T> p{S, blocks, invd, b, nbr, x, r, d, Ap, s, w->partial, dst, w->bar, vec_blocks(3 * S)};
+    if (mf) {
+      p.mf = w->mf;
+      p.share = w->mfShare;
+      p.damped = w->damped32;
+    }
+    esf_status e = init_state(dst, eps, maxIt, st, inner);
+    if (e) return e;
+    return solid_pcr_persist<T>(p, mf, w->hst, st, out);
+  }
+  SolidKernels<T> k{S, blocks, invd, b, nbr, x, r, d, Ap, s, w->partial, dst};
   if (mf) {
     k.mf = &w->mf;
     k.share = w->mfShare;
