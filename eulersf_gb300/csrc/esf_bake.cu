@@ -12,16 +12,27 @@
 // agree away from the threshold; nodes whose distance lies within the SDF
 // grid's interpolation error of dh / 2 can fall either side.
 //
-// One thread per node; the triangles are staged through shared memory in
-// tiles, every thread testing every triangle (a closed mesh of a few thousand
-// triangles and a 220^3 grid is ~2e10 point-triangle tests, tens of ms).
 // Distances and solid angles are evaluated in FP32 relative to the node
 // (coordinates of a few tenths, thresholds of 5e-4), the mass written in FP64.
+//
+// Every node against every triangle (k_bake_mass) is 1.4e10 point-triangle
+// tests for the shipped sphere's resolution (220^3 nodes, 1280 triangles),
+// bound by their FP32 instructions. On a closed mesh the winding number changes
+// only across the surface, so a cube of nodes that stays clear of the surface
+// by more than the threshold has one answer, its centre's: k_bake_cubes decides
+// cubes of 8^3, 4^3 and 2^3 nodes by their centres, each level only inside the
+// cubes the one before left mixed, k_bake_nodes the nodes of the 2^3 cubes that
+// are still mixed, with k_bake_mass's test, and k_bake_fill writes the grid:
+// 6e8 tests in place of 1.4e10, and the same masses. Measured, the whole
+// call: 69 -> 5.7 ms (220^3 nodes, 1280 triangles), 269 -> 19 ms with 5120
+// triangles, 2.1 -> 0.84 ms (100^3, 320). Meshes that are not closed, where the
+// winding number is no integer, keep k_bake_mass.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
 
+#include <unordered_map>
 #include <vector>
 
 #include "esf_common.cuh"
@@ -90,27 +101,18 @@ __device__ float tri_solid_angle(const float3 p, const float3 a, const float3 b,
   return 2.0f * atan2f(det, den);
 }
 
-__global__ void k_bake_mass(int X, int Y, int Z, double dh, double ox, double oy, double oz,
-                            const float* __restrict__ tri, int ntri, double rx, double ry, double rz,
-                            double density,
-                            double* __restrict__ mass, unsigned long long* __restrict__ count) {
-  __shared__ float st[TILE * 9];
-  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)X * Y * Z;
-  const bool live = n < total;
-  const int x = live ? (int)(n % X) : 0, y = live ? (int)((n / X) % Y) : 0;
-  const int z = live ? (int)(n / ((long long)X * Y)) : 0;
-  // node position (the reference's pos = (x, y, z) dh + box_min, in FP64),
-  // then relative to the mesh's reference point in FP32
-  const float3 p = make_float3((float)(x * dh + ox - rx), (float)(y * dh + oy - ry),
-                               (float)(z * dh + oz - rz));
-  float best = 3.4e38f, angle = 0.0f;
+// Smallest squared distance to, and solid angle of, the triangles of one of
+// `slices` equal shares (share `part`), all threads of the block together.
+__device__ __forceinline__ void test_triangles(const float3 p, const float* __restrict__ tri, int ntri, int part,
+                                               int slices, float* st, float& best, float& angle) {
+  best = 3.4e38f;
+  angle = 0.0f;
   for (int t0 = 0; t0 < ntri; t0 += TILE) {
     const int nt = min(TILE, ntri - t0);
     __syncthreads();
     for (int i = threadIdx.x; i < nt * 9; i += blockDim.x) st[i] = tri[(long long)t0 * 9 + i];
     __syncthreads();
-    for (int k = 0; k < nt; k++) {
+    for (int k = part; k < nt; k += slices) {
       const float* q = st + 9 * k;
       const float3 a = make_float3(q[0], q[1], q[2]), b = make_float3(q[3], q[4], q[5]),
                    c = make_float3(q[6], q[7], q[8]);
@@ -118,14 +120,222 @@ __global__ void k_bake_mass(int X, int Y, int Z, double dh, double ox, double oy
       angle += tri_solid_angle(p, a, b, c);
     }
   }
-  if (!live) return;
-  // winding number angle / 4 pi: ~1 inside a closed outward-oriented mesh,
-  // ~0 outside
+}
+
+struct BakeGrid {
+  int X, Y, Z;
+  double dh, o[3], r[3];  // spacing, origin, the mesh's reference point
+};
+// position of node (x, y, z), halves allowed (the reference's pos = (x, y, z)
+// dh + box_min, in FP64), relative to the reference point in FP32
+__device__ __forceinline__ float3 node_at(const BakeGrid& g, double x, double y, double z) {
+  return make_float3((float)(x * g.dh + g.o[0] - g.r[0]), (float)(y * g.dh + g.o[1] - g.r[1]),
+                     (float)(z * g.dh + g.o[2] - g.r[2]));
+}
+// solid where the signed distance is at most dh / 2: the winding number
+// angle / 4 pi is ~1 inside a closed outward-oriented mesh, ~0 outside
+__device__ __forceinline__ bool solid_node(const BakeGrid& g, float best, float angle) {
   const bool inside = fabsf(angle) > 6.2831853f;
   const float sd = inside ? -sqrtf(best) : sqrtf(best);
-  const bool solid = sd <= (float)(0.5 * dh);
-  mass[n] = solid ? density : 0.0;
-  if (solid) atomicAdd(count, 1ull);
+  return sd <= (float)(0.5 * g.dh);
+}
+__device__ __forceinline__ void count_solid(bool solid, unsigned long long* count) {
+  const unsigned m = __ballot_sync(0xffffffffu, solid);
+  if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, (unsigned long long)__popc(m));
+}
+
+__global__ void k_bake_mass(BakeGrid g, const float* __restrict__ tri, int ntri, double density,
+                            double* __restrict__ mass, unsigned long long* __restrict__ count) {
+  __shared__ float st[TILE * 9];
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long total = (long long)g.X * g.Y * g.Z;
+  const bool live = n < total;
+  const int x = live ? (int)(n % g.X) : 0, y = live ? (int)((n / g.X) % g.Y) : 0;
+  const int z = live ? (int)(n / ((long long)g.X * g.Y)) : 0;
+  float best, angle;
+  test_triangles(node_at(g, x, y, z), tri, ntri, 0, 1, st, best, angle);
+  const bool solid = live && solid_node(g, best, angle);
+  if (live) mass[n] = solid ? density : 0.0;
+  count_solid(solid, count);
+}
+
+// ---- closed meshes, by cubes. Cubes of one level are numbered x fastest in a
+// grid of n[] cubes; level l + 1 has twice as many along each axis.
+enum BakeSide { B_OUT = 0, B_SOLID = 1, B_MIXED = 2 };
+struct BakeCubes {
+  int n[3];
+  unsigned char* side;  // per cube; written for the children of mixed cubes only
+  int* mixed;           // the mixed cubes
+  int* nMixed;
+};
+__device__ __forceinline__ int3 cube_xyz(const int n[3], int id) {
+  return make_int3(id % n[0], (id / n[0]) % n[1], id / (n[0] * n[1]));
+}
+// item i: cube i of the level (no parents), or child i % 8 of the parents'
+// mixed cube i / 8; its place, false if it lies beyond the grid
+__device__ __forceinline__ bool child_at(const BakeCubes* parents, const int n[3], long long i, int3& c) {
+  if (!parents) {
+    c = cube_xyz(n, (int)i);
+    return true;
+  }
+  const int k = (int)(i & 7);
+  c = cube_xyz(parents->n, parents->mixed[i >> 3]);
+  c = make_int3(2 * c.x + (k & 1), 2 * c.y + ((k >> 1) & 1), 2 * c.z + (k >> 2));
+  return true;
+}
+// One level: cubes of `edge` nodes a side. SLICES neighbouring threads share a
+// cube's triangles, so that the coarse levels' few cubes fill the GPU. `clear`:
+// a centre farther than this from the surface decides its cube.
+template <int SLICES>
+__global__ void __launch_bounds__(BT) k_bake_cubes(BakeGrid g, const float* __restrict__ tri, int ntri, int edge,
+                                                   const BakeCubes parents, int fromParents, const BakeCubes cubes,
+                                                   float clear) {
+  __shared__ float st[TILE * 9];
+  const long long items = fromParents ? 8LL * *parents.nMixed : (long long)cubes.n[0] * cubes.n[1] * cubes.n[2];
+  constexpr int PER = BT / SLICES;
+  for (long long i0 = (long long)blockIdx.x * PER; i0 < items; i0 += (long long)gridDim.x * PER) {
+    const long long i = i0 + threadIdx.x / SLICES;
+    int3 c = make_int3(0, 0, 0);
+    bool live = i < items && child_at(fromParents ? &parents : nullptr, cubes.n, i, c);
+    live = live && c.x * edge < g.X && c.y * edge < g.Y && c.z * edge < g.Z;
+    const double half = 0.5 * (edge - 1);
+    float best, angle;
+    test_triangles(node_at(g, c.x * edge + half, c.y * edge + half, c.z * edge + half), tri, ntri,
+                   threadIdx.x % SLICES, SLICES, st, best, angle);
+#pragma unroll
+    for (int o = SLICES / 2; o > 0; o >>= 1) {
+      best = fminf(best, __shfl_down_sync(0xffffffffu, best, o, SLICES));
+      angle += __shfl_down_sync(0xffffffffu, angle, o, SLICES);
+    }
+    if (!live || threadIdx.x % SLICES) continue;
+    const int id = c.x + cubes.n[0] * (c.y + cubes.n[1] * c.z);
+    // (not `best > ..`: a NaN distance leaves the cube mixed)
+    const int side = sqrtf(best) > clear ? (fabsf(angle) > 6.2831853f ? B_SOLID : B_OUT) : B_MIXED;
+    cubes.side[id] = (unsigned char)side;
+    if (side == B_MIXED) cubes.mixed[atomicAdd(cubes.nMixed, 1)] = id;
+  }
+}
+__global__ void __launch_bounds__(BT) k_bake_nodes(BakeGrid g, const float* __restrict__ tri, int ntri,
+                                                   const BakeCubes parents, unsigned char* __restrict__ node) {
+  __shared__ float st[TILE * 9];
+  const long long items = 8LL * *parents.nMixed;
+  for (long long i0 = (long long)blockIdx.x * BT; i0 < items; i0 += (long long)gridDim.x * BT) {
+    const long long i = i0 + threadIdx.x;
+    int3 c = make_int3(0, 0, 0);
+    const bool live = i < items && child_at(&parents, nullptr, i, c) && c.x < g.X && c.y < g.Y && c.z < g.Z;
+    float best, angle;
+    test_triangles(node_at(g, c.x, c.y, c.z), tri, ntri, 0, 1, st, best, angle);
+    if (live) node[c.x + (long long)g.X * (c.y + (long long)g.Y * c.z)] = solid_node(g, best, angle);
+  }
+}
+__global__ void __launch_bounds__(BT) k_bake_fill(BakeGrid g, const BakeCubes c8, const BakeCubes c4,
+                                                  const BakeCubes c2, const unsigned char* __restrict__ node,
+                                                  double density, double* __restrict__ mass,
+                                                  unsigned long long* __restrict__ count) {
+  const long long total = (long long)g.X * g.Y * g.Z;
+  for (long long n0 = (long long)blockIdx.x * BT; n0 < total; n0 += (long long)gridDim.x * BT) {
+    const long long n = n0 + threadIdx.x;
+    bool solid = false;
+    if (n < total) {
+      const int x = (int)(n % g.X), y = (int)((n / g.X) % g.Y), z = (int)(n / ((long long)g.X * g.Y));
+      int s = c8.side[x / 8 + c8.n[0] * (y / 8 + c8.n[1] * (z / 8))];
+      if (s == B_MIXED) s = c4.side[x / 4 + c4.n[0] * (y / 4 + c4.n[1] * (z / 4))];
+      if (s == B_MIXED) s = c2.side[x / 2 + c2.n[0] * (y / 2 + c2.n[1] * (z / 2))];
+      if (s == B_MIXED) s = node[n];
+      solid = s == B_SOLID;
+      mass[n] = solid ? density : 0.0;
+    }
+    count_solid(solid, count);
+  }
+}
+
+// Whether the triangles form a closed, consistently oriented surface (each edge
+// runs as often one way as the other, corners matched by position) of finite
+// corners: what makes the winding number an integer off the surface.
+bool closed_mesh(const double* v, int nv, const int* t, int nt) {
+  struct Pos {
+    double x, y, z;
+    bool operator==(const Pos& o) const { return x == o.x && y == o.y && z == o.z; }
+  };
+  struct Hash {
+    size_t operator()(const Pos& p) const {
+      size_t h = 0;
+      for (double d : {p.x, p.y, p.z}) {
+        d += 0.0;  // -0 and 0 are one place
+        uint64_t u;
+        memcpy(&u, &d, 8);
+        h = (h ^ (size_t)u) * 0x9e3779b97f4a7c15ull;
+        h ^= h >> 29;
+      }
+      return h;
+    }
+  };
+  std::unordered_map<Pos, int, Hash> place;
+  place.reserve(nv);
+  std::vector<int> at(nv);
+  for (int i = 0; i < nv; i++) {
+    const Pos p{v[3 * i], v[3 * i + 1], v[3 * i + 2]};
+    if (!isfinite(p.x) || !isfinite(p.y) || !isfinite(p.z)) return false;
+    at[i] = place.emplace(p, i).first->second;
+  }
+  std::unordered_map<uint64_t, int> net;  // (a, b), a < b: times run upwards less times run downwards
+  net.reserve((size_t)nt * 3 / 2 + 1);
+  for (int i = 0; i < nt; i++)
+    for (int k = 0; k < 3; k++) {
+      const uint32_t a = at[t[3 * i + k]], b = at[t[3 * i + (k + 1) % 3]];
+      if (a < b) net[(uint64_t)a << 32 | b]++;
+      else if (b < a) net[(uint64_t)b << 32 | a]--;
+    }
+  for (const auto& e : net)
+    if (e.second) return false;
+  return true;
+}
+
+// The three levels, the nodes and the fill, queued on the default stream;
+// scratch: bake_scratch bytes.
+struct BakePlan {
+  BakeCubes c[3];
+  size_t bytes;
+};
+BakePlan bake_plan(const BakeGrid& g, unsigned char* scratch) {
+  BakePlan p;
+  size_t at = 256;  // the levels' counters
+  for (int l = 0; l < 3; l++) {
+    const int edge = 8 >> l;
+    BakeCubes& c = p.c[l];
+    // twice the level before, so that children are found by doubling
+    if (l == 0) {
+      c.n[0] = (g.X + edge - 1) / edge;
+      c.n[1] = (g.Y + edge - 1) / edge;
+      c.n[2] = (g.Z + edge - 1) / edge;
+    } else {
+      for (int k = 0; k < 3; k++) c.n[k] = 2 * p.c[l - 1].n[k];
+    }
+    const size_t n = (size_t)c.n[0] * c.n[1] * c.n[2];
+    c.nMixed = reinterpret_cast<int*>(scratch + 16 * l);
+    c.mixed = reinterpret_cast<int*>(scratch + at);
+    at += (n * 4 + 255) / 256 * 256;
+    c.side = scratch + at;
+    at += (n + 255) / 256 * 256;
+  }
+  p.bytes = at;  // then one byte a node
+  return p;
+}
+void bake_by_cubes(const BakeGrid& g, const float* tri, int ntri, const BakePlan& p, unsigned char* node,
+                   double density, double* mass, unsigned long long* count) {
+  // a centre this far from the surface has its whole cube at least dh / 2 away
+  // on one side: the half diagonal of the cube's nodes, dh / 2, and a margin
+  // for FP32 positions
+  const double extent = fmax(fmax(g.X, g.Y), (double)g.Z) * g.dh + fmax(fmax(fabs(g.o[0]), fabs(g.o[1])), fabs(g.o[2]));
+  auto clear = [&](int edge) { return (float)((0.5 * (edge - 1) * 1.7320509 + 0.55) * g.dh + 2e-6 * extent); };
+  const long long total = (long long)g.X * g.Y * g.Z;
+  const int wide = 152 * 8;
+  ESF_COUNTED k_bake_cubes<8><<<wide, BT>>>(g, tri, ntri, 8, p.c[0], 0, p.c[0], clear(8));
+  ESF_COUNTED k_bake_cubes<4><<<wide, BT>>>(g, tri, ntri, 4, p.c[0], 1, p.c[1], clear(4));
+  ESF_COUNTED k_bake_cubes<1><<<wide, BT>>>(g, tri, ntri, 2, p.c[1], 1, p.c[2], clear(2));
+  ESF_COUNTED k_bake_nodes<<<wide, BT>>>(g, tri, ntri, p.c[2], node);
+  ESF_COUNTED k_bake_fill<<<(int)((total + BT - 1) / BT < wide ? (total + BT - 1) / BT : wide), BT>>>(
+      g, p.c[0], p.c[1], p.c[2], node, density, mass, count);
 }
 
 }  // namespace
@@ -174,23 +384,46 @@ extern "C" esf_status esf_rasterize_solid(const double* vertices, int num_vertic
     for (int c = 0; c < 3; c++)
       for (int k = 0; k < 3; k++)
         tri[9 * t + 3 * c + k] = (float)(vertices[3 * triangles[3 * t + c] + k] - (double)ref[k]);
+  BakeGrid g;
+  g.X = res[0];
+  g.Y = res[1];
+  g.Z = res[2];
+  g.dh = mass_dh;
+  for (int k = 0; k < 3; k++) {
+    g.o[k] = origin[k];
+    g.r[k] = (double)ref[k];
+  }
+  // (small grids: five launches of few blocks take as long as every test;
+  // 0.75 against 0.70 ms at 7e7 tests, 1.9 against 2.0 ms at 2.8e8)
+  bool cubes = (double)total * num_triangles >= 2e8 && total < (1LL << 31);
+  try {
+    cubes = cubes && closed_mesh(vertices, num_vertices, triangles, num_triangles);
+  } catch (...) {  // no host memory for the edges: the kernel that needs none
+    cubes = false;
+  }
+  const BakePlan size = bake_plan(g, nullptr);
   float* dTri = nullptr;
   double* dMass = nullptr;
   unsigned long long* dCount = nullptr;
+  unsigned char* scratch = nullptr;
   esf_status e = ESF_OK;
   if (cudaMalloc(&dTri, tri.size() * 4) != cudaSuccess || cudaMalloc(&dMass, total * 8) != cudaSuccess ||
-      cudaMalloc(&dCount, 8) != cudaSuccess) {
+      cudaMalloc(&dCount, 8) != cudaSuccess ||
+      (cubes && cudaMalloc(&scratch, size.bytes + total) != cudaSuccess)) {
     set_error("esf_rasterize_solid: device allocation failed");
     e = ESF_ERR_OOM;
   }
   if (!e && (cudaMemcpy(dTri, tri.data(), tri.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-             cudaMemset(dCount, 0, 8) != cudaSuccess))
+             cudaMemset(dCount, 0, 8) != cudaSuccess ||
+             (cubes && cudaMemset(scratch, 0, 256) != cudaSuccess)))
     e = ESF_ERR_CUDA;
   if (!e) {
-    const int blocks = (int)((total + BT - 1) / BT);
-    ESF_COUNTED k_bake_mass<<<blocks, BT>>>(res[0], res[1], res[2], mass_dh, origin[0], origin[1], origin[2],
-                                            dTri, num_triangles, (double)ref[0], (double)ref[1],
-                                            (double)ref[2], density, dMass, dCount);
+    if (cubes) {
+      bake_by_cubes(g, dTri, num_triangles, bake_plan(g, scratch), scratch + size.bytes, density, dMass, dCount);
+    } else {
+      const int blocks = (int)((total + BT - 1) / BT);
+      ESF_COUNTED k_bake_mass<<<blocks, BT>>>(g, dTri, num_triangles, density, dMass, dCount);
+    }
     if (cudaGetLastError() != cudaSuccess) e = ESF_ERR_CUDA;
   }
   unsigned long long cnt = 0;
@@ -201,6 +434,7 @@ extern "C" esf_status esf_rasterize_solid(const double* vertices, int num_vertic
   cudaFree(dTri);
   cudaFree(dMass);
   cudaFree(dCount);
+  cudaFree(scratch);
   if (!e && total_mass) *total_mass = (double)cnt * density * mass_dh * mass_dh * mass_dh;
   return e;
 }
