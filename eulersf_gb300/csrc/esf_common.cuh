@@ -113,6 +113,9 @@ struct PcrState {
   int pp;            // one-pass FP32 iteration: which buffer set holds r, t, q
   unsigned int ticket[4];
   double deltaPrev;  // one-pass double-float run: r.s of the iterate before the current one
+  // fixed-point FP64 stencil: bounds as high words (fixed_mag) of x, 1/m, the
+  // stencil's input r - alpha Ap/diag, and what phase A collects for that
+  unsigned int hx, hm, hv, hr, hq;
 };
 
 // Solid system layout ("sliced"): the 27 neighbour 3x3 blocks of solid node a,

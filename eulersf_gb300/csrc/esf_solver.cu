@@ -30,6 +30,7 @@
 #include <cudaTypedefs.h>
 
 #include "esf_common.cuh"
+#include "esf_fixed.cuh"
 
 namespace esf {
 
@@ -47,6 +48,19 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
   }
   return r;  // valid in thread 0
+}
+
+// The largest of a block's words into *out, by thread 0 (whose fence in
+// last_block_sum orders it); all threads call.
+__device__ __forceinline__ void block_max(unsigned mine, unsigned* out) {
+  __shared__ unsigned top;
+  __syncthreads();
+  if (threadIdx.x == 0) top = 0;
+  __syncthreads();
+  mine = __reduce_max_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0) atomicMax(&top, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(out, top);
 }
 
 // Deposit this block's partial; returns true in the block that arrives last,
@@ -110,6 +124,21 @@ __device__ __forceinline__ void finish_update(PcrState* st, double total) {
     } else if (!(st->iter > 0 && st->iter % 5 == 0)) {
       st->iter++;
     }
+  }
+  if (!(total == total)) {
+    st->status = ESF_ERR_NUMERIC;
+    st->done = 1;
+  }
+}
+
+// After the residual check of a reference solve (CONJUGATE_RESIDUAL.inl:162-171).
+__device__ __forceinline__ void finish_check(PcrState* st, double total) {
+  st->resid2 = total;
+  if (sqrt(total) < st->eps * sqrt(st->bnorm2)) {
+    st->converged = 1;
+    st->done = 1;
+  } else {
+    st->iter++;
   }
   if (!(total == total)) {
     st->status = ESF_ERR_NUMERIC;
@@ -329,16 +358,10 @@ __global__ void __launch_bounds__(NT) pressure_stencil(GridDev g, StencilArgs<T>
     PcrState* st = a.st;
     if (MODE == S_UPDATE) {
       finish_update(st, total);
-    } else if (MODE == S_CHECK || MODE == S_RESID64) {
+    } else if (MODE == S_CHECK) {
+      finish_check(st, total);
+    } else if (MODE == S_RESID64) {
       st->resid2 = total;
-      if (MODE == S_CHECK) {
-        if (sqrt(total) < st->eps * sqrt(st->bnorm2)) {
-          st->converged = 1;
-          st->done = 1;
-        } else {
-          st->iter++;
-        }
-      }
       if (!(total == total)) {
         st->status = ESF_ERR_NUMERIC;
         st->done = 1;
@@ -349,6 +372,7 @@ __global__ void __launch_bounds__(NT) pressure_stencil(GridDev g, StencilArgs<T>
   }
 }
 
+#include "esf_stencil_fixed.cuh"
 #include "esf_tma.cuh"
 #include "esf_pcr_fused.cuh"
 
@@ -359,7 +383,9 @@ constexpr int VT = 256;
 // [UPDR] r = r - alpha_{i-1} Ap_{i-1}/diag (the residual update of the
 // previous iteration); d = beta d + r; Ap = beta Ap + s;
 // alpha_i = delta / (Ap . Ap/diag).
-template <typename T, bool UPDR>
+// [BOUND] the largest |r| and |Ap/diag| too, for the scale of the fixed-point
+// stencil that follows.
+template <typename T, bool UPDR, bool BOUND = false>
 __global__ void __launch_bounds__(VT) pcr_phase_a(long long n, T* d, T* r, T* Ap, const T* s,
                                                   const T* invd, double* partial, PcrState* st) {
   __shared__ double sred[32];
@@ -371,6 +397,7 @@ __global__ void __launch_bounds__(VT) pcr_phase_a(long long n, T* d, T* r, T* Ap
   const T beta = (T)st->beta;
   const T alpha = (T)st->alpha;
   T acc = 0;
+  unsigned hr = 0, hq = 0;
   // four independent element chains per thread keep enough loads in flight
   const long long stride = (long long)gridDim.x * VT;
   long long i = blockIdx.x * (long long)VT + threadIdx.x;
@@ -396,7 +423,12 @@ __global__ void __launch_bounds__(VT) pcr_phase_a(long long n, T* d, T* r, T* Ap
       T an = beta * a[u] + sv[u];
       d[j] = dn;
       Ap[j] = an;
-      acc += an * (an * iv[u]);
+      const T q = an * iv[u];
+      acc += an * q;
+      if constexpr (BOUND) {
+        hr = max(hr, fixed_mag(rv[u]));
+        hq = max(hq, fixed_mag(q));
+      }
     }
   }
   for (; i < n; i += stride) {
@@ -409,13 +441,26 @@ __global__ void __launch_bounds__(VT) pcr_phase_a(long long n, T* d, T* r, T* Ap
     T av = beta * a + s[i];
     d[i] = dv;
     Ap[i] = av;
-    acc += av * (av * iv);
+    const T q = av * iv;
+    acc += av * q;
+    if constexpr (BOUND) {
+      hr = max(hr, fixed_mag(rv));
+      hq = max(hq, fixed_mag(q));
+    }
+  }
+  if constexpr (BOUND) {
+    block_max(hr, &st->hr);
+    block_max(hq, &st->hq);
   }
   double bs = block_sum<VT>((double)acc, sred);
   double total;
   if (last_block_sum<VT>(bs, partial, &st->ticket[0], gridDim.x, &total, sred) &&
       threadIdx.x == 0) {
     st->alpha = (fabs(total) > 0.0) ? st->delta / total : total;
+    if constexpr (BOUND) {
+      st->hv = fixed_bound(__ldcg(&st->hr), __ldcg(&st->hq), st->alpha);
+      st->hr = st->hq = 0;
+    }
     if (!(total == total)) {
       st->status = ESF_ERR_NUMERIC;
       st->done = 1;
@@ -729,6 +774,13 @@ esf_status pressure_apply(const GridDev& g, const T* minv, const T* in, T* out, 
   a.in = in;
   a.minv = minv;
   a.out = out;
+  if constexpr (std::is_same<T, double>::value) {
+    if (fixed_pays(g)) {
+      launch_fixed<S_APPLY>(g, a, st);
+      ESF_LAUNCH_CHECK();
+      return ESF_OK;
+    }
+  }
   ESF_COUNTED pressure_stencil<T, S_APPLY><<<stencil_grid<T>(g), NT, 0, st>>>(g, a, stencil_cz(g));
   ESF_LAUNCH_CHECK();
   return ESF_OK;
@@ -965,11 +1017,13 @@ struct PressureKernels {
   double* partial;
   PcrState* st;
   const TmaMaps* tma = nullptr;  // FP32 only: TMA-staged update kernel
+  bool fixed = false;            // FP64 only: the stencil on integers
   void setup_warm(cudaStream_t cs) const {  // r = (b - Ax)/diag, ||b||; then s = Ar, delta
     StencilArgs<T> a;
     memset(&a, 0, sizeof a);
     a.in = x; a.b = b; a.r = r; a.invd = invd; a.minv = minv; a.partial = partial; a.st = st;
-    ESF_COUNTED pressure_stencil<T, S_RESID_INIT><<<stencil_grid<T>(g), NT, 0, cs>>>(g, a, stencil_cz(g));
+    if (!stencil<S_RESID_INIT>(a, cs))
+      ESF_COUNTED pressure_stencil<T, S_RESID_INIT><<<stencil_grid<T>(g), NT, 0, cs>>>(g, a, stencil_cz(g));
     ESF_COUNTED zero2<T><<<vec_blocks(g.R), VT, 0, cs>>>(g.R, d, Ap);
     update(cs);
   }
@@ -978,7 +1032,24 @@ struct PressureKernels {
     update(cs);
   }
   void phase_a(cudaStream_t cs) const {
+    if constexpr (std::is_same<T, double>::value) {
+      if (fixed) {
+        ESF_COUNTED pcr_phase_a<T, true, true><<<vec_blocks(g.R), VT, 0, cs>>>(g.R, d, r, Ap, s, invd, partial, st);
+        return;
+      }
+    }
     ESF_COUNTED pcr_phase_a<T, true><<<vec_blocks(g.R), VT, 0, cs>>>(g.R, d, r, Ap, s, invd, partial, st);
+  }
+  // the fixed-point stencil, where it is in use
+  template <int MODE>
+  bool stencil(const StencilArgs<T>& a, cudaStream_t cs) const {
+    if constexpr (std::is_same<T, double>::value) {
+      if (fixed) {
+        launch_fixed<MODE>(g, a, cs);
+        return true;
+      }
+    }
+    return false;
   }
   void update(cudaStream_t cs) const {
     if constexpr (std::is_same<T, float>::value) {
@@ -993,12 +1064,14 @@ struct PressureKernels {
     memset(&a, 0, sizeof a);
     a.x = x; a.d = d; a.r = r; a.Ap = Ap; a.invd = invd; a.minv = minv; a.out = s;
     a.partial = partial; a.st = st;
+    if (stencil<S_UPDATE>(a, cs)) return;
     ESF_COUNTED pressure_stencil<T, S_UPDATE><<<stencil_grid<T>(g), NT, 0, cs>>>(g, a, stencil_cz(g));
   }
   void check(cudaStream_t cs) const {
     StencilArgs<T> a;
     memset(&a, 0, sizeof a);
     a.in = x; a.b = b; a.minv = minv; a.partial = partial; a.st = st;
+    if (stencil<S_CHECK>(a, cs)) return;
     ESF_COUNTED pressure_stencil<T, S_CHECK><<<stencil_grid<T>(g), NT, 0, cs>>>(g, a, stencil_cz(g));
   }
   // iterations [i0, i0+n) followed by the residual check of iteration
@@ -1091,6 +1164,23 @@ static esf_status init_state(PcrState* d, double eps, int maxIt, cudaStream_t st
   return ESF_OK;
 }
 
+// Whether an FP64 solve (state *st initialised) runs its stencil on integers: a
+// grid for which that pays, and bounds of x and 1/m, which this leaves in the
+// state, far from the ends of the exponent range.
+static esf_status fixed_start(const GridDev& g, const double* minv, const double* x, PcrState* st, cudaStream_t cs,
+                              bool* fixed) {
+  *fixed = false;
+  if (!fixed_pays(g)) return ESF_OK;
+  ESF_COUNTED fixed_bounds<<<vec_blocks(g.T), 256, 0, cs>>>(g, x, minv, &st->hx, &st->hm);
+  ESF_LAUNCH_CHECK();
+  unsigned h[2];
+  ESF_CUDA(cudaMemcpyAsync(h, &st->hx, sizeof h, cudaMemcpyDeviceToHost, cs));
+  ESF_CUDA(cudaStreamSynchronize(cs));
+  const int e = fixed_exp(h[0]) + fixed_exp(h[1]);
+  *fixed = h[0] < 0x7ff00000u && h[1] < 0x7ff00000u && e < 500 && (e > -500 || h[0] == 0);
+  return ESF_OK;
+}
+
 static esf_status batched_inner_solve(PressureWork* w, const GridDev& g, cudaStream_t st, PcrState* out);
 static bool batching_pays(PressureWork* w);
 static esf_status df_buffers(PressureWork* w, const GridDev& g);
@@ -1121,7 +1211,12 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
   // per iteration replayed as graphs, true-residual check every 5th.
   auto fp64_solve = [&](int itCap, PcrState* out) -> esf_status {
     PressureKernels<double> k{g, minv64, w->invd, b, x, w->r, w->d, w->Ap, w->s, w->partial, w->st};
-    const void* key[8] = {minv64, diag64, b, x, nullptr, nullptr, nullptr, nullptr};
+    {
+      esf_status e = init_state(w->st, eps, itCap, st);
+      if (!e) e = fixed_start(g, minv64, x, w->st, st, &k.fixed);
+      if (e) return e;
+    }
+    const void* key[8] = {minv64, diag64, b, x, k.fixed ? w : nullptr, nullptr, nullptr, nullptr};
     bool rebuild = !w->graphsFor64 || memcmp(key, w->keyA, sizeof key) != 0;
     if (rebuild) {
       esf_status e = capture(w->capStream, k, true, true, &w->gFirst, &w->kFirst);
@@ -1131,8 +1226,6 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
       memcpy(w->keyA, key, sizeof key);
       w->graphsFor64 = true;
     }
-    esf_status e = init_state(w->st, eps, itCap, st);
-    if (e) return e;
     return run_graph_solve(w->hst, w->ev, w->st, w->gFirst, w->gChunk, w->kFirst, w->kChunk, itCap, st, out);
   };
   if (precision == ESF_FP64) {
@@ -2726,6 +2819,10 @@ esf_status pressure_solve_static(void* scratch, const GridDev& g, const double* 
     if (e) return e;
   }
   PressureKernels<double> k{g, minv, invd, b, x, r, d, Ap, s, partial, state};
+  {
+    esf_status e = fixed_start(g, minv, x, state, st, &k.fixed);
+    if (e) return e;
+  }
   k.setup_warm(st);
   k.chunk(st, 6, true);
   ESF_LAUNCH_CHECK();

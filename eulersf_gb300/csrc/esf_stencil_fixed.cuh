@@ -1,0 +1,361 @@
+// The FP64 pressure stencil on integers (esf_fixed.cuh). Included by
+// esf_solver.cu inside namespace esf after pressure_stencil, whose modes and
+// arguments it shares.
+//
+// A warp owns 32 cell columns (30 of them its output, one halo column a side)
+// and RY output rows, and marches along z over a chunk of cz layers with
+// everything in registers: the previous layer's values, the node rows' products
+// of the layer below, and row by row the sums; neighbours along x come by
+// shuffle. The next layer's inputs are on their way into shared memory
+// (cp.async, zero-filled outside the grid, each lane reading back only what it
+// fetched) while a layer is computed; there is no barrier.
+//   cell row:  P = v(k-1) + v(k), Q = v(k-1) - v(k); with the next column's P', Q':
+//              P - P', P + P', Q + Q'
+//   node row (between two cell rows):  J^T v = ((P-P') + (P-P')+, (P+P') - (P+P')+,
+//              (Q+Q') + (Q+Q')+), times 1/m; A, B, C = with the layer below's
+//   cell:      (A + C - B) + (C - A - B)' of the lower node row plus
+//              (A + C + B) + (C - A + B)' of the upper (' of the column before)
+//
+// Bound: instruction issue (192^3 UPDATE: 127 M warp instructions, half a one a
+// cycle and scheduler, its three warps waiting on their own chains; DRAM at a
+// third). Measured against pressure_stencil<double>, whose bound is the FP64
+// pipe: product 32^3 19.1 -> 8.1 us, 64^3 29.5 -> 17.6, 128^3 159 -> 65,
+// 161x127x190 343 -> 104, 256^3 1154 -> 377; solve iteration (phase A included)
+// 34.7 -> 21, 57.8 -> 43, 260 -> 142, 499 -> 218, 1749 -> 800 us. Error of a
+// product against extended precision: 3/4 of the FP64 kernel's (2-norm).
+#pragma once
+
+constexpr int FX_T = 128;              // threads a block: four warps, stacked along y
+constexpr int FX_W = FX_T / 32, FX_COLS = 30;
+constexpr long long FX_MAX_BLOCKS = 16384;  // the static solve's partial sums; ESF_MAX_PARTIALS is more
+// values a lane fetches for a layer: the stencil's input rows (UPDATE: r, Ap
+// and 1/diag), the node rows' 1/m, and for UPDATE the own rows' x and d
+template <int MODE, int RY>
+__host__ __device__ constexpr int fx_slots() {
+  return (MODE == S_UPDATE ? 3 : 1) * (RY + 2) + (RY + 1) + (MODE == S_UPDATE ? 2 * RY : 0);
+}
+template <int MODE, int RY>
+__host__ __device__ constexpr int fx_smem() {
+  return 2 * fx_slots<MODE, RY>() * FX_T * 8;
+}
+// 8 bytes from global to shared memory, or zeros
+__device__ __forceinline__ void fetch8(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(in ? 8 : 0)
+               : "memory");
+}
+
+__device__ __forceinline__ Fix shfl_down(Fix a) {
+  return Fix{__shfl_down_sync(0xffffffffu, a.l0, 1), __shfl_down_sync(0xffffffffu, a.l1, 1),
+             __shfl_down_sync(0xffffffffu, a.l2, 1)};
+}
+__device__ __forceinline__ Fix shfl_up(Fix a) {
+  return Fix{__shfl_up_sync(0xffffffffu, a.l0, 1), __shfl_up_sync(0xffffffffu, a.l1, 1),
+             __shfl_up_sync(0xffffffffu, a.l2, 1)};
+}
+
+// (J diag(1/m) J^T v) of one cell in FP64, in pressure_stencil's order, from
+// memory: the warps whose values do not fit a scale (NaN, infinities, negative
+// 1/m, the ends of the exponent range).
+__device__ double stencil_cell_direct(const GridDev& g, const double* v, const double* minv, int x, int y, int z) {
+  auto at = [&](int i, int j, int k) {
+    return i >= 0 && j >= 0 && k >= 0 && i < g.cX && j < g.cY && k < g.cZ
+               ? v[i + (long long)j * g.cX + (long long)k * g.cslab] : 0.0;
+  };
+  double m[2][2][2][3];
+  for (int dz = 0; dz < 2; dz++)
+    for (int dy = 0; dy < 2; dy++)
+      for (int dx = 0; dx < 2; dx++) {
+        const int i = x + dx, j = y + dy, k = z + dz;  // node; its cells are i-1..i, j-1..j, k-1..k
+        double p[2][2], q[2][2];
+        for (int b = 0; b < 2; b++)
+          for (int a = 0; a < 2; a++) {
+            const double lo = at(i - 1 + a, j - 1 + b, k - 1), hi = at(i - 1 + a, j - 1 + b, k);
+            p[b][a] = lo + hi;
+            q[b][a] = lo - hi;
+          }
+        const bool inside = i > 0 && j > 0 && k > 0 && i < g.X - 1 && j < g.Y - 1 && k < g.Z - 1;
+        const double mi = inside ? minv[i + (long long)j * g.X + (long long)k * g.slab] : 0.0;
+        m[dz][dy][dx][0] = ((p[0][0] + p[1][0]) - (p[0][1] + p[1][1])) * mi;
+        m[dz][dy][dx][1] = ((p[0][0] + p[0][1]) - (p[1][0] + p[1][1])) * mi;
+        m[dz][dy][dx][2] = ((q[0][0] + q[0][1]) + (q[1][0] + q[1][1])) * mi;
+      }
+  double A[2][2], B[2][2], C[2][2];
+  for (int dy = 0; dy < 2; dy++)
+    for (int dx = 0; dx < 2; dx++) {
+      A[dy][dx] = m[0][dy][dx][0] + m[1][dy][dx][0];
+      B[dy][dx] = m[0][dy][dx][1] + m[1][dy][dx][1];
+      C[dy][dx] = m[1][dy][dx][2] - m[0][dy][dx][2];
+    }
+  return ((A[0][1] + A[1][1]) - (A[0][0] + A[1][0])) + ((B[1][0] + B[1][1]) - (B[0][0] + B[0][1])) +
+         ((C[0][0] + C[0][1]) + (C[1][0] + C[1][1]));
+}
+
+// The bound of v = r - alpha Ap/diag from the largest |r| and |Ap/diag|, as a
+// high word (fixed_mag); what lies below the scale's range gets its lowest.
+__device__ __forceinline__ unsigned fixed_bound(unsigned hr, unsigned hq, double alpha) {
+  const double b = from_words(hr, ~0u) + fabs(alpha) * from_words(hq, ~0u);
+  return fixed_mag(b * 1.0000001);
+}
+template <int MODE, int RY>
+__global__ void __launch_bounds__(FX_T, 3) pressure_stencil_fixed(GridDev g, StencilArgs<double> a, int cz) {
+  extern __shared__ double ring[];  // [2][slots][FX_T]
+  __shared__ double sred[32];
+  if (MODE != S_APPLY && a.st->done) return;
+  constexpr int SLOTS = fx_slots<MODE, RY>();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cx = blockIdx.x * FX_COLS + lane - 1;  // this lane's cell column; its node column is cx + 1
+  const int y0 = (blockIdx.y * FX_W + warp) * RY;
+  const int z0 = blockIdx.z * cz, z1 = min(z0 + cz, g.cZ);
+  const bool col = cx >= 0 && cx < g.cX;
+  const bool own = col && lane >= 1 && lane <= FX_COLS;
+  const bool nodeCol = cx >= 0 && cx < g.cX - 1;
+  const double alpha = MODE == S_UPDATE ? a.st->alpha : 0.0;
+  double acc = 0.0;
+  unsigned hx = 0;  // UPDATE: largest new x; RESID_INIT: largest r
+  auto cell = [&](int y, int z) { return cx + (long long)y * g.cX + (long long)z * g.cslab; };
+  auto node = [&](int y, int z) { return cx + 1 + (long long)y * g.X + (long long)z * g.slab; };
+  if (y0 < g.cY) {
+    unsigned hv, hm;
+    if (MODE == S_APPLY) {  // this warp's own values
+      hv = hm = 0;
+      // (four layers' loads in flight: one layer at a time the scan took as long
+      // as the march)
+      for (int z = z0 - 1; z <= z1; z += 4) {
+        double v[4][RY + 2], m[4][RY + 1];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+          for (int j = 0; j < RY + 2; j++) {
+            const int y = y0 - 1 + j, zk = z + k;
+            v[k][j] = col && y >= 0 && y < g.cY && zk >= 0 && zk < g.cZ && zk <= z1 ? a.in[cell(y, zk)] : 0.0;
+            if (j > 0) m[k][j - 1] = nodeCol && y > 0 && y < g.Y - 1 && zk > 0 && zk <= z1 && zk < g.Z - 1 ? a.minv[node(y, zk)] : 0.0;
+          }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+          for (int j = 0; j < RY + 2; j++) {
+            hv = max(hv, fixed_mag1(v[k][j]));
+            if (j > 0) hm = max(hm, hi_word(m[k][j - 1]) | (lo_word(m[k][j - 1]) ? 1u : 0u));
+          }
+      }
+      hv = __reduce_max_sync(0xffffffffu, hv);
+      hm = __reduce_max_sync(0xffffffffu, hm);
+    } else {
+      hm = a.st->hm;
+      hv = MODE == S_UPDATE ? a.st->hv : a.st->hx;
+    }
+    const int Em = fixed_exp(hm), Ev = fixed_scale(hv, hm);
+    const bool ok = fixed_ok(hv, hm);
+    if (MODE == S_APPLY && (!ok || fixed_low(hv, hm))) {
+      for (int z = z0; z < z1; z++)
+        for (int j = 0; j < RY; j++)
+          if (own && y0 + j < g.cY) a.out[cell(y0 + j, z)] = stencil_cell_direct(g, a.in, a.minv, cx, y0 + j, z);
+      return;
+    }
+    // (in a solve, a scale that does not fit is a value on its way to infinity,
+    // or NaN: the sums say so)
+    if (!ok) acc = from_words(0x7ff80000u, 0u);
+    Fix prev[RY + 2], mpx[RY + 1], mpy[RY + 1], mpz[RY + 1];
+    double vo[RY];  // UPDATE: v of the own rows, layer kk - 1
+#pragma unroll
+    for (int j = 0; j < RY + 2; j++) prev[j] = Fix{0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < RY + 1; j++) mpx[j] = mpy[j] = mpz[j] = Fix{0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < RY; j++) vo[j] = 0.0;
+    auto fetch = [&](int kk) {
+      double* q = ring + ((kk & 1) * SLOTS) * FX_T + threadIdx.x;
+      const bool layer = kk >= 0 && kk < g.cZ;
+      int slot = 0;
+#pragma unroll
+      for (int j = 0; j < RY + 2; j++) {
+        const int y = y0 - 1 + j;
+        const bool in = layer && col && y >= 0 && y < g.cY;
+        const long long c = in ? cell(y, kk) : 0;
+        if (MODE == S_UPDATE) {
+          fetch8(q + FX_T * slot++, a.r + c, in);
+          fetch8(q + FX_T * slot++, a.Ap + c, in);
+          fetch8(q + FX_T * slot++, a.invd + c, in);
+        } else {
+          fetch8(q + FX_T * slot++, a.in + c, in);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < RY + 1; j++) {
+        const int ny = y0 + j;
+        const bool in = nodeCol && ny > 0 && ny < g.Y - 1 && kk > 0 && kk < g.Z - 1;
+        fetch8(q + FX_T * slot++, a.minv + (in ? node(ny, kk) : 0), in);
+      }
+      if (MODE == S_UPDATE)
+#pragma unroll
+        for (int j = 0; j < RY; j++) {
+          const bool in = own && y0 + j < g.cY && kk >= z0 && kk < z1;
+          const long long c = in ? cell(y0 + j, kk) : 0;
+          fetch8(q + FX_T * slot++, a.x + c, in);
+          fetch8(q + FX_T * slot++, a.d + c, in);
+        }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (ok) fetch(z0 - 1);
+    for (int kk = z0 - 1; kk <= z1 && ok; kk++) {
+      if (kk < z1) {
+        fetch(kk + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      const double* q = ring + ((kk & 1) * SLOTS) * FX_T + threadIdx.x;
+      constexpr int IN = (MODE == S_UPDATE ? 3 : 1), M0 = IN * (RY + 2), X0 = M0 + RY + 1;
+      double v[RY + 2];
+#pragma unroll
+      for (int j = 0; j < RY + 2; j++)
+        v[j] = MODE == S_UPDATE
+                   ? upd_r(q[FX_T * (3 * j)], alpha, q[FX_T * (3 * j + 1)], q[FX_T * (3 * j + 2)])
+                   : q[FX_T * j];
+      if (MODE == S_UPDATE && kk >= z0 && kk < z1) {
+#pragma unroll
+        for (int j = 0; j < RY; j++)
+          if (own && y0 + j < g.cY) {
+            const double xn = q[FX_T * (X0 + 2 * j)] + alpha * q[FX_T * (X0 + 2 * j + 1)];
+            a.x[cell(y0 + j, kk)] = xn;
+            hx = max(hx, fixed_mag(xn));
+          }
+      }
+      Fix dp, xp, xq, vp = Fix{0, 0, 0};  // of the cell row before; a + c - b of the node row before
+#pragma unroll
+      for (int j = 0; j < RY + 2; j++) {
+        const Fix f = fixed_from(v[j], Ev);
+        const Fix P = prev[j] + f, Q = prev[j] - f;
+        prev[j] = f;
+        if (kk < z0) continue;
+        const Fix pn = shfl_down(P), qn = shfl_down(Q);
+        const Fix dp1 = P - pn, xp1 = P + pn, xq1 = Q + qn;
+        if (j > 0) {
+          const NodeFactor m = factor_from(q[FX_T * (M0 + j - 1)], Em);
+          const Fix mx = fixed_mul(dp + dp1, m), my = fixed_mul(xp - xp1, m), mz = fixed_mul(xq + xq1, m);
+          if (kk > z0) {
+            const Fix A = mpx[j - 1] + mx, B = mpy[j - 1] + my, C = mz - mpz[j - 1];
+            const Fix CA = C - A, AC = A + C;
+            const Fix up = shfl_up(CA + B), um = shfl_up(CA - B);
+            if (j > 1) {  // output cell row y0 + j - 2, layer kk - 1
+              const double o = fixed_to((vp + up) + (AC + B), Ev + Em);
+              if (own && y0 + j - 2 < g.cY) {
+                const long long c = cell(y0 + j - 2, kk - 1);
+                if (MODE == S_APPLY) {
+                  a.out[c] = o;
+                } else if (MODE == S_UPDATE) {
+                  a.out[c] = o;
+                  acc += vo[j - 2] * o;
+                } else if (MODE == S_CHECK) {
+                  const double e = o - a.b[c];
+                  acc += e * e;
+                } else if (MODE == S_RESID_INIT) {
+                  const double bb = a.b[c], rn = (bb - o) * a.invd[c];
+                  a.r[c] = rn;
+                  hx = max(hx, fixed_mag(rn));
+                  acc += bb * bb;
+                }
+              }
+            }
+            vp = (AC - B) + um;
+          }
+          mpx[j - 1] = mx;
+          mpy[j - 1] = my;
+          mpz[j - 1] = mz;
+        }
+        dp = dp1;
+        xp = xp1;
+        xq = xq1;
+      }
+      if (MODE == S_UPDATE)
+#pragma unroll
+        for (int j = 0; j < RY; j++) vo[j] = v[j + 1];
+    }
+  }
+  if (MODE == S_APPLY) return;
+  if (MODE == S_UPDATE || MODE == S_RESID_INIT) block_max(hx, MODE == S_UPDATE ? &a.st->hx : &a.st->hr);
+  const double bs = block_sum<FX_T>(acc, sred);
+  const int nblocks = gridDim.x * gridDim.y * gridDim.z;
+  double total;
+  if (last_block_sum<FX_T>(bs, a.partial, &a.st->ticket[1], nblocks, &total, sred) && threadIdx.x == 0) {
+    PcrState* st = a.st;
+    if (MODE == S_UPDATE) {
+      finish_update(st, total);
+    } else if (MODE == S_CHECK) {
+      finish_check(st, total);
+    } else if (MODE == S_RESID_INIT) {
+      st->bnorm2 = total;
+      st->hv = fixed_bound(st->hr, 0u, 0.0);
+      st->hr = 0;
+    }
+  }
+}
+
+// Bounds a fixed-point solve starts from: the largest |x|, and the largest 1/m
+// of the interior nodes (a negative one's sign bit makes it the largest). The
+// words are zero before.
+__global__ void __launch_bounds__(256) fixed_bounds(GridDev g, const double* x, const double* minv, unsigned* hx,
+                                                    unsigned* hm) {
+  unsigned mx = 0, mm = 0;
+  const long long stride = (long long)gridDim.x * 256;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < g.R; i += stride) mx = max(mx, fixed_mag(x[i]));
+  for (long long n = blockIdx.x * 256LL + threadIdx.x; n < g.T; n += stride) {
+    const int i = (int)(n % g.X), j = (int)((n / g.X) % g.Y), k = (int)(n / g.slab);
+    if (i > 0 && j > 0 && k > 0 && i < g.X - 1 && j < g.Y - 1 && k < g.Z - 1) mm = max(mm, hi_word(minv[n]));
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  mm = __reduce_max_sync(0xffffffffu, mm);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(hx, mx);
+    atomicMax(hm, mm);
+  }
+}
+
+// Launch shape: rows a warp, and the z-chunk depth from the warps wanted an SM.
+// More rows share halo rows and conversions, fewer give small grids warps (solve
+// iteration, 2 against 4 rows: 32^3 22 and 26 us, 64^3 50 and 54, 96^3 87 and
+// 85, 256^3 equal, its product 431 and 377). Twelve warps an SM are resident;
+// chunks pay two extra layers each, so small grids take one wave of them and
+// large ones more, for the tail (12, 24, 48 warps: 64^3 54, 60, 60 us, 96^3 85,
+// 92, 99, 128^3 160, 146, 164, 161x127x190 287, 222, 240, 256^3 953, 850, 802).
+struct FixedShape {
+  int ry, cz;
+  dim3 grid;
+};
+static FixedShape fixed_shape(const GridDev& g) {
+  FixedShape s;
+  const int ry = s.ry = g.R < 600000 ? 2 : 4;
+  const int warps = g.R < 1500000 ? 12 : g.R < 8000000 ? 24 : 48;
+  const long long cols = (long long)((g.cX + FX_COLS - 1) / FX_COLS) * ((g.cY + ry - 1) / ry);
+  int n = (int)((warps * 152 + cols - 1) / cols);
+  n = n < 1 ? 1 : n > g.cZ ? g.cZ : n;
+  s.cz = (g.cZ + n - 1) / n;
+  s.grid = dim3((g.cX + FX_COLS - 1) / FX_COLS, (g.cY + FX_W * ry - 1) / (FX_W * ry), (g.cZ + s.cz - 1) / s.cz);
+  return s;
+}
+template <int MODE, int RY>
+static void launch_fixed_rows(const GridDev& g, const StencilArgs<double>& a, const FixedShape& s, cudaStream_t st) {
+  constexpr int smem = fx_smem<MODE, RY>();
+  static const cudaError_t attr = cudaFuncSetAttribute(pressure_stencil_fixed<MODE, RY>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  (void)attr;  // a refusal shows as the launch's error
+  ESF_COUNTED pressure_stencil_fixed<MODE, RY><<<s.grid, FX_T, smem, st>>>(g, a, s.cz);
+}
+template <int MODE>
+static void launch_fixed(const GridDev& g, const StencilArgs<double>& a, cudaStream_t st) {
+  const FixedShape s = fixed_shape(g);
+  if (s.ry == 2) launch_fixed_rows<MODE, 2>(g, a, s, st);
+  else launch_fixed_rows<MODE, 4>(g, a, s, st);
+}
+// Whether a grid's FP64 products and solves use it. It is the faster one at
+// every size and shape measured: 8^3 8.1 against 19.2 us a product, 20 against
+// 34 a solve iteration; 3x200x200 cells 9.5 and 19; 32x33x300 37 and 41. Below
+// 8192 cells, where a step is its launches, FP64 in pressure_stencil's order
+// stays, whose results to the last bit whole steps on such grids are compared
+// by. More blocks than the sums have room for stay too.
+static bool fixed_pays(const GridDev& g) {
+  if (g.R < 8192) return false;
+  const FixedShape s = fixed_shape(g);
+  return (long long)s.grid.x * s.grid.y * s.grid.z <= FX_MAX_BLOCKS && s.grid.y <= 65535 && s.grid.z <= 65535;
+}
