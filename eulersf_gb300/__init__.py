@@ -27,7 +27,7 @@ EXPORTS = [
     "esf_time_pressure_kernels", "esf_scene_footprint", "esf_server_create", "esf_server_submit",
     "esf_server_poll", "esf_server_wait", "esf_server_get_field", "esf_server_release",
     "esf_server_destroy", "esf_server_batch_stats", "esf_selftest_bounded_wait", "esf_rasterize_solid",
-    "esf_solid_load_rest_sdf", "esf_rest_sdf_query", "esf_svol_read",
+    "esf_solid_load_rest_sdf", "esf_rest_sdf_query", "esf_svol_read", "esf_release_workspaces",
 ]
 
 

@@ -170,6 +170,14 @@ esf_status pressure_apply(const GridDev& g, const T* minv, const T* in, T* out, 
 struct PressureWork;  // device work arrays of one pressure solve
 esf_status pressure_work_alloc(PressureWork** w, const GridDev& g, int mixed);
 void pressure_work_free(PressureWork* w);
+// a work for one call of the solver seam, and back when the call is done (idle:
+// nothing runs on it any more); see esf_solver.cu
+esf_status pressure_work_take(PressureWork** w, const GridDev& g, int mixed);
+void pressure_work_give(PressureWork* w, bool idle);
+// frees those waiting for a next call on the device (-1: on all); whether any were
+bool pressure_work_release_idle(int device);
+// a non-blocking stream of the work's own
+cudaStream_t pressure_work_stream(PressureWork* w);
 // Full pressure solve; x is the warm start / result. minv64 per node.
 esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv64,
                           const double* diag64, const double* b, double* x, double eps, int maxIt,

@@ -28,6 +28,7 @@
 namespace esf {
 void set_error(const char* fmt, ...);
 struct InnerBatcher;
+bool pressure_work_release_idle(int device);
 esf_status batcher_create(int device, InnerBatcher** out, bool autotune);
 void batcher_destroy(InnerBatcher* b);
 void batcher_stats(InnerBatcher* b, esf_batch_stats* out);
@@ -233,6 +234,7 @@ extern "C" esf_status esf_server_create(const esf_server_config* cfg, esf_server
   esf_server* s = new esf_server();
   cudaGetDevice(&s->device);
   size_t freeB = 0, totalB = 0;
+  esf::pressure_work_release_idle(s->device);
   cudaMemGetInfo(&freeB, &totalB);
   s->budget = (cfg && cfg->hbm_budget_bytes) ? cfg->hbm_budget_bytes : (size_t)(0.85 * (double)freeB);
   s->maxActive = (cfg && cfg->max_active > 0) ? cfg->max_active : 8;

@@ -17,6 +17,7 @@
 #include <mutex>
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <condition_variable>
 #include <deque>
 #include <map>
@@ -602,6 +603,14 @@ struct PressureWork {
   // inner solves handed to a batcher shared with other scenes or systems
   InnerBatcher* batcher;
   cudaEvent_t batchReady, batchDone;
+  // taken for one call (pressure_work_take): its FP64 graphs must not hold the
+  // caller's addresses, so they run on copies (up to kCopyCells; larger grids'
+  // iterations are launched one by one); and the place it was taken for
+  bool perCall;
+  double *m64, *b64, *x64;
+  int device;
+  unsigned long long ctx;
+  bool mixedBuffers;
 };
 
 // ---- FP32 vectors of the inner solves in compressible memory. They are
@@ -790,13 +799,8 @@ template esf_status pressure_apply<double>(const GridDev&, const double*, const 
 template esf_status pressure_apply<float>(const GridDev&, const float*, const float*, float*,
                                           cudaStream_t);
 
-esf_status pressure_work_alloc(PressureWork** out, const GridDev& g, int mixed) {
-  PressureWork* w = new PressureWork();
-  memset(w, 0, sizeof *w);
-  w->R = g.R;
-  w->T = g.T;
-  w->g = g;
-  size_t R = g.R;
+static esf_status work_buffers(PressureWork* w, const GridDev& g, int mixed) {
+  const size_t R = g.R;
   ESF_CUDA(cudaMalloc(&w->r, R * 8));
   ESF_CUDA(cudaMalloc(&w->d, R * 8));
   ESF_CUDA(cudaMalloc(&w->Ap, R * 8));
@@ -804,13 +808,21 @@ esf_status pressure_work_alloc(PressureWork** out, const GridDev& g, int mixed) 
   ESF_CUDA(cudaMalloc(&w->invd, R * 8));
   if (mixed) {
     w->mpitch = (g.X + 3) / 4 * 4;
+    // (mapping eleven vectors takes 2 ms; below 2 MB, the granularity, a work
+    // for one call does without, its vectors stay in L2 anyway)
+    const bool map = !w->perCall || R * 4 >= (2u << 20);
+    auto vec = [&](float** v, size_t bytes) -> esf_status {
+      if (map) return vec_alloc(&w->mapped, v, bytes);
+      ESF_CUDA(cudaMalloc(v, bytes));
+      return ESF_OK;
+    };
     float** vecs[] = {&w->x32, &w->r32, &w->d32, &w->Ap32, &w->s32, &w->invd32,
                       &w->b32, &w->r32b, &w->s32b, &w->Ap32b};
     for (float** v : vecs) {
-      esf_status e = vec_alloc(&w->mapped, v, R * 4);
+      esf_status e = vec(v, R * 4);
       if (e) return e;
     }
-    esf_status e = vec_alloc(&w->mapped, &w->minv32p, (size_t)w->mpitch * g.Y * g.Z * 4);
+    esf_status e = vec(&w->minv32p, (size_t)w->mpitch * g.Y * g.Z * 4);
     if (e) return e;
     ESF_CUDA(cudaMalloc(&w->minv32, g.T * 4));
   }
@@ -823,8 +835,26 @@ esf_status pressure_work_alloc(PressureWork** out, const GridDev& g, int mixed) 
   ESF_CUDA(cudaMallocHost(&w->hst, 8 * sizeof(PcrState)));
   ESF_CUDA(cudaStreamCreateWithFlags(&w->capStream, cudaStreamNonBlocking));
   for (int i = 0; i < 4; i++) ESF_CUDA(cudaEventCreateWithFlags(&w->ev[i], cudaEventDisableTiming));
+  return ESF_OK;
+}
+static esf_status work_alloc(PressureWork** out, const GridDev& g, int mixed, bool perCall) {
+  PressureWork* w = new PressureWork();
+  memset(w, 0, sizeof *w);
+  w->R = g.R;
+  w->T = g.T;
+  w->g = g;
+  w->perCall = perCall;
+  w->mixedBuffers = mixed != 0;
+  esf_status e = work_buffers(w, g, mixed);
+  if (e) {
+    pressure_work_free(w);
+    return e;
+  }
   *out = w;
   return ESF_OK;
+}
+esf_status pressure_work_alloc(PressureWork** out, const GridDev& g, int mixed) {
+  return work_alloc(out, g, mixed, false);
 }
 
 void pressure_work_free(PressureWork* w) {
@@ -835,6 +865,7 @@ void pressure_work_free(PressureWork* w) {
     vec_free(&w->mapped, v);
   cudaFree(w->minv32);
   cudaFree(w->edf);
+  for (double* v : {w->m64, w->b64, w->x64}) cudaFree(v);
   cudaFree(w->ddf);
   cudaFree(w->partial); cudaFree(w->st); cudaFree(w->st32); cudaFree(w->stT);
   if (w->hst) cudaFreeHost(w->hst);
@@ -851,6 +882,135 @@ void pressure_work_free(PressureWork* w) {
   if (w->batchDone) cudaEventDestroy(w->batchDone);
   delete w;
 }
+
+// ---- works of the solver seam. A call needs a work of its grid's shape for as
+// long as it runs; building one takes longer than many solves (allocations,
+// streams, events, the inner iteration's graph: of 64 systems of 32^3 78 of 87
+// ms). Those that calls are done with wait here for the next of the same
+// device, context, shape and precision. A work is one call's alone from take to
+// give, and is given back idle (its stream synchronised). Bounded: 1/128 of the
+// device's memory and kMaxIdle works, the longest unused leave first; all leave
+// where an allocation of the library fails, where a server looks how much
+// memory is free, and on esf_release_workspaces. Nothing in a work depends on a
+// caller's address or data.
+namespace {
+struct IdleWorks {
+  static constexpr int kMaxIdle = 256;
+  std::mutex m;
+  PressureWork* w[kMaxIdle];  // the longest unused first
+  int n = 0;
+  PressureWork* remove(int i) {
+    PressureWork* p = w[i];
+    for (int k = i + 1; k < n; k++) w[k - 1] = w[k];
+    n--;
+    return p;
+  }
+};
+IdleWorks& idle_works() {
+  static IdleWorks* p = new IdleWorks;  // never destroyed: the driver may be gone by then
+  return *p;
+}
+size_t work_bytes(const PressureWork* w) {
+  const size_t vec = w->mixedBuffers ? 11 * (size_t)w->R * 4 + (size_t)w->T * 4 : 0;
+  return (size_t)w->R * 40 + vec + (w->edf ? (size_t)w->R * 16 : 0) + (w->m64 ? (size_t)w->T * 24 : 0) +
+         ESF_MAX_PARTIALS * 8 + (1 << 20);
+}
+size_t idle_limit(int device) {
+  static std::atomic<size_t> known[64];
+  size_t unused = 0, total = device < 64 ? known[device].load() : 0;
+  if (total) return total / 128;
+  if (cudaMemGetInfo(&unused, &total) != cudaSuccess) return 0;
+  if (device < 64) known[device].store(total);
+  return total / 128;
+}
+}  // namespace
+static bool current_context_id(unsigned long long* id);
+
+bool pressure_work_release_idle(int device) {
+  IdleWorks& P = idle_works();
+  PressureWork* out[IdleWorks::kMaxIdle];
+  int n = 0;
+  {
+    std::lock_guard<std::mutex> g(P.m);
+    for (int i = 0; i < P.n;)
+      if (device < 0 || P.w[i]->device == device) out[n++] = P.remove(i);
+      else i++;
+  }
+  int dev = 0;
+  if (n) cudaGetDevice(&dev);
+  for (int i = 0; i < n; i++) {
+    unsigned long long id = 0;
+    cudaSetDevice(out[i]->device);
+    if (current_context_id(&id) && id == out[i]->ctx) pressure_work_free(out[i]);
+    else delete out[i];  // its context is gone, and its memory with it
+  }
+  if (n) cudaSetDevice(dev);
+  return n > 0;
+}
+
+esf_status pressure_work_take(PressureWork** out, const GridDev& g, int mixed) {
+  IdleWorks& P = idle_works();
+  int dev = 0;
+  unsigned long long id = 0;
+  ESF_CUDA(cudaGetDevice(&dev));
+  // (ESF_VMM_COMP is there to compare allocations: with it set each call has its own)
+  const bool known = current_context_id(&id) && !getenv("ESF_VMM_COMP");
+  if (known) {
+    std::lock_guard<std::mutex> lock(P.m);
+    for (int i = P.n - 1; i >= 0; i--) {
+      const PressureWork* w = P.w[i];
+      if (w->device == dev && w->ctx == id && w->mixedBuffers == (mixed != 0) && w->g.cX == g.cX &&
+          w->g.cY == g.cY && w->g.cZ == g.cZ) {
+        *out = P.remove(i);
+        return ESF_OK;
+      }
+    }
+  }
+  esf_status e = work_alloc(out, g, mixed, true);
+  if (e && pressure_work_release_idle(dev)) {
+    cudaGetLastError();
+    e = work_alloc(out, g, mixed, true);
+  }
+  if (!e) {
+    (*out)->device = dev;
+    (*out)->ctx = known ? id : 0;  // 0: not kept
+  }
+  return e;
+}
+
+void pressure_work_give(PressureWork* w, bool idle) {
+  if (!w) return;
+  const size_t limit = idle_limit(w->device);
+  size_t used = work_bytes(w);
+  if (!idle || !w->ctx || used > limit) {
+    pressure_work_free(w);
+    return;
+  }
+  pressure_work_set_batcher(w, nullptr);
+  IdleWorks& P = idle_works();
+  PressureWork* out[IdleWorks::kMaxIdle];
+  int n = 0;
+  {
+    std::lock_guard<std::mutex> lock(P.m);
+    for (int i = 0; i < P.n; i++)
+      if (P.w[i]->device == w->device) used += work_bytes(P.w[i]);
+    for (int i = 0; i < P.n && (used > limit || P.n == IdleWorks::kMaxIdle);) {
+      if (P.w[i]->device == w->device) {
+        used -= work_bytes(P.w[i]);
+        out[n++] = P.remove(i);
+      } else {
+        i++;
+      }
+    }
+    if (P.n < IdleWorks::kMaxIdle) P.w[P.n++] = w;
+    else out[n++] = w;
+  }
+  for (int i = 0; i < n; i++) {
+    if (out[i]->ctx == w->ctx) pressure_work_free(out[i]);
+    else delete out[i];
+  }
+}
+cudaStream_t pressure_work_stream(PressureWork* w) { return w->capStream; }
 
 // ---- tensor maps of the TMA update kernel
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -1113,21 +1273,20 @@ static esf_status capture(cudaStream_t cs, const K& k, bool first, bool warm, cu
   return ESF_OK;
 }
 
-// Runs one PCR solve from graphs; keeps up to 3 chunks in flight and polls
-// pinned copies of the device state.
-static esf_status run_graph_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst,
-                                  cudaGraphExec_t gFirst, cudaGraphExec_t gChunk,
-                                  unsigned long long kFirst, unsigned long long kChunk, int maxIt,
-                                  cudaStream_t st, PcrState* out) {
+// Runs one PCR solve by `chunk(first)`, which queues its set-up and first six
+// iterations or five more; keeps up to 3 chunks in flight and polls pinned
+// copies of the device state.
+template <typename Chunk>
+static esf_status run_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst, int maxIt, cudaStream_t st, PcrState* out,
+                            Chunk chunk) {
   const int inflight = 3;
   int launched = 0, waited = 0;
   const int maxChunks = maxIt / 5 + 3;
   bool done = false;
   while (!done) {
     if (launched < maxChunks) {
-      const bool first = launched == 0 && gFirst;
-      ESF_CUDA(cudaGraphLaunch(first ? gFirst : gChunk, st));
-      note_graph_replay(first ? kFirst : kChunk);
+      esf_status e = chunk(launched == 0);
+      if (e) return e;
       ESF_CUDA(cudaMemcpyAsync(&hst[launched % 4], dst, sizeof(PcrState), cudaMemcpyDeviceToHost, st));
       ESF_CUDA(cudaEventRecord(ev[launched % 4], st));
       launched++;
@@ -1149,6 +1308,19 @@ static esf_status run_graph_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst,
   ESF_CUDA(cudaStreamSynchronize(st));
   ESF_CUDA(cudaMemcpy(out, dst, sizeof(PcrState), cudaMemcpyDeviceToHost));
   return ESF_OK;
+}
+
+// The same from graphs (gFirst null: chunks only).
+static esf_status run_graph_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst,
+                                  cudaGraphExec_t gFirst, cudaGraphExec_t gChunk,
+                                  unsigned long long kFirst, unsigned long long kChunk, int maxIt,
+                                  cudaStream_t st, PcrState* out) {
+  return run_solve(hst, ev, dst, maxIt, st, out, [&](bool first) -> esf_status {
+    first = first && gFirst;
+    ESF_CUDA(cudaGraphLaunch(first ? gFirst : gChunk, st));
+    note_graph_replay(first ? kFirst : kChunk);
+    return ESF_OK;
+  });
 }
 
 static esf_status init_state(PcrState* d, double eps, int maxIt, cudaStream_t st, int inner = 0) {
@@ -1210,13 +1382,35 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
   // FP64 PCR from the warm start x (the reference's solvePCR): two kernels
   // per iteration replayed as graphs, true-residual check every 5th.
   auto fp64_solve = [&](int itCap, PcrState* out) -> esf_status {
-    PressureKernels<double> k{g, minv64, w->invd, b, x, w->r, w->d, w->Ap, w->s, w->partial, w->st};
+    // a graph takes 0.3 ms to build, a copy of these grids' vectors 10 us; one
+    // launch an iteration and kernel keeps up where a kernel runs 50 us, but
+    // not from the many threads of a batch of small systems
+    constexpr long long kCopyCells = 1 << 21;
+    const bool copies = w->perCall && g.R <= kCopyCells;
+    if (copies) {
+      if (!w->m64) ESF_CUDA(cudaMalloc(&w->m64, g.T * 8));
+      if (!w->b64) ESF_CUDA(cudaMalloc(&w->b64, g.R * 8));
+      if (!w->x64) ESF_CUDA(cudaMalloc(&w->x64, g.R * 8));
+      ESF_CUDA(cudaMemcpyAsync(w->m64, minv64, g.T * 8, cudaMemcpyDeviceToDevice, st));
+      ESF_CUDA(cudaMemcpyAsync(w->b64, b, g.R * 8, cudaMemcpyDeviceToDevice, st));
+      ESF_CUDA(cudaMemcpyAsync(w->x64, x, g.R * 8, cudaMemcpyDeviceToDevice, st));
+    }
+    const double *pm = copies ? w->m64 : minv64, *pb = copies ? w->b64 : b;
+    double* px = copies ? w->x64 : x;
+    PressureKernels<double> k{g, pm, w->invd, pb, px, w->r, w->d, w->Ap, w->s, w->partial, w->st};
     {
       esf_status e = init_state(w->st, eps, itCap, st);
-      if (!e) e = fixed_start(g, minv64, x, w->st, st, &k.fixed);
+      if (!e) e = fixed_start(g, pm, px, w->st, st, &k.fixed);
       if (e) return e;
     }
-    const void* key[8] = {minv64, diag64, b, x, k.fixed ? w : nullptr, nullptr, nullptr, nullptr};
+    if (w->perCall && !copies)
+      return run_solve(w->hst, w->ev, w->st, itCap, st, out, [&](bool first) -> esf_status {
+        if (first) k.setup_warm(st);
+        k.chunk(st, first ? 6 : 5, true);
+        ESF_LAUNCH_CHECK();
+        return ESF_OK;
+      });
+    const void* key[8] = {pm, w->invd, pb, px, k.fixed ? w : nullptr, nullptr, nullptr, nullptr};
     bool rebuild = !w->graphsFor64 || memcmp(key, w->keyA, sizeof key) != 0;
     if (rebuild) {
       esf_status e = capture(w->capStream, k, true, true, &w->gFirst, &w->kFirst);
@@ -1226,7 +1420,9 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
       memcpy(w->keyA, key, sizeof key);
       w->graphsFor64 = true;
     }
-    return run_graph_solve(w->hst, w->ev, w->st, w->gFirst, w->gChunk, w->kFirst, w->kChunk, itCap, st, out);
+    esf_status e = run_graph_solve(w->hst, w->ev, w->st, w->gFirst, w->gChunk, w->kFirst, w->kChunk, itCap, st, out);
+    if (copies && !e) ESF_CUDA(cudaMemcpyAsync(x, px, g.R * 8, cudaMemcpyDeviceToDevice, st));
+    return e;
   };
   if (precision == ESF_FP64) {
     PcrState h;

@@ -222,6 +222,11 @@ esf_status esf_params_default(const esf_grid* g, esf_params* p) {
 
 static esf_status dalloc(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes ? bytes : 8);
+  int dev = 0;
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess && pressure_work_release_idle(dev)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes ? bytes : 8);
+  }
   if (e != cudaSuccess) {
     set_error("cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
     return ESF_ERR_OOM;
@@ -331,6 +336,10 @@ extern "C" esf_status esf_create(const esf_grid* g, const esf_params* p, void* s
     cudaMemsetAsync(s->rhs, 0, R * 8, s->stream);
     cudaMemsetAsync(s->b1, 0, R * 8, s->stream);
     e = pressure_work_alloc(&s->pw, G, p->precision != ESF_FP64);
+    if (e == ESF_ERR_OOM && pressure_work_release_idle(s->device)) {
+      cudaGetLastError();
+      e = pressure_work_alloc(&s->pw, G, p->precision != ESF_FP64);
+    }
   }
   if (!e && cudaEventCreate(&s->e0) != cudaSuccess) e = ESF_ERR_CUDA;
   if (!e && cudaEventCreate(&s->e1) != cudaSuccess) e = ESF_ERR_CUDA;
@@ -1729,13 +1738,13 @@ extern "C" esf_status esf_pressure_solve(const esf_grid* g, const double* minv, 
   }
   GridDev G = grid_dev(g);
   PressureWork* w = nullptr;
-  TRY(pressure_work_alloc(&w, G, precision != ESF_FP64));
+  TRY(pressure_work_take(&w, G, precision != ESF_FP64));
   int it = 0, rf = 0, cv = 0;
   double rr = 0;
   esf_status e = pressure_solve(w, G, minv, diag, b, x, eps, maxIt, precision, 1e-4, 50, &it, &rr, &rf,
                                 &cv, (cudaStream_t)stream);
-  cudaStreamSynchronize((cudaStream_t)stream);
-  pressure_work_free(w);
+  const bool idle = cudaStreamSynchronize((cudaStream_t)stream) == cudaSuccess;
+  pressure_work_give(w, idle && (e == ESF_OK || e == ESF_ERR_NUMERIC));
   if (iters) *iters = it;
   if (relres) *relres = rr;
   return e;
@@ -1779,16 +1788,14 @@ extern "C" esf_status esf_pressure_solve_batch(int n, const esf_grid* grids, con
   // every system's work is attached before any solve starts, so systems of
   // one grid shape find each other in the batcher from their first inner solve
   std::vector<PressureWork*> works(n, nullptr);
-  std::vector<cudaStream_t> streams(n, nullptr);
+  std::vector<char> idle(n, 1);
   esf_status e = ESF_OK;
   for (int i = 0; i < n && !e; i++) {
-    if (cudaStreamCreateWithFlags(&streams[i], cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamWaitEvent(streams[i], start, 0) != cudaSuccess) {
+    e = pressure_work_take(&works[i], grid_dev(&grids[i]), precision != ESF_FP64);
+    if (!e && cudaStreamWaitEvent(pressure_work_stream(works[i]), start, 0) != cudaSuccess) {
       set_error("esf_pressure_solve_batch: %s", cudaGetErrorString(cudaGetLastError()));
       e = ESF_ERR_CUDA;
-      break;
     }
-    e = pressure_work_alloc(&works[i], grid_dev(&grids[i]), precision != ESF_FP64);
     if (!e && batcher) e = pressure_work_set_batcher(works[i], batcher);
   }
   if (!e) {
@@ -1801,20 +1808,20 @@ extern "C" esf_status esf_pressure_solve_batch(int n, const esf_grid* grids, con
         cudaSetDevice(dev);
         int rf = 0, cv = 0;
         st[i] = pressure_solve(works[i], grid_dev(&grids[i]), minv[i], diag[i], b[i], x[i], eps, maxIt,
-                               precision, 1e-4, 50, &it[i], &rr[i], &rf, &cv, streams[i]);
-        cudaStreamSynchronize(streams[i]);
+                               precision, 1e-4, 50, &it[i], &rr[i], &rf, &cv, pressure_work_stream(works[i]));
+        idle[i] = cudaStreamSynchronize(pressure_work_stream(works[i])) == cudaSuccess &&
+                  (st[i] == ESF_OK || st[i] == ESF_ERR_NUMERIC);
       });
     for (auto& t : threads) t.join();
-  }
-  for (int i = 0; i < n; i++) {
-    pressure_work_free(works[i]);
-    if (streams[i]) cudaStreamDestroy(streams[i]);
   }
   if (stats) {
     memset(stats, 0, sizeof *stats);
     if (batcher) batcher_stats(batcher, stats);
   }
-  batcher_destroy(batcher);
+  for (int i = 0; i < n; i++)
+    if (works[i]) pressure_work_set_batcher(works[i], nullptr);
+  batcher_destroy(batcher);  // (waits for its launches, which may still name a finished system's work)
+  for (int i = 0; i < n; i++) pressure_work_give(works[i], !e && idle[i]);
   cudaEventDestroy(start);
   for (int i = 0; i < n; i++) {
     if (iters) iters[i] = it[i];
@@ -1823,6 +1830,8 @@ extern "C" esf_status esf_pressure_solve_batch(int n, const esf_grid* grids, con
   }
   return e;
 }
+
+extern "C" void esf_release_workspaces(void) { pressure_work_release_idle(-1); }
 
 extern "C" esf_status esf_pressure_solve_static(const esf_grid* g, const double* minv,
                                                 const double* diag, const double* b, double* x,

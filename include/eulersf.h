@@ -280,6 +280,12 @@ esf_status esf_pressure_solve(const esf_grid* grid, const double* mass_inv_node,
                               double eps, int max_iterations, int precision,
                               int* iterations, double* rel_residual, void* stream);
 
+/* esf_pressure_solve and esf_pressure_solve_batch keep the workspaces of past
+ * calls for later calls on the same device with the same grid shape: at most
+ * 1/128 of the device's memory. This frees those that no call is using; the
+ * library does so itself before an allocation of its own fails. */
+void esf_release_workspaces(void);
+
 /* Batched solver seam: n independent pressure systems solved together, each
  * with its own grid, m^-1, diagonal, right-hand side and warm start (arrays of
  * n device pointers; iterations and rel_residual NULL or arrays of n). No
