@@ -1194,7 +1194,13 @@ struct PressureKernels {
   void phase_a(cudaStream_t cs) const {
     if constexpr (std::is_same<T, double>::value) {
       if (fixed) {
-        ESF_COUNTED pcr_phase_a<T, true, true><<<vec_blocks(g.R), VT, 0, cs>>>(g.R, d, r, Ap, s, invd, partial, st);
+        // one wave (76 registers: three blocks an SM): a block's sum costs as much
+        // of the FP64 pipe as eight rows of its threads. Against vec_blocks, which
+        // the FP64 stencil's solves keep for their bits, an iteration takes 36.4
+        // for 42.8 us at 64^3, 71 for 78 at 96^3, 133 for 142 at 128^3, 783 for
+        // 805 at 256^3 (two blocks an SM 36.3, 70, 136, 795; four 40, 75, 145, 828)
+        const int blocks = std::min(vec_blocks(g.R), 3 * 152);
+        ESF_COUNTED pcr_phase_a<T, true, true><<<blocks, VT, 0, cs>>>(g.R, d, r, Ap, s, invd, partial, st);
         return;
       }
     }

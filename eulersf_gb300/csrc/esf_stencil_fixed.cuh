@@ -21,7 +21,7 @@
 // third). Measured against pressure_stencil<double>, whose bound is the FP64
 // pipe: product 32^3 19.1 -> 8.1 us, 64^3 29.5 -> 17.6, 128^3 159 -> 65,
 // 161x127x190 343 -> 104, 256^3 1154 -> 377; solve iteration (phase A included)
-// 34.7 -> 21, 57.8 -> 43, 260 -> 142, 499 -> 218, 1749 -> 800 us. Error of a
+// 34.7 -> 21, 57.8 -> 36, 260 -> 133, 499 -> 215, 1749 -> 783 us. Error of a
 // product against extended precision: 3/4 of the FP64 kernel's (2-norm).
 #pragma once
 
