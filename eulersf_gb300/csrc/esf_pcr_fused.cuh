@@ -60,7 +60,16 @@ constexpr int FU_OFF_B = FU_OFF_A + TW_NP * NYN * 4;
 constexpr int FU_OFF_C = FU_OFF_B + TW_NP * NYN * 4;
 constexpr int FU_OFF_RED = (FU_OFF_C + TW_NP * NYN * 4 + 15) / 16 * 16;
 constexpr int FU_SMEM = FU_OFF_RED + 32 * 8;  // about 47 KB: four blocks per SM
+constexpr unsigned FU_LOOP_WAIT = 1u << 22;  // polls of a loop's block at its barrier, 1 to 2 s
 constexpr int FU_SUMS = 4;                    // delta, mu, nu, omega
+
+// (by their bits: an FP64 comparison is 100 cycles on the way to the next pass)
+__device__ __forceinline__ bool is_nan(double v) {
+  return (unsigned)(__double2hiint(v) & 0x7fffffff) + (__double2loint(v) != 0) > 0x7ff00000u;
+}
+__device__ __forceinline__ bool is_positive(double v) {
+  return __double_as_longlong(v) > 0 && !is_nan(v);
+}
 
 // Scalars after a fused pass: totals of (r', s'), (s', t'), (s', q), (Ap, q).
 __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu, double nu,
@@ -71,9 +80,9 @@ __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu,
     // the old r, recomputed for the new one
     const double beta = (st->deltaPrev > 0.0) ? dl / st->deltaPrev : 0.0;
     double den = mu + 2.0 * beta * nu + beta * beta * om;
-    if (!(den > 0.0)) den = mu;
+    if (!is_positive(den)) den = mu;
     st->beta = beta;
-    st->alpha = (den > 0.0) ? dl / den : 0.0;
+    st->alpha = is_positive(den) ? dl / den : 0.0;
     st->delta = dl;
     st->delta0 = dl;
     st->rebase = 0;
@@ -97,9 +106,9 @@ __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu,
   } else {
     const double beta = dl / st->delta;
     double den = mu + 2.0 * beta * nu + beta * beta * om;
-    if (!(den > 0.0)) den = mu;  // rounding guard; (Ap, Ap/diag) is positive
+    if (!is_positive(den)) den = mu;  // rounding guard; (Ap, Ap/diag) is positive
     st->beta = beta;
-    st->alpha = (den > 0.0) ? dl / den : 0.0;
+    st->alpha = is_positive(den) ? dl / den : 0.0;
     st->deltaPrev = st->delta;
     st->delta = dl;
     st->iter++;
@@ -109,12 +118,21 @@ __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu,
     }
   }
   st->pp ^= 1;
-  if (!(dl == dl) || !(mu == mu) || !(nu == nu) || !(om == om)) {
+  if (is_nan(dl) || is_nan(mu) || is_nan(nu) || is_nan(om)) {
     st->status = ESF_ERR_NUMERIC;
     st->done = 1;
   }
 }
 
+// (double)v; of a float by its bits where it is a normal number or zero: a
+// conversion takes as much of the FP64 pipe as an addition.
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+  const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
+  if (m - 0x00800000u < 0x7f000000u || m == 0u)
+    return __hiloint2double((int)((u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u)), (int)(m << 29));
+  return (double)v;
+}
 // Four block sums at once, each with block_sum's tree and so its bits: lane 8 j
 // of warp 0 gets sum j (its lanes 8 j .. 8 j + 7 do). The first two levels send
 // half of the values across instead of adding all four in every lane, after
@@ -122,20 +140,28 @@ __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu,
 // stage instead of 4 times 10, each 19 cycles of an SM's FP64 pipe and 63 of
 // latency. With the last block's four folds in one and its copy of the state
 // read beside them, a pass at 32^3 and 64^3, where it is a chain of latencies,
-// went from 18.6 and 18.9 us to 12.8 and 13.0, at 128^3 from 34.2 to 25.4, at
-// 256^3 from 134 to 124. sh: NT / 8 doubles.
+// went from 18.6 and 18.9 us to 12.4, at 128^3 from 34.2 to 24.5, at 256^3 from
+// 134 to 124.
+// Of a larger block the first NT threads' values count, and of those the first n
+// (the others' are 0, whose additions are left out a warp at a time); all call.
+// sh: NT / 8 doubles.
 template <typename V>
-__device__ __forceinline__ double block_sum4(const V (&v)[FU_SUMS], double* sh) {
+__device__ __forceinline__ double block_sum4(const V (&v)[FU_SUMS], double* sh, int n = NT) {
   static_assert(NT == 256 && FU_SUMS == 4, "eight warps, four sums: a lane for each");
   constexpr unsigned all = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const bool u16 = lane & 16, u8 = lane & 8;
-  const V s0 = __shfl_xor_sync(all, u16 ? v[0] : v[2], 16), s1 = __shfl_xor_sync(all, u16 ? v[1] : v[3], 16);
-  const double p0 = (double)(u16 ? v[2] : v[0]) + (double)s0, p1 = (double)(u16 ? v[3] : v[1]) + (double)s1;
-  double q = (u8 ? p1 : p0) + __shfl_xor_sync(all, u8 ? p0 : p1, 8);
-  for (int o = 4; o > 0; o >>= 1) q += __shfl_xor_sync(all, q, o);
   __syncthreads();
-  if ((lane & 7) == 0) sh[lane + w] = q;
+  if (threadIdx.x < NT) {
+    double q = 0;
+    if (w * 32 < n) {
+      const bool u16 = lane & 16, u8 = lane & 8;
+      const V s0 = __shfl_xor_sync(all, u16 ? v[0] : v[2], 16), s1 = __shfl_xor_sync(all, u16 ? v[1] : v[3], 16);
+      const double p0 = widen(u16 ? v[2] : v[0]) + widen(s0), p1 = widen(u16 ? v[3] : v[1]) + widen(s1);
+      q = (u8 ? p1 : p0) + __shfl_xor_sync(all, u8 ? p0 : p1, 8);
+      for (int o = 4; o > 0; o >>= 1) q += __shfl_xor_sync(all, q, o);
+    }
+    if ((lane & 7) == 0) sh[lane + w] = q;
+  }
   __syncthreads();
   double r = 0;
   if (w == 0) {
@@ -143,6 +169,21 @@ __device__ __forceinline__ double block_sum4(const V (&v)[FU_SUMS], double* sh) 
     for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(all, r, o);
   }
   return r;
+}
+// The sums of nb partials each, in block order, as block_sum4 leaves them. A
+// thread's first partial is taken as it is, the others added.
+__device__ __forceinline__ double fold4(const double* partial, int nb, double* sh) {
+  double f[FU_SUMS] = {0, 0, 0, 0};
+  const int tid = threadIdx.x;
+  if (tid < nb && tid < NT) {
+#pragma unroll
+    for (int h = 0; h < FU_SUMS; h++) f[h] = __ldcg(partial + h * nb + tid);
+    for (int q = tid + NT; q < nb; q += NT) {
+#pragma unroll
+      for (int h = 0; h < FU_SUMS; h++) f[h] += __ldcg(partial + h * nb + q);
+    }
+  }
+  return block_sum4(f, sh, nb < NT ? nb : NT);
 }
 
 // Double-float ("df") arithmetic on FP32 pairs (hi, lo), value hi + lo with
@@ -170,6 +211,15 @@ __device__ __forceinline__ float2 df_add_scaled(float2 e, float a, float2 d) {
   const float2 s = df_two_sum(e.x, ph);
   const float t = __fadd_rn(__fadd_rn(__fmaf_rn(a, d.y, pl), e.y), s.y);
   return df_two_sum(s.x, t);
+}
+
+// This block's four sums (of its first NT threads) into the partials.
+__device__ __forceinline__ void put4(const float (&sums)[FU_SUMS], double* partial, int nb, int bid, double* sh) {
+  const double ps = block_sum4(sums, sh);
+  if (threadIdx.x < 32) {
+    if ((threadIdx.x & 7) == 0) __stcg(partial + (threadIdx.x >> 3) * nb + bid, ps);
+    __syncwarp();
+  }
 }
 
 // One block's share of a pass: the 64 x 8-cell column (bx, by) over the cell
@@ -447,26 +497,17 @@ __device__ __forceinline__ void fused_pass(const GridDev& g, const FusedMaps& tm
   }
   // the four sums: block partials, folded in block order by the last block
   const float sums[FU_SUMS] = {sDl, sMu, sNu, sOm};
-  const double ps = block_sum4(sums, sred);
-  if (tid < 32) {
-    if ((tid & 7) == 0) {
-      partial[(tid >> 3) * nb + bid] = ps;
-      __threadfence();
-    }
-    __syncwarp();
-    if (tid == 0) amLast = atomicAdd(&st->ticket[1], 1u) + 1 == (unsigned)nb;
+  put4(sums, partial, nb, bid, sred);
+  if (tid == 0) {
+    unsigned t;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(&st->ticket[1]) : "memory");
+    amLast = t + 1 == (unsigned)nb;
   }
   __syncthreads();
   if (!amLast) return;
-  __threadfence();
   PcrState L;  // (on its way while the sums are folded)
   if (tid == 0) L = *st;
-  double f[FU_SUMS] = {0, 0, 0, 0};
-  for (int q = tid; q < nb; q += NT) {
-#pragma unroll
-    for (int h = 0; h < FU_SUMS; h++) f[h] += __ldcg(partial + h * nb + q);
-  }
-  const double total = block_sum4(f, sred);
+  const double total = fold4(partial, nb, sred);
   if (tid < 32) {
     const double tMu = __shfl_sync(0xffffffffu, total, 8), tNu = __shfl_sync(0xffffffffu, total, 16),
                  tOm = __shfl_sync(0xffffffffu, total, 24);

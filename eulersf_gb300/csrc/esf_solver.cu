@@ -376,6 +376,7 @@ __global__ void __launch_bounds__(NT) pressure_stencil(GridDev g, StencilArgs<T>
 #include "esf_stencil_fixed.cuh"
 #include "esf_tma.cuh"
 #include "esf_pcr_fused.cuh"
+#include "esf_pcr_flat.cuh"
 
 // ------------------------------------------------------- vector kernels
 constexpr int VT = 256;
@@ -592,6 +593,8 @@ struct PressureWork {
   float *r32b, *s32b, *Ap32b;
   FusedMaps fmaps;
   bool fusedOk;
+  FlatMaps flatMaps;  // of the loops, where a grid has them
+  bool flatOk;
   // ESF_MIXED_X64: the double-float correction and search direction
   // (allocated on first use) and the graph of its iteration chunk
   float *edf, *ddf;
@@ -1026,9 +1029,9 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// 3-D FP32 array [d][h][w] (w a multiple of 4), box bw x bh x 1, zero fill
+// 3-D FP32 array [d][h][w] (w a multiple of 4), box bw x bh x bd, zero fill
 static esf_status encode3d(CUtensorMap* m, const void* base, long long w, long long h, long long d,
-                           unsigned bw, unsigned bh) {
+                           unsigned bw, unsigned bh, unsigned bd = 1) {
   PFN_cuTensorMapEncodeTiled_v12000 fn = tensor_map_encoder();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
@@ -1036,7 +1039,7 @@ static esf_status encode3d(CUtensorMap* m, const void* base, long long w, long l
   }
   cuuint64_t dims[3] = {(cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)d};
   cuuint64_t strides[2] = {(cuuint64_t)w * 4, (cuuint64_t)w * h * 4};
-  cuuint32_t box[3] = {bw, bh, 1};
+  cuuint32_t box[3] = {bw, bh, bd};
   cuuint32_t es[3] = {1, 1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, es,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -1054,6 +1057,32 @@ enum Fp32Path {
   P32_TMA = 1,       // pcr_phase_a + pressure_update_tma (same bits as P32_REGISTER)
   P32_FUSED = 2      // pcr_iteration_fused: the whole iteration in one pass
 };
+
+// Whether a grid's iterations run in loops (pcr_loop_flat): chunks of FL_L layers
+// at most, and one block an SM for a pass (64^3 cells and less), the first
+// condition for the kernel's shared memory, the second for its barrier. Where
+// both hold it is the faster one (8.2 against 12.4 us an iteration at 64^3).
+// ESF_PRESSURE_KERNEL=pass takes a launch an iteration everywhere (for
+// comparison; same bits).
+static bool loop_fits(const GridDev& g) {
+  static const long long slots = [] {
+    int dev = 0, sms = 0, coop = 0, a = 0, b = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    auto fits = [](auto* kernel, int* per) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FL_SMEM) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, kernel, FL_G * NT, FL_SMEM) == cudaSuccess;
+    };
+    if (!coop || !fits(pcr_loop_flat<false>, &a) || !fits(pcr_loop_flat<true>, &b)) return 0LL;
+    return (long long)sms * (a < b ? a : b);
+  }();
+  const char* pick = getenv("ESF_PRESSURE_KERNEL");
+  if (pick && strcmp(pick, "pass") == 0) return false;
+  const int cz = fused_cz(g);
+  const dim3 gr = tma_grid(g, cz);
+  return cz <= FL_L && (long long)gr.x * gr.y * gr.z <= slots;
+}
 
 // Chooses the FP32 kernels for the mixed path. The TMA kernels need cell
 // rows that are a multiple of 4 floats (16-byte row strides); with them the
@@ -1125,6 +1154,21 @@ static esf_status prepare_tma(PressureWork* w, const GridDev& g, const double* m
     w->fmaps = m;
     w->fusedOk = true;
   }
+  if (!w->flatOk && loop_fits(g)) {
+    FlatMaps m;
+    esf_status e;
+    float* rs[2] = {w->r32, w->r32b};
+    float* ts[2] = {w->s32, w->s32b};
+    float* qs[2] = {w->Ap32, w->Ap32b};
+    for (int k = 0; k < 2; k++) {
+      if ((e = encode3d(&m.r[k], rs[k], g.cX, g.cY, g.cZ, TMA_HW, TMA_HH, FL_H))) return e;
+      if ((e = encode3d(&m.t[k], ts[k], g.cX, g.cY, g.cZ, TMA_HW, TMA_HH, FL_H))) return e;
+      if ((e = encode3d(&m.q[k], qs[k], g.cX, g.cY, g.cZ, TMA_HW, TMA_HH, FL_H))) return e;
+    }
+    if ((e = encode3d(&m.m, w->minv32p, w->mpitch, g.Y, g.Z, TMA_NW, TMA_NH, FL_L + 1))) return e;
+    w->flatMaps = m;
+    w->flatOk = true;
+  }
   *path = P32_FUSED;
   return ESF_OK;
 }
@@ -1147,6 +1191,24 @@ struct FusedKernels {
     }
     ESF_COUNTED pcr_iteration_fused<<<tma_grid(g, cz), NT, FU_SMEM, cs>>>(g, *tm, p, partial, st, cz);
   }
+  // iterations by pcr_loop_flat, FL_CHUNK a launch, where loop_fits
+  const FlatMaps* flat = nullptr;
+  const float* invd = nullptr;
+  bool loops() const { return flat && loop_fits(g); }
+  esf_status loop(cudaStream_t cs, int budget) const {
+    GridDev gd = g;
+    int cz = fused_cz(g);
+    FusedPtrs pt = p;
+    const float* iv = invd;
+    float *e = edf, *d = ddf;
+    double* pa = partial;
+    PcrState* s = st;
+    void* args[] = {&gd, const_cast<FlatMaps*>(flat), &pt, &iv, &e, &d, &pa, &s, &cz, &budget};
+    note_launch();
+    ESF_CUDA(cudaLaunchCooperativeKernel(edf ? (const void*)pcr_loop_flat<true> : (const void*)pcr_loop_flat<false>,
+                                         tma_grid(g, cz), dim3(FL_G * NT), args, FL_SMEM, cs));
+    return ESF_OK;
+  }
   // graph capture interface of PressureKernels (inner solves only)
   void setup_warm(cudaStream_t) const {}
   void setup_zero(cudaStream_t) const {}
@@ -1165,6 +1227,8 @@ static FusedKernels fused_kernels(PressureWork* w, const GridDev& g, PcrState* s
   k.p.d = w->d32;
   k.partial = w->partial;
   k.st = st;
+  k.flat = w->flatOk ? &w->flatMaps : nullptr;
+  k.invd = w->invd32;
   return k;
 }
 
@@ -1280,14 +1344,14 @@ static esf_status capture(cudaStream_t cs, const K& k, bool first, bool warm, cu
 }
 
 // Runs one PCR solve by `chunk(first)`, which queues its set-up and first six
-// iterations or five more; keeps up to 3 chunks in flight and polls pinned
+// iterations or five more (or `per`); keeps up to 3 chunks in flight and polls pinned
 // copies of the device state.
 template <typename Chunk>
 static esf_status run_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst, int maxIt, cudaStream_t st, PcrState* out,
-                            Chunk chunk) {
+                            Chunk chunk, int per = 5) {
   const int inflight = 3;
   int launched = 0, waited = 0;
-  const int maxChunks = maxIt / 5 + 3;
+  const int maxChunks = maxIt / per + 3;
   bool done = false;
   while (!done) {
     if (launched < maxChunks) {
@@ -1327,6 +1391,13 @@ static esf_status run_graph_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst,
     note_graph_replay(first ? kFirst : kChunk);
     return ESF_OK;
   });
+}
+
+// The one-pass iteration until the state is done: by loops, or by a graph.
+static esf_status run_fused(PressureWork* w, const FusedKernels& k, cudaGraphExec_t graph, unsigned long long kernels,
+                            int maxIt, cudaStream_t st, PcrState* out) {
+  if (!k.loops()) return run_graph_solve(w->hst, w->ev, k.st, nullptr, graph, 0, kernels, maxIt, st, out);
+  return run_solve(w->hst, w->ev, k.st, maxIt, st, out, [&](bool) { return k.loop(st, FL_CHUNK); }, FL_CHUNK);
 }
 
 static esf_status init_state(PcrState* d, double eps, int maxIt, cudaStream_t st, int inner = 0) {
@@ -1469,7 +1540,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
   const void* key[8] = {w->minv32, w->invd32, w->b32, w->x32, tma, &w->fmaps,
                         reinterpret_cast<const void*>(static_cast<uintptr_t>(path + 1)),
                         reinterpret_cast<const void*>(static_cast<uintptr_t>(fused_cz(g)))};
-  if (!w->graphsFor32 || memcmp(key, w->keyB, sizeof key) != 0) {
+  if ((!fused || !kf.loops()) && (!w->graphsFor32 || memcmp(key, w->keyB, sizeof key) != 0)) {
     esf_status e = fused ? capture(w->capStream, kf, false, false, &w->gChunk32, &w->kChunk32)
                          : capture(w->capStream, k32, false, false, &w->gChunk32, &w->kChunk32);
     if (e) return e;
@@ -1555,7 +1626,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     kx.ddf = w->ddf;
     const void* keyx[8] = {w->minv32, w->invd32, w->edf, w->ddf, tma, &w->fmaps,
                            reinterpret_cast<const void*>(static_cast<uintptr_t>(fused_cz(g))), nullptr};
-    if (!w->graphsForX || memcmp(keyx, w->keyX, sizeof keyx) != 0) {
+    if (!kx.loops() && (!w->graphsForX || memcmp(keyx, w->keyX, sizeof keyx) != 0)) {
       esf_status e = capture(w->capStream, kx, false, false, &w->gChunkX, &w->kChunkX);
       if (e) return e;
       memcpy(w->keyX, keyx, sizeof keyx);
@@ -1583,8 +1654,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     ESF_LAUNCH_CHECK();
     for (;;) {
       PcrState hi;
-      esf_status e = run_graph_solve(w->hst, w->ev, w->st32, nullptr, w->gChunkX, 0, w->kChunkX, maxIt,
-                                     st, &hi);
+      esf_status e = run_fused(w, kx, w->gChunkX, w->kChunkX, maxIt, st, &hi);
       if (e) return e;
       total = hi.iter;
       if (hi.status) {
@@ -1654,6 +1724,8 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
       PcrState hi;
       esf_status e = (fused && batching_pays(w))
                          ? batched_inner_solve(w, g, st, &hi)
+                     : fused
+                         ? run_fused(w, kf, w->gChunk32, w->kChunk32, maxIt, st, &hi)
                          : run_graph_solve(w->hst, w->ev, w->st32, nullptr, w->gChunk32, 0, w->kChunk32,
                                            maxIt, st, &hi);
       if (e) return e;
