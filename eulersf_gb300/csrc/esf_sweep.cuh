@@ -44,6 +44,22 @@ __device__ __forceinline__ double third(double x) {
   return __fma_rn(__fma_rn(-3.0, q, x), y, q);
 }
 
+// a < b of numbers (no NaN) by their bits, 20 cycles where an FP64 comparison and
+// a select on it take 104; zeros of either sign order by their sign, which no
+// caller can tell.
+__device__ __forceinline__ long long order_key(double a) {
+  const int hi = __double2hiint(a), m = hi >> 31;
+  return ((long long)(hi ^ (m & 0x7fffffff)) << 32) | (unsigned)(__double2loint(a) ^ m);
+}
+__device__ __forceinline__ bool less_bits(double a, double b) { return order_key(a) < order_key(b); }
+// x to 24 bits, towards zero, as a float, 0 below 2^-126, by its bits (a conversion is an FP64
+// operation); for numbers below 2^128.
+__device__ __forceinline__ float near_float(double x) {
+  const int hi = __double2hiint(x), m = hi & 0x7fffffff;
+  const int e = m - (896 << 20);
+  return __int_as_float((hi & 0x80000000) | (e > 0 ? (e << 3) | (int)((unsigned)__double2loint(x) >> 29) : 0));
+}
+
 // The same update, with the FP64 work that cannot change its outcome left
 // out. GB300 issues two FP64 operations a cycle and SM, and a square root
 // followed by a division is most of a node's latency, so:
@@ -51,7 +67,7 @@ __device__ __forceinline__ double third(double x) {
 //    new distance is the root of sum over ds_i < t of (t - ds_i)^2 = 1, whose
 //    left side grows with t: where it is below `skipBelow` (0.99) at t = v,
 //    the root is above v. FP32 copies decide it; their rounding moves the sum
-//    by at most 2e-3 for distances up to 4096, and callers with larger ones
+//    by at most 4e-3 for distances up to 4096, and callers with larger ones
 //    pass skipBelow = 0, which skips nothing;
 //  * the reference tries the three-, two- and one-neighbour root in turn and
 //    takes the first that is not below its largest neighbour. The i-neighbour
@@ -66,8 +82,9 @@ __device__ __forceinline__ bool solve_distance_fast(double p, double q, double r
                                                     float fr, float fv, float skipBelow) {
   const float tp = fmaxf(fv - fp, 0.0f), tq = fmaxf(fv - fq, 0.0f), tr = fmaxf(fv - fr, 0.0f);
   if (tp * tp + tq * tq + tr * tr < skipBelow) return false;
-  const double mqr = (r < q) ? r : q, Mqr = (q < r) ? r : q;
-  const double ds0 = (mqr < p) ? mqr : p, ds2 = (p < Mqr) ? Mqr : p;
+  const bool rq = less_bits(r, q);
+  const double mqr = rq ? r : q, Mqr = rq ? q : r;  // (equal ones are the same)
+  const double ds0 = less_bits(mqr, p) ? mqr : p, ds2 = less_bits(p, Mqr) ? Mqr : p;
   const double ds1 = p + q + r - ds0 - ds2;
   const float lo = fminf(fminf(fp, fq), fr), hi = fmaxf(fmaxf(fp, fq), fr), mid = fp + fq + fr - lo - hi;
   const float e1 = mid - lo, e2 = hi - lo, e21 = hi - mid;
@@ -85,17 +102,24 @@ __device__ __forceinline__ bool solve_distance_fast(double p, double q, double r
     return n == 2 ? third(t) : n == 1 ? t * 0.5 : t;
   };
   double discrim = disc(i);
-  if (i < 2 && !(discrim > 0.0)) {
+  auto positive = [](double d) { return __double_as_longlong(d) > 0; };  // (a difference: no NaN, no -0)
+  auto negative = [](double d) { return __double2hiint(d) < 0; };
+  if (i < 2 && !positive(discrim)) {
     i = 2;
     discrim = disc(2);
   }
+  // nd is NaN only from a negative discriminant
+  bool nan = negative(discrim);
   double nd = root(i, discrim);
-  while (discrim < 0.0 || nd < (i == 2 ? ds2 : i == 1 ? ds1 : ds0)) {
+  while (negative(discrim) || (!nan && less_bits(nd, i == 2 ? ds2 : i == 1 ? ds1 : ds0))) {
     if (--i < 0) break;
     discrim = disc(i);
-    if (discrim > 0.0) nd = root(i, discrim);
+    if (positive(discrim)) {
+      nd = root(i, discrim);
+      nan = false;
+    }
   }
-  if (!(nd < v)) return false;
+  if (nan || !less_bits(nd, v)) return false;
   v = nd;
   return true;
 }
@@ -501,7 +525,7 @@ __global__ void __launch_bounds__(KT) k_sweep_seeds(GridDev g, const double* __r
     if (ms[n] != 0) continue;
     const double p = ph[n - w.di], q = ph[n - (long long)w.dj * g.X], r = ph[n - w.dk * g.slab];
     double v = ph[n];
-    if (solve_distance_fast(p, q, r, v, (float)p, (float)q, (float)r, (float)v, skipBelow)) {
+    if (solve_distance_fast(p, q, r, v, near_float(p), near_float(q), near_float(r), near_float(v), skipBelow)) {
       m[0] = min(m[0], a);
       m[1] = min(m[1], b);
       m[2] = min(m[2], c);
@@ -561,7 +585,7 @@ __global__ void __launch_bounds__(32) k_sweep_march(GridDev g, double* f, const 
     double* const outB = sendB ? mail + (J * w.nk + c) * w.ni : mail;
     double* const outC = sendC ? mailC + (K * w.nj + b) * w.ni : mail;
     double val = f[base - w.di];
-    float fval = (float)val;
+    float fval = near_float(val);
     // the own values, mass and upwind values from outside of D steps, loaded
     // one batch ahead
     double nov[D], nms[D], nub[D], nuc[D];
@@ -578,11 +602,14 @@ __global__ void __launch_bounds__(32) k_sweep_march(GridDev g, double* f, const 
     };
     fetch(0);
     for (int q0 = 0; q0 < steps; q0 += D) {
-      double ov[D], om[D], ub[D], uc[D];
+      double ov[D], ub[D], uc[D];
+      float fo[D];
+      bool om[D];
 #pragma unroll
       for (int s = 0; s < D; s++) {
         ov[s] = nov[s];
-        om[s] = nms[s];
+        fo[s] = near_float(nov[s]);
+        om[s] = (__double2hiint(nms[s]) & 0x7fffffff) | __double2loint(nms[s]);
         ub[s] = nub[s];
         uc[s] = nuc[s];
       }
@@ -619,13 +646,13 @@ __global__ void __launch_bounds__(32) k_sweep_march(GridDev g, double* f, const 
         float fb = __shfl_up_sync(0xffffffffu, fval, 1), fc = __shfl_up_sync(0xffffffffu, fval, MARCH_B);
         vb = needB ? ub[s] : vb;
         vc = needC ? uc[s] : vc;
-        fb = needB ? (float)vb : fb;
-        fc = needC ? (float)vc : fc;
+        fb = needB ? near_float(vb) : fb;
+        fc = needC ? near_float(vc) : fc;
         double v = ov[s];
-        if (in && om[s] == 0.0 && solve_distance_fast(val, vb, vc, v, fval, fb, fc, (float)v, skipBelow))
+        if (in && !om[s] && solve_distance_fast(val, vb, vc, v, fval, fb, fc, fo[s], skipBelow))
           f[base + ac * w.di] = v;
         val = in ? v : val;
-        fval = (float)val;
+        fval = near_float(val);
         if (sendB && in) mail_store(outB + ac, val);
         if (sendC && in) mail_store(outC + ac, val);
       }
