@@ -437,11 +437,15 @@ __device__ __forceinline__ double bspline(double d) {
 }
 // The 4 weights per axis of a particle's 4^3 stencil, whose first node is
 // floor((p - o)/dh) - 1 on each axis: w[4*axis + k] for node base + k.
+__device__ __forceinline__ void stencil_base(const GridDev& g, const double* pos, int base[3]) {
+#pragma unroll
+  for (int q = 0; q < 3; q++) base[q] = (int)floor((pos[q] - g.o[q]) / g.dh) - 1;
+}
 __device__ __forceinline__ void stencil_weights(const GridDev& g, const double* pos, int base[3],
                                                 double w[12]) {
+  stencil_base(g, pos, base);
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    base[q] = (int)floor((pos[q] - g.o[q]) / g.dh) - 1;
     const double f = g.dhInv * (pos[q] - g.o[q]);
 #pragma unroll
     for (int k = 0; k < 4; k++) w[4 * q + k] = bspline(f - (base[q] + k));
@@ -570,7 +574,7 @@ __global__ void k_grid_to_particle(GridDev g, SolidDev s, long long np, double* 
 // block, one atomic per block and bound; the box words start at
 // +/- 2^30 on the host).
 __global__ void __launch_bounds__(256) k_p2g_keys(GridDev g, long long np, const double* part, unsigned int* keys,
-                                                  unsigned int* vals, int* pbox, double* pw) {
+                                                  unsigned int* vals, int* pbox) {
   __shared__ int sb[6];
   if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
   __syncthreads();
@@ -579,9 +583,7 @@ __global__ void __launch_bounds__(256) k_p2g_keys(GridDev g, long long np, const
   FOR_N(np, c) {
     const double* P = part + 10 * c;
     int bb[3];
-    double wt[12];
-    stencil_weights(g, P, bb, wt);
-    for (int q = 0; q < 12; q++) pw[12 * c + q] = wt[q];
+    stencil_base(g, P, bb);
     int i = bb[0], j = bb[1], k = bb[2];
     unsigned int key = (unsigned int)(KX * KY * KZ);
     if (i >= -3 && i <= g.X - 1 && j >= -3 && j <= g.Y - 1 && k >= -3 && k <= g.Z - 1) {
@@ -625,35 +627,102 @@ __global__ void k_bucket_bounds(long long np, const unsigned int* skeys, int* bs
     if (c == np - 1 || skeys[c + 1] != k) bend[k] = (int)c + 1;
   }
 }
+// The particles in bucket order, as the gather reads them: velocity, the four z
+// weights, the sixteen products of an x and a y weight (x fastest).
+constexpr int P2G_REC = 24;
+__global__ void __launch_bounds__(KT) k_p2g_records(GridDev g, long long np, const double* part,
+                                                    const unsigned int* sval, double* rec) {
+  FOR_N(np, e) {
+    const double* P = part + 10 * (long long)sval[e];
+    const double pos[3] = {P[0], P[1], P[2]};
+    int bb[3];
+    double wt[12];
+    stencil_weights(g, pos, bb, wt);
+    double2* R = reinterpret_cast<double2*>(rec + P2G_REC * e);
+    R[0] = make_double2(P[3], P[4]);
+    R[1] = make_double2(P[5], 0.0);
+    R[2] = make_double2(wt[8], wt[9]);
+    R[3] = make_double2(wt[10], wt[11]);
+#pragma unroll
+    for (int y = 0; y < 4; y++) {
+      R[4 + 2 * y] = make_double2(wt[0] * wt[4 + y], wt[1] * wt[4 + y]);
+      R[5 + 2 * y] = make_double2(wt[2] * wt[4 + y], wt[3] * wt[4 + y]);
+    }
+  }
+}
 // DEFOR_SOLID_3D::particleToGrid (DEFOR_SOLID_3D.cpp:1036-1107) as a
 // per-node gather over the 4^3 buckets whose stencils reach the node, in
-// bucket order then particle order (deterministic).
-__global__ void k_p2g_gather(GridDev g, SolidDev s, Box nodes, const double* part,
-                             const double* pw, const unsigned int* sval, const int* bstart,
-                             const int* bend, int cutoff) {
+// bucket order then particle order (deterministic). Bound: FP64 (eight
+// operations a pair of particle and node; 7.8 million pairs at 64^3, 122
+// thousand particles, are 0.12 ms) and as many cycles of L1, whose every load
+// touches a record a lane; warps at the solid's edge are partly idle. Reading
+// particles through their sorted indices one at a time, a node was a chain of
+// 2048 loads: the phase 1.69 -> 0.89 ms at 64^3 and 3.45 -> 2.56 at 128^3 (0.98
+// and 2.69 bucket by bucket without the next records on their way; eight ahead
+// 0.87 and 2.62).
+// A row of four buckets along x is one run of records, read P2G_AHEAD at a time,
+// the next ones while these are added.
+constexpr int P2G_THREADS = 64, P2G_AHEAD = 4;
+__global__ void __launch_bounds__(P2G_THREADS) k_p2g_gather(GridDev g, SolidDev s, Box nodes, const double* rec,
+                                                            const int* bstart, const int* bend, int cutoff) {
+  constexpr int D = P2G_AHEAD;
   const long long KX = g.X + 3, KY = g.Y + 3;
   FOR_BOX(nodes, x, y, z) {
     double acc[4] = {0, 0, 0, 0};
     bool touched = false;
-    for (int bz = z - 3; bz <= z; bz++)
-      for (int by = y - 3; by <= y; by++)
-        for (int bx = x - 3; bx <= x; bx++) {
-          if (bx < -3 || by < -3 || bz < -3) continue;
-          long long key = (bx + 3) + KX * ((by + 3) + KY * (long long)(bz + 3));
-          int b0 = bstart[key], b1 = bend[key];
-          const int ox = x - bx, oy = 4 + y - by, oz = 8 + z - bz;
-          for (int e = b0; e < b1; e++) {
-            const long long pi = sval[e];
-            const double* P = part + 10 * pi;
-            const double* W = pw + 12 * pi;
-            double w = W[ox] * W[oy] * W[oz];
-            touched = true;
-            acc[0] += w * P[3];
-            acc[1] += w * P[4];
-            acc[2] += w * P[5];
-            acc[3] += w;
+    for (int bz = max(z - 3, -3); bz <= z; bz++)
+      for (int by = max(y - 3, -3); by <= y; by++) {
+        const long long row = KX * ((by + 3) + KY * (long long)(bz + 3)) + x;
+        int b0[4], b1[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          b0[k] = bstart[row + k];
+          b1[k] = bend[row + k];
+        }
+        // [e0, e1): the run; a particle at or past m[k] is in a later bucket than k
+        int e0 = 0, e1 = 0, m[4];
+#pragma unroll
+        for (int k = 3; k >= 0; k--) e0 = b0[k] < b1[k] ? b0[k] : e0;
+        e1 = e0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) m[k] = e1 = b0[k] < b1[k] ? b1[k] : e1;
+        if (e0 >= e1) continue;
+        touched = true;
+        const double* const R = rec + 4 + z - bz;            // z weight
+        const double* const Q = rec + 8 + 4 * (y - by) + 3;  // products
+        double2 v[D], vn[D];
+        double vz[D], wz[D], wxy[D], vzn[D], wzn[D], wxyn[D];
+        auto load = [&](int e, double2* a, double* az, double* c, double* d) {
+#pragma unroll
+          for (int u = 0; u < D; u++) {
+            const int i = min(e + u, e1 - 1);
+            const int k = (i >= m[0]) + (i >= m[1]) + (i >= m[2]);
+            const long long o = (long long)P2G_REC * i;
+            a[u] = *reinterpret_cast<const double2*>(rec + o);
+            az[u] = rec[o + 2];
+            c[u] = R[o];
+            d[u] = Q[o - k];
+          }
+        };
+        load(e0, v, vz, wz, wxy);
+        for (int e = e0; e < e1; e += D) {
+          load(e + D, vn, vzn, wzn, wxyn);
+#pragma unroll
+          for (int u = 0; u < D; u++) {
+            if (e + u < e1) {
+              const double w = wxy[u] * wz[u];
+              acc[0] += w * v[u].x;
+              acc[1] += w * v[u].y;
+              acc[2] += w * vz[u];
+              acc[3] += w;
+            }
+            v[u] = vn[u];
+            vz[u] = vzn[u];
+            wz[u] = wzn[u];
+            wxy[u] = wxyn[u];
           }
         }
+      }
     long long n = nidx(g, x, y, z);
     if (touched && !(acc[3] < (double)cutoff)) {
       for (int q = 0; q < 3; q++) s.vel[3 * n + q] = acc[q] / acc[3];

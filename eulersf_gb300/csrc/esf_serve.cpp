@@ -218,7 +218,8 @@ extern "C" size_t esf_scene_footprint(const esf_grid* g, const esf_params* p, in
     double cells = 1.0;
     for (int q = 0; q < 3; q++) cells *= std::max(0.0, (hi[q] - lo[q]) / g->dh + 2.0);
     const double solidNodes = 0.55 * cells;  // sphere / box volume, plus a margin
-    bytes += solidNodes * (27 * 9 * 8 * 1.5 + 27 * 4 + 400) + solidNodes * p->particles_per_cell * 80.0;
+    // (a particle: its state, and 96 bytes more in its P2G record than the fit had)
+    bytes += solidNodes * (27 * 9 * 8 * 1.5 + 27 * 4 + 400) + solidNodes * p->particles_per_cell * 160.0;
   }
   return (size_t)(bytes * 1.1) + (140u << 20);
 }

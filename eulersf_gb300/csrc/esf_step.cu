@@ -1417,13 +1417,13 @@ extern "C" esf_status esf_step(esf_scene* sc, esf_step_report* rep) {
     TRY(sc->svals.ensure(np * 4));
     TRY(sc->bstart.ensure((size_t)nkeys * 4));
     TRY(sc->bend.ensure((size_t)nkeys * 4));
-    TRY(sc->pweights.ensure((size_t)np * 96));
+    TRY(sc->pweights.ensure((size_t)np * P2G_REC * 8));
     int pinit[6] = {1 << 30, 1 << 30, 1 << 30, -(1 << 30), -(1 << 30), -(1 << 30)};
     memcpy(sc->hInts, pinit, sizeof pinit);
     ESF_CUDA(cudaMemcpyAsync(sc->dInts, sc->hInts, sizeof pinit, cudaMemcpyHostToDevice, st));
     ESF_COUNTED k_p2g_keys<<<kblocks(np), 256, 0, st>>>(G, np, d->part.as<double>(), sc->keys.as<unsigned int>(),
-                                           sc->vals.as<unsigned int>(), sc->dInts, sc->pweights.as<double>());
-    tm.mark("p2g: keys and weights");
+                                           sc->vals.as<unsigned int>(), sc->dInts);
+    tm.mark("p2g: keys");
     int bits = 1;
     while (bits < 32 && (1ull << bits) <= nkeys) bits++;
     size_t tb = 0;
@@ -1433,6 +1433,8 @@ extern "C" esf_status esf_step(esf_scene* sc, esf_step_report* rep) {
     cub::DeviceRadixSort::SortPairs(sc->cubTmp.p, tb, sc->keys.as<unsigned int>(), sc->skeys.as<unsigned int>(),
                                     sc->vals.as<unsigned int>(), sc->svals.as<unsigned int>(), (int)np, 0, bits, st);
     tm.mark("p2g: sort");
+    ESF_COUNTED k_p2g_records<<<kblocks(np), KT, 0, st>>>(G, np, d->part.as<double>(), sc->svals.as<unsigned int>(),
+                                              sc->pweights.as<double>());
     ESF_CUDA(cudaMemsetAsync(sc->bstart.p, 0, (size_t)nkeys * 4, st));
     ESF_CUDA(cudaMemsetAsync(sc->bend.p, 0, (size_t)nkeys * 4, st));
     ESF_COUNTED k_bucket_bounds<<<kblocks(np), KT, 0, st>>>(np, sc->skeys.as<unsigned int>(), sc->bstart.as<int>(),
@@ -1443,8 +1445,8 @@ extern "C" esf_status esf_step(esf_scene* sc, esf_step_report* rep) {
                    std::min(sc->hInts[3] + 4, G.X), std::min(sc->hInts[4] + 4, G.Y), std::min(sc->hInts[5] + 4, G.Z));
     tm.mark("p2g: bucket bounds");
     if (boxn(nb) > 0)
-      ESF_COUNTED k_p2g_gather<<<kblocks(boxn(nb)), KT, 0, st>>>(G, d->d, nb, d->part.as<double>(), sc->pweights.as<double>(), sc->svals.as<unsigned int>(),
-                                                     sc->bstart.as<int>(), sc->bend.as<int>(), sc->p.flip_cutoff);
+      ESF_COUNTED k_p2g_gather<<<kblocks(boxn(nb), P2G_THREADS), P2G_THREADS, 0, st>>>(
+          G, d->d, nb, sc->pweights.as<double>(), sc->bstart.as<int>(), sc->bend.as<int>(), sc->p.flip_cutoff);
     ESF_LAUNCH_CHECK();
     tm.mark("p2g: gather");
   }
