@@ -68,15 +68,10 @@ __device__ __forceinline__ bool persist_sync(unsigned* bar, unsigned& target) {
   __syncthreads();
   return ok;
 }
-// The sum of n partials in last_block_sum's order, in every block (thread 0's value).
-__device__ __forceinline__ double persist_fold(const double* partial, int n, double* sh) {
-  double acc = 0;
-  for (int i = threadIdx.x; i < n; i += VT) acc += __ldcg(partial + i);
-  return block_sum<VT>(acc, sh);
-}
-// The same for a row pass: n warp sums, eight to a virtual block, added up as
+// The sum of a row pass in every block, in fold_partials' order (thread 0's
+// value): n warp sums, eight to a virtual block, added up as
 // block_sum's second stage adds them.
-__device__ __forceinline__ double persist_fold_rows(const double* sums, int n, double* sh) {
+__device__ __forceinline__ double persist_fold_rows(const double* sums, int n) {
   double acc = 0;
   for (int v = threadIdx.x; 8 * v < n; v += VT) {
     double w[8];
@@ -84,7 +79,7 @@ __device__ __forceinline__ double persist_fold_rows(const double* sums, int n, d
     for (int k = 0; k < 8; k++) w[k] = 8 * v + k < n ? __ldcg(sums + 8 * v + k) : 0.0;
     acc += ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
   }
-  return block_sum<VT>(acc, sh);
+  return block_sum<VT>(acc);
 }
 // a warp's sum in block_sum's first stage (lane 0's value)
 __device__ __forceinline__ double warp_tree(double v) {
@@ -132,7 +127,6 @@ __device__ __forceinline__ T spmv_component(const T* __restrict__ blocks, const 
 // SM's registers to other streams' kernels)
 template <typename T, bool MATRIX_FREE>
 __global__ void __launch_bounds__(VT, std::is_same<T, float>::value ? 2 : 1) solid_pcr_persistent(SolidPersist<T> a, int budget) {
-  __shared__ double sred[32];
   __shared__ T sy[2][3][32];
   __shared__ PcrState L;  // every block's copy of the state; block 0's goes back
   const int tid = threadIdx.x, G = gridDim.x;
@@ -153,7 +147,7 @@ __global__ void __launch_bounds__(VT, std::is_same<T, float>::value ? 2 : 1) sol
       auto acc = zero;
       for (long long i = v * (long long)VT + tid; i < n; i += (long long)a.vb * VT) body(i, acc);
       if (sums) {
-        const double bs = block_sum<VT>((double)acc, sred);
+        const double bs = block_sum<VT>((double)acc);
         if (tid == 0) sums[v] = bs;
       }
     }
@@ -232,7 +226,7 @@ __global__ void __launch_bounds__(VT, std::is_same<T, float>::value ? 2 : 1) sol
       });
     }
     if (!persist_sync(a.bar, target)) return false;
-    const double total = persist_fold_rows(ps, slices, sred);
+    const double total = persist_fold_rows(ps, slices);
     if (tid == 0) finish_update(&L, total);
     __syncthreads();
     return true;
@@ -248,7 +242,7 @@ __global__ void __launch_bounds__(VT, std::is_same<T, float>::value ? 2 : 1) sol
       acc += (double)bv * (double)bv;
     });
     ok = persist_sync(a.bar, target);
-    const double total = persist_fold(pz, a.vb, sred);
+    const double total = fold_partials<VT>(pz, a.vb);
     if (tid == 0) L.bnorm2 = total;
     __syncthreads();
     ok = ok && apply((T)0, false);
@@ -272,7 +266,7 @@ __global__ void __launch_bounds__(VT, std::is_same<T, float>::value ? 2 : 1) sol
     });
     ok = persist_sync(a.bar, target);
     if (!ok) break;
-    const double total = persist_fold(pv, a.vb, sred);
+    const double total = fold_partials<VT>(pv, a.vb);
     if (tid == 0) {
       L.alpha = (fabs(total) > 0.0) ? L.delta / total : total;
       if (!(total == total)) {
@@ -304,7 +298,7 @@ __global__ void __launch_bounds__(VT, std::is_same<T, float>::value ? 2 : 1) sol
           }
         });
         ok = persist_sync(a.bar, target);
-        const double res = persist_fold_rows(pc, slices, sred);
+        const double res = persist_fold_rows(pc, slices);
         if (tid == 0) {
           L.resid2 = res;
           if (sqrt(res) < L.eps * sqrt(L.bnorm2)) {

@@ -36,19 +36,38 @@
 namespace esf {
 
 // ------------------------------------------------------------ reductions
+// Sum of a block's values, in thread 0: within each warp the tree of halves 16,
+// 8, 4, 2, 1, then the warps' sums by the same tree. One warp forms it all from
+// shared memory, a lane taking every (32 / NW)th value of a warp, so the tree is
+// 12 FP64 instructions (NW = 8) where all warps shuffling took 45, each 19 cycles
+// of the SM's FP64 pipe. With the last block's reads of partials and state at
+// once, and one release and acquire on its ticket for two fences, an iteration
+// of the FP64 solve takes 19.0 for 21.6 us at 32^3, 33.7 for 36.4 at 64^3, 130
+// for 133 at 128^3, and the mixed solid solve of a step at 128^3 2.72 for 2.90 ms.
 template <int NT>
-__device__ __forceinline__ double block_sum(double v, double* sh) {
+__device__ __forceinline__ double block_sum(double v) {
+  constexpr int NW = NT / 32, STEP = 32 / NW, PITCH = 36;
+  static_assert(NW == 4 || NW == 8, "a lane for each warp and step");
+  __shared__ double values[NW * PITCH];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __syncthreads();
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
+  values[w * PITCH + lane] = v;
   __syncthreads();
   double r = 0;
   if (threadIdx.x < 32) {
-    r = (threadIdx.x < NT / 32) ? sh[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+    const double* q = values + (lane % NW) * PITCH + lane / NW;
+    double t[NW];
+#pragma unroll
+    for (int k = 0; k < NW; k++) t[k] = q[STEP * k];
+#pragma unroll
+    for (int h = NW / 2; h > 0; h /= 2)
+#pragma unroll
+      for (int k = 0; k < h; k++) t[k] += t[k + h];
+    r = t[0];
+    for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if (__double_as_longlong(r) == (long long)0x8000000000000000ull) r = 0.0;  // (never -0)
   }
-  return r;  // valid in thread 0
+  return r;
 }
 
 // The largest of a block's words into *out, by thread 0 (whose fence in
@@ -64,30 +83,52 @@ __device__ __forceinline__ void block_max(unsigned mine, unsigned* out) {
   if (threadIdx.x == 0) atomicMax(out, top);
 }
 
-// Deposit this block's partial; returns true in the block that arrives last,
-// after which `*total` holds the sum of all partials in block order.
-template <int NT>
-__device__ bool last_block_sum(double mine, double* partial, unsigned int* ticket, int nblocks,
-                               double* total, double* sh) {
+// Deposit this block's partial (thread 0's); true in the block that arrives
+// last, where the others' are there to be read.
+__device__ __forceinline__ bool last_block(double mine, double* partial, unsigned int* ticket, int nblocks) {
   __shared__ bool amLast;
   const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
   if (threadIdx.x == 0) {
-    partial[bid] = mine;
-    __threadfence();
-    unsigned int t = atomicAdd(ticket, 1u);
-    amLast = (t == (unsigned)nblocks - 1);
+    __stcg(partial + bid, mine);
+    unsigned t;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(ticket) : "memory");
+    amLast = t == (unsigned)nblocks - 1;
   }
   __syncthreads();
-  if (!amLast) return false;
-  __threadfence();
-  double acc = 0;
-  for (int i = threadIdx.x; i < nblocks; i += NT) acc += __ldcg(partial + i);
-  double s = block_sum<NT>(acc, sh);
+  return amLast;
+}
+// The sum of n partials in block order, in thread 0.
+template <int NT>
+__device__ __forceinline__ double fold_partials(const double* partial, int n) {
+  int i = threadIdx.x;
+  double acc = i < n ? __ldcg(partial + i) : 0.0;
+  for (i += NT; i < n; i += NT) acc += __ldcg(partial + i);
+  return block_sum<NT>(acc);
+}
+// Both: in the last block, `*total` holds the sum of all partials in block order.
+template <int NT>
+__device__ bool last_block_sum(double mine, double* partial, unsigned int* ticket, int nblocks, double* total) {
+  if (!last_block(mine, partial, ticket, nblocks)) return false;
+  const double s = fold_partials<NT>(partial, nblocks);
   if (threadIdx.x == 0) {
     *total = s;
     *ticket = 0;
   }
   return true;
+}
+// The same with a solve's ticket W, and in the last block's thread 0 a copy of the
+// state with the ticket cleared, read while the partials are: to be changed and
+// written back. True in that thread only.
+template <int NT, int W>
+__device__ __forceinline__ bool last_block_state(double mine, double* partial, PcrState* st, int nblocks,
+                                                 double* total, PcrState* L) {
+  if (!last_block(mine, partial, &st->ticket[W], nblocks)) return false;
+  if (threadIdx.x == 0) {
+    *L = *st;
+    L->ticket[W] = 0;
+  }
+  *total = fold_partials<NT>(partial, nblocks);
+  return threadIdx.x == 0;
 }
 
 // Scalars after the phase-B reduction r.s (CONJUGATE_RESIDUAL.inl:150-154).
@@ -188,7 +229,6 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(NT) pressure_stencil(GridDev g, StencilArgs<T> a, int cz) {
   __shared__ T sP[NHALO], sQ[NHALO], sV[2][NHALO];
   __shared__ T sA[NNODE], sB[NNODE], sC[NNODE];
-  __shared__ double sred[32];
   if (MODE != S_APPLY && a.st->done) return;
   const int tid = threadIdx.x;
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * cz;
@@ -351,12 +391,11 @@ __global__ void __launch_bounds__(NT) pressure_stencil(GridDev g, StencilArgs<T>
   if (MODE == S_APPLY) return;
   if (MODE == S_UPDATE) acc = (double)accT;
   __syncthreads();
-  double bs = block_sum<NT>(acc, sred);
+  double bs = block_sum<NT>(acc);
   const int nblocks = gridDim.x * gridDim.y * gridDim.z;
   double total;
-  if (last_block_sum<NT>(bs, a.partial, &a.st->ticket[1], nblocks, &total, sred) &&
-      threadIdx.x == 0) {
-    PcrState* st = a.st;
+  PcrState L, *const st = &L;
+  if (last_block_state<NT, 1>(bs, a.partial, a.st, nblocks, &total, st)) {
     if (MODE == S_UPDATE) {
       finish_update(st, total);
     } else if (MODE == S_CHECK) {
@@ -370,6 +409,7 @@ __global__ void __launch_bounds__(NT) pressure_stencil(GridDev g, StencilArgs<T>
     } else if (MODE == S_RESID_INIT) {
       st->bnorm2 = total;
     }
+    *a.st = L;
   }
 }
 
@@ -390,7 +430,6 @@ constexpr int VT = 256;
 template <typename T, bool UPDR, bool BOUND = false>
 __global__ void __launch_bounds__(VT) pcr_phase_a(long long n, T* d, T* r, T* Ap, const T* s,
                                                   const T* invd, double* partial, PcrState* st) {
-  __shared__ double sred[32];
   if (st->done) return;
   if (st->iter >= st->maxIt) {
     if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1;
@@ -454,19 +493,20 @@ __global__ void __launch_bounds__(VT) pcr_phase_a(long long n, T* d, T* r, T* Ap
     block_max(hr, &st->hr);
     block_max(hq, &st->hq);
   }
-  double bs = block_sum<VT>((double)acc, sred);
+  double bs = block_sum<VT>((double)acc);
   double total;
-  if (last_block_sum<VT>(bs, partial, &st->ticket[0], gridDim.x, &total, sred) &&
-      threadIdx.x == 0) {
-    st->alpha = (fabs(total) > 0.0) ? st->delta / total : total;
+  PcrState L;
+  if (last_block_state<VT, 0>(bs, partial, st, gridDim.x, &total, &L)) {
+    L.alpha = (fabs(total) > 0.0) ? L.delta / total : total;
     if constexpr (BOUND) {
-      st->hv = fixed_bound(__ldcg(&st->hr), __ldcg(&st->hq), st->alpha);
-      st->hr = st->hq = 0;
+      L.hv = fixed_bound(L.hr, L.hq, L.alpha);
+      L.hr = L.hq = 0;
     }
     if (!(total == total)) {
-      st->status = ESF_ERR_NUMERIC;
-      st->done = 1;
+      L.status = ESF_ERR_NUMERIC;
+      L.done = 1;
     }
+    *st = L;
   }
 }
 
@@ -475,7 +515,6 @@ template <typename T>
 __global__ void __launch_bounds__(VT) pcr_zero_start(long long n, const T* b, const T* invd, T* x,
                                                      T* r, T* d, T* Ap, double* partial,
                                                      PcrState* st) {
-  __shared__ double sred[32];
   double acc = 0;
   for (long long i = blockIdx.x * (long long)VT + threadIdx.x; i < n; i += (long long)gridDim.x * VT) {
     T bv = b[i];
@@ -485,9 +524,9 @@ __global__ void __launch_bounds__(VT) pcr_zero_start(long long n, const T* b, co
     Ap[i] = 0;
     acc += (double)bv * (double)bv;
   }
-  double bs = block_sum<VT>(acc, sred);
+  double bs = block_sum<VT>(acc);
   double total;
-  if (last_block_sum<VT>(bs, partial, &st->ticket[2], gridDim.x, &total, sred) &&
+  if (last_block_sum<VT>(bs, partial, &st->ticket[2], gridDim.x, &total) &&
       threadIdx.x == 0)
     st->bnorm2 = total;
 }
@@ -496,13 +535,12 @@ __global__ void __launch_bounds__(VT) pcr_zero_start(long long n, const T* b, co
 template <typename T>
 __global__ void __launch_bounds__(VT) vec_norm2(long long n, const T* b, double* partial,
                                                 unsigned int* ticket, double* out) {
-  __shared__ double sred[32];
   double acc = 0;
   for (long long i = blockIdx.x * (long long)VT + threadIdx.x; i < n; i += (long long)gridDim.x * VT)
     acc += (double)b[i] * (double)b[i];
-  double bs = block_sum<VT>(acc, sred);
+  double bs = block_sum<VT>(acc);
   double total;
-  if (last_block_sum<VT>(bs, partial, ticket, gridDim.x, &total, sred) && threadIdx.x == 0)
+  if (last_block_sum<VT>(bs, partial, ticket, gridDim.x, &total) && threadIdx.x == 0)
     *out = total;
 }
 
@@ -1934,7 +1972,6 @@ __global__ void __launch_bounds__(VT) solid_spmv(long long S, const T* __restric
                                                  const int* __restrict__ nbr, const T* in,
                                                  const T* b, T* r, T* out, float* out32,
                                                  double* partial, PcrState* st) {
-  __shared__ double sred[32];
   if (MODE != S_APPLY && st->done) return;
   double acc = 0;
   T accT = 0;
@@ -1980,27 +2017,22 @@ __global__ void __launch_bounds__(VT) solid_spmv(long long S, const T* __restric
   }
   if (MODE == S_APPLY) return;
   if (MODE == S_UPDATE) acc = (double)accT;
-  double bs = block_sum<VT>(acc, sred);
+  double bs = block_sum<VT>(acc);
   double total;
-  if (last_block_sum<VT>(bs, partial, &st->ticket[1], gridDim.x, &total, sred) &&
-      threadIdx.x == 0) {
+  PcrState L;
+  if (last_block_state<VT, 1>(bs, partial, st, gridDim.x, &total, &L)) {
     if (MODE == S_UPDATE) {
-      finish_update(st, total);
+      finish_update(&L, total);
+    } else if (MODE == S_CHECK) {
+      finish_check(&L, total);
     } else {
-      st->resid2 = total;
-      if (MODE == S_CHECK) {
-        if (sqrt(total) < st->eps * sqrt(st->bnorm2)) {
-          st->converged = 1;
-          st->done = 1;
-        } else {
-          st->iter++;
-        }
-      }
+      L.resid2 = total;
       if (!(total == total)) {
-        st->status = ESF_ERR_NUMERIC;
-        st->done = 1;
+        L.status = ESF_ERR_NUMERIC;
+        L.done = 1;
       }
     }
+    *st = L;
   }
 }
 
@@ -2129,7 +2161,6 @@ __device__ __forceinline__ void mf_node(const SolidMF& m, long long a, const flo
 __global__ void __launch_bounds__(VT) k_mf_gather(SolidMF m, long long S, const float* __restrict__ share,
                                                    const float* __restrict__ damped, const float* in, float* out,
                                                    double* partial, PcrState* st) {
-  __shared__ double sred[32];
   if (st->done) return;
   float accT = 0;
   for (long long a = blockIdx.x * (long long)VT + threadIdx.x; a < S; a += (long long)gridDim.x * VT) {
@@ -2143,10 +2174,13 @@ __global__ void __launch_bounds__(VT) k_mf_gather(SolidMF m, long long S, const 
       accT += in[i] * y[r];
     }
   }
-  const double bs = block_sum<VT>((double)accT, sred);
+  const double bs = block_sum<VT>((double)accT);
   double total;
-  if (last_block_sum<VT>(bs, partial, &st->ticket[1], gridDim.x, &total, sred) && threadIdx.x == 0)
-    finish_update(st, total);
+  PcrState L;
+  if (last_block_state<VT, 1>(bs, partial, st, gridDim.x, &total, &L)) {
+    finish_update(&L, total);
+    *st = L;
+  }
 }
 
 // x += alpha d; r -= alpha Ap/diag (pointwise part of phase B).

@@ -100,7 +100,6 @@ __device__ __forceinline__ unsigned fixed_bound(unsigned hr, unsigned hq, double
 template <int MODE, int RY>
 __global__ void __launch_bounds__(FX_T, 3) pressure_stencil_fixed(GridDev g, StencilArgs<double> a, int cz) {
   extern __shared__ double ring[];  // [2][slots][FX_T]
-  __shared__ double sred[32];
   if (MODE != S_APPLY && a.st->done) return;
   constexpr int SLOTS = fx_slots<MODE, RY>();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -275,11 +274,11 @@ __global__ void __launch_bounds__(FX_T, 3) pressure_stencil_fixed(GridDev g, Ste
   }
   if (MODE == S_APPLY) return;
   if (MODE == S_UPDATE || MODE == S_RESID_INIT) block_max(hx, MODE == S_UPDATE ? &a.st->hx : &a.st->hr);
-  const double bs = block_sum<FX_T>(acc, sred);
+  const double bs = block_sum<FX_T>(acc);
   const int nblocks = gridDim.x * gridDim.y * gridDim.z;
   double total;
-  if (last_block_sum<FX_T>(bs, a.partial, &a.st->ticket[1], nblocks, &total, sred) && threadIdx.x == 0) {
-    PcrState* st = a.st;
+  PcrState L, *const st = &L;
+  if (last_block_state<FX_T, 1>(bs, a.partial, a.st, nblocks, &total, st)) {
     if (MODE == S_UPDATE) {
       finish_update(st, total);
     } else if (MODE == S_CHECK) {
@@ -289,6 +288,7 @@ __global__ void __launch_bounds__(FX_T, 3) pressure_stencil_fixed(GridDev g, Ste
       st->hv = fixed_bound(st->hr, 0u, 0.0);
       st->hr = 0;
     }
+    *a.st = L;
   }
 }
 

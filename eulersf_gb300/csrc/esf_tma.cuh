@@ -63,8 +63,7 @@ constexpr int TW_OFF_Q = TW_OFF_P + TW_PP * HY * 4;
 constexpr int TW_OFF_A = TW_OFF_Q + TW_PP * HY * 4;
 constexpr int TW_OFF_B = TW_OFF_A + TW_NP * NYN * 4;
 constexpr int TW_OFF_C = TW_OFF_B + TW_NP * NYN * 4;
-constexpr int TW_OFF_RED = (TW_OFF_C + TW_NP * NYN * 4 + 15) / 16 * 16;
-constexpr int TW_OFF_ACC = TW_OFF_RED + 32 * 8;
+constexpr int TW_OFF_ACC = (TW_OFF_C + TW_NP * NYN * 4 + 15) / 16 * 16;
 constexpr int TW_SMEM = TW_OFF_ACC + 2 * NT * 4;  // about 45 KB: four blocks per SM
 // bounded waits: 2^18 polls before a block reports a stuck copy. An
 // unsuccessful mbarrier.try_wait suspends the thread for its own time limit
@@ -126,7 +125,6 @@ __global__ void __launch_bounds__(NT, 4) pressure_update_tma(GridDev g, const __
   float* sA = reinterpret_cast<float*>(smem + TW_OFF_A);
   float* sB = reinterpret_cast<float*>(smem + TW_OFF_B);
   float* sC = reinterpret_cast<float*>(smem + TW_OFF_C);
-  double* sred = reinterpret_cast<double*>(smem + TW_OFF_RED);
   float* sAcc = reinterpret_cast<float*>(smem + TW_OFF_ACC);
   __shared__ bool amLast;
   if (st->done) return;
@@ -337,7 +335,7 @@ __global__ void __launch_bounds__(NT, 4) pressure_update_tma(GridDev g, const __
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     __syncthreads();
-    part[h] = block_sum<NT>((double)sAcc[h * NT + tid], sred);
+    part[h] = block_sum<NT>((double)sAcc[h * NT + tid]);
   }
   if (tid == 0) {
     unsigned cnt = 0;
@@ -357,7 +355,7 @@ __global__ void __launch_bounds__(NT, 4) pressure_update_tma(GridDev g, const __
   __threadfence();
   double a = 0;
   for (int q = tid; q < nOld; q += NT) a += __ldcg(partial + q);
-  const double total = block_sum<NT>(a, sred);
+  const double total = block_sum<NT>(a);
   if (tid == 0) {
     st->ticket[1] = 0;
     finish_update(st, total);
