@@ -7,6 +7,7 @@
 
 #include "esf_common.cuh"
 #include "esf_contact.cuh"
+#include "esf_root.cuh"
 
 namespace esf {
 

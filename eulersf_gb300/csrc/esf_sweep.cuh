@@ -60,6 +60,15 @@ __device__ __forceinline__ float near_float(double x) {
   return __int_as_float((hi & 0x80000000) | (e > 0 ? (e << 3) | (int)((unsigned)__double2loint(x) >> 29) : 0));
 }
 
+// sqrt(x), x not negative
+__device__ __forceinline__ double root(double x) {
+  if ((unsigned)(__double2hiint(x) - (923 << 20)) >= (200u << 20)) return sqrt(x);  // not in 2^-100 .. 2^100
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(near_float(x)));
+  const unsigned u = __float_as_uint(y);
+  return root_from(x, __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29)));
+}
+
 // The same update, with the FP64 work that cannot change its outcome left
 // out. GB300 issues two FP64 operations a cycle and SM, and a square root
 // followed by a division is most of a node's latency, so:
@@ -91,33 +100,31 @@ __device__ __forceinline__ bool solve_distance_fast(double p, double q, double r
   int i = 2;
   if (skipBelow > 0.0f && e2 * e2 + e21 * e21 > 1.01f)
     i = (e1 * e1 > 1.01f && fabsf(e1 * e1 - 2.0f) > 0.02f) ? 0 : 1;
-  const double b0 = ds0, c0 = ds0 * ds0 - 1.0;
-  const double b1 = ds1 + b0, c1 = ds1 * ds1 + c0;
+  const double c0 = ds0 * ds0 - 1.0;
+  const double b1 = ds1 + ds0, c1 = ds1 * ds1 + c0;
   const double b2 = ds2 + b1, c2 = ds2 * ds2 + c1;
-  auto disc = [&](int n) {
-    return n == 2 ? b2 * b2 - 3.0 * c2 : n == 1 ? b1 * b1 - 2.0 * c1 : b0 * b0 - c0;
-  };
-  auto root = [&](int n, double d) {
-    const double t = (n == 2 ? b2 : n == 1 ? b1 : b0) + sqrt(d);
-    return n == 2 ? third(t) : n == 1 ? t * 0.5 : t;
-  };
-  double discrim = disc(i);
   auto positive = [](double d) { return __double_as_longlong(d) > 0; };  // (a difference: no NaN, no -0)
   auto negative = [](double d) { return __double2hiint(d) < 0; };
-  if (i < 2 && !positive(discrim)) {
-    i = 2;
-    discrim = disc(2);
-  }
-  // nd is NaN only from a negative discriminant
-  bool nan = negative(discrim);
-  double nd = root(i, discrim);
-  while (negative(discrim) || (!nan && less_bits(nd, i == 2 ? ds2 : i == 1 ? ds1 : ds0))) {
-    if (--i < 0) break;
-    discrim = disc(i);
-    if (positive(discrim)) {
-      nd = root(i, discrim);
+  // lanes of all i take the one path: K and the operands are selected, not the
+  // results (1 c and 2 c are exact, t / 2 as well)
+  bool nan = true, first = true;  // nd is NaN until a discriminant is not negative
+  double nd = 0.0;
+  for (;;) {
+    const double b = i == 2 ? b2 : i == 1 ? b1 : ds0, c = i == 2 ? c2 : i == 1 ? c1 : c0;
+    const double k = i == 2 ? 3.0 : i == 1 ? 2.0 : 1.0;
+    const double discrim = b * b - k * c;
+    if (first && i < 2 && !positive(discrim)) {
+      i = 2;
+      continue;
+    }
+    if (first ? !negative(discrim) : positive(discrim)) {
+      const double t = b + root(discrim);
+      nd = i == 2 ? third(t) : i == 1 ? t * 0.5 : t;
       nan = false;
     }
+    first = false;
+    if (!negative(discrim) && (nan || !less_bits(nd, i == 2 ? ds2 : i == 1 ? ds1 : ds0))) break;
+    if (--i < 0) break;
   }
   if (nan || !less_bits(nd, v)) return false;
   v = nd;
