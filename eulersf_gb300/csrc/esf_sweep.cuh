@@ -44,7 +44,7 @@ __device__ __forceinline__ double third(double x) {
   return __fma_rn(__fma_rn(-3.0, q, x), y, q);
 }
 
-// a < b of numbers (no NaN) by their bits, 20 cycles where an FP64 comparison and
+// a < b of numbers (no NaN) by their bits, 40 cycles where an FP64 comparison and
 // a select on it take 104; zeros of either sign order by their sign, which no
 // caller can tell.
 __device__ __forceinline__ long long order_key(double a) {
@@ -62,16 +62,16 @@ __device__ __forceinline__ float near_float(double x) {
 
 // sqrt(x), x not negative
 __device__ __forceinline__ double root(double x) {
-  if ((unsigned)(__double2hiint(x) - (923 << 20)) >= (200u << 20)) return sqrt(x);  // not in 2^-100 .. 2^100
+  if ((unsigned)(__double2hiint(x) - (963 << 20)) >= (120u << 20)) return sqrt(x);  // not in 2^-60 .. 2^60
   float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(near_float(x)));
-  const unsigned u = __float_as_uint(y);
-  return root_from(x, __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29)));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(leading_float(x)));
+  return root_from(x, y);
 }
 
 // The same update, with the FP64 work that cannot change its outcome left
-// out. GB300 issues two FP64 operations a cycle and SM, and a square root
-// followed by a division is most of a node's latency, so:
+// out. GB300 takes an FP64 instruction from a warp every 63 cycles, so their
+// number is most of a node's time (27 here at first with sqrt() and the quotient
+// by FMAs, 2740 cycles a node of a lone chain; 20 now, 2200), so:
 //  * a node whose value v already lies below the new distance keeps it. The
 //    new distance is the root of sum over ds_i < t of (t - ds_i)^2 = 1, whose
 //    left side grows with t: where it is below `skipBelow` (0.99) at t = v,
@@ -119,7 +119,10 @@ __device__ __forceinline__ bool solve_distance_fast(double p, double q, double r
     }
     if (first ? !negative(discrim) : positive(discrim)) {
       const double t = b + root(discrim);
-      nd = i == 2 ? third(t) : i == 1 ? t * 0.5 : t;
+      if ((unsigned)(__double2hiint(t) - (100 << 20)) < (1900u << 20))
+        nd = i == 2 ? third_of(t) : i == 1 ? half_of(t) : t;
+      else  // (not a positive normal number)
+        nd = i == 2 ? third(t) : i == 1 ? t * 0.5 : t;
       nan = false;
     }
     first = false;
@@ -478,9 +481,10 @@ __global__ void __launch_bounds__(EXTEND_THREADS) k_extend_field(GridDev g, doub
 // (MARCH_WAIT_LIMIT polls): a warp that gives up sets *err and stops waiting,
 // as does every warp that sees *err, so the launch ends; the host reports it.
 // Measured (mesh, SDF and particle phase of a step, GB300): 11.3 ms with the
-// wave and 6.5 with the march at 64^3, 16.1 and 9.5 at 128^3. What is left is
-// the chain of square roots, about 1.7 us a step where lanes update. A
-// version with progress counters (release and acquire every batch) took 8.3,
+// wave and 6.5 with the march at 64^3, 16.1 and 9.5 at 128^3; 5.2 and 7.7 with
+// comparisons on the numbers' bits and the root and the third of esf_root.cuh.
+// What is left is the chain of FP64 instructions, 2200 cycles a step where lanes
+// update. A version with progress counters (release and acquire every batch) took 8.3,
 // and one that loaded mailboxes step by step 8.0 ms a step's passes at 64^3.
 constexpr int MARCH_B = 8, MARCH_C = 4, MARCH_BATCH = 4;
 constexpr int MARCH_SKEW = (MARCH_B - 1) + (MARCH_C - 1);
