@@ -582,6 +582,27 @@ __global__ void add_correction(long long n, double* x, const float* e) {
   for (long long i = blockIdx.x * (long long)VT + threadIdx.x; i < n; i += (long long)gridDim.x * VT)
     x[i] += (double)e[i];
 }
+// x += e, e = 0
+__global__ void fold_correction(long long n, double* x, float* e) {
+  for (long long i = blockIdx.x * (long long)VT + threadIdx.x; i < n; i += (long long)gridDim.x * VT) {
+    x[i] += (double)e[i];
+    e[i] = 0.0f;
+  }
+}
+// A state from the launch's arguments: no copy that a synchronisation must keep
+// the source for.
+__global__ void put_state(PcrState* d, const __grid_constant__ PcrState h) { *d = h; }
+// The same with up to four vectors zeroed (null: fewer): the start of an inner solve.
+__global__ void __launch_bounds__(VT) start_inner(long long n, float* a, float* b, float* c, float* e, PcrState* d,
+                                                  const __grid_constant__ PcrState h) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *d = h;
+  for (long long i = blockIdx.x * (long long)VT + threadIdx.x; i < n; i += (long long)gridDim.x * VT) {
+    a[i] = 0.0f;
+    b[i] = 0.0f;
+    if (c) c[i] = 0.0f;
+    if (e) e[i] = 0.0f;
+  }
+}
 
 static int vec_blocks(long long n) {
   long long b = (n + VT - 1) / VT;
@@ -1412,9 +1433,7 @@ static esf_status run_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst, int m
       }
     }
   }
-  // drain chunks still queued (they exit at once on `done`)
-  ESF_CUDA(cudaStreamSynchronize(st));
-  ESF_CUDA(cudaMemcpy(out, dst, sizeof(PcrState), cudaMemcpyDeviceToHost));
+  // (chunks still queued exit at once on `done`; what follows on the stream comes after them)
   return ESF_OK;
 }
 
@@ -1445,9 +1464,8 @@ static esf_status init_state(PcrState* d, double eps, int maxIt, cudaStream_t st
   h.maxIt = maxIt;
   h.setup = 1;
   h.inner = inner;
-  ESF_CUDA(cudaMemcpyAsync(d, &h, sizeof h, cudaMemcpyHostToDevice, st));
-  // the pageable source must not change before the copy runs
-  ESF_CUDA(cudaStreamSynchronize(st));
+  ESF_COUNTED put_state<<<1, 1, 0, st>>>(d, h);
+  ESF_LAUNCH_CHECK();
   return ESF_OK;
 }
 
@@ -1563,13 +1581,14 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
   // direction are FP32, whose rounding reaches the residual amplified by the
   // operator's conditioning (ESF_MIXED_X64, above, carries it with both in
   // double-float).
-  ESF_COUNTED convert_vec<double, float><<<vec_blocks(g.T), VT, 0, st>>>(g.T, minv64, w->minv32);
   const TmaMaps* tma = nullptr;
   int path = P32_REGISTER;
   {
     esf_status e = prepare_tma(w, g, minv64, st, &tma, &path);
     if (e) return e;
   }
+  if (path != P32_FUSED)  // (the one-pass kernels read the padded copy)
+    ESF_COUNTED convert_vec<double, float><<<vec_blocks(g.T), VT, 0, st>>>(g.T, minv64, w->minv32);
   PressureKernels<float> k32{g, w->minv32, w->invd32, w->b32, w->x32, w->r32, w->d32, w->Ap32,
                              w->s32, w->partial, w->st32};
   k32.tma = tma;
@@ -1587,11 +1606,10 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
   }
   // start of an inner solve: zero directions (and, one-pass, t of the first
   // buffer set, which the set-up pass reads), then the set-up pass s = A r
-  auto inner_setup = [&]() -> esf_status {
-    ESF_CUDA(cudaMemsetAsync(w->d32, 0, g.R * 4, st));
-    ESF_CUDA(cudaMemsetAsync(w->Ap32, 0, g.R * 4, st));
+  auto inner_setup = [&](const PcrState& h, bool first) -> esf_status {
+    ESF_COUNTED start_inner<<<vec_blocks(g.R), VT, 0, st>>>(g.R, w->d32, w->Ap32, fused ? w->s32 : nullptr,
+                                                            first ? w->x32 : nullptr, w->st32, h);
     if (fused) {
-      ESF_CUDA(cudaMemsetAsync(w->s32, 0, g.R * 4, st));
       kf.iteration(st);
     } else {
       k32.update(st);  // s = A r, delta (set-up: alpha = 0)
@@ -1615,7 +1633,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     a.partial = w->partial; a.st = w->st;
     ESF_COUNTED pressure_stencil<double, S_RESID64><<<stencil_grid<double>(g), NT, 0, st>>>(g, a, stencil_cz(g));
     ESF_LAUNCH_CHECK();
-    PcrState h;
+    PcrState& h = w->hst[4];  // (pinned)
     ESF_CUDA(cudaMemcpyAsync(&h, w->st, sizeof h, cudaMemcpyDeviceToHost, st));
     ESF_CUDA(cudaStreamSynchronize(st));
     *resid2 = h.resid2;
@@ -1677,8 +1695,6 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     };
     ESF_CUDA(cudaMemsetAsync(w->edf, 0, g.R * 8, st));
     ESF_CUDA(cudaMemsetAsync(w->ddf, 0, g.R * 8, st));
-    ESF_CUDA(cudaMemsetAsync(w->Ap32, 0, g.R * 4, st));
-    ESF_CUDA(cudaMemsetAsync(w->s32, 0, g.R * 4, st));
     PcrState h;
     memset(&h, 0, sizeof h);
     h.eps = predicted(resid2);
@@ -1686,8 +1702,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     h.setup = 1;
     h.inner = 1;
     h.cap = kX64CheckEvery;
-    ESF_CUDA(cudaMemcpyAsync(w->st32, &h, sizeof h, cudaMemcpyHostToDevice, st));
-    ESF_CUDA(cudaStreamSynchronize(st));
+    ESF_COUNTED start_inner<<<vec_blocks(g.R), VT, 0, st>>>(g.R, w->Ap32, w->s32, nullptr, nullptr, w->st32, h);
     kx.iteration(st);  // set-up pass: s = A r, delta; d = r; e unchanged (alpha 0)
     ESF_LAUNCH_CHECK();
     for (;;) {
@@ -1711,7 +1726,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
       a.minv = minv64; a.partial = w->partial; a.st = w->st;
       ESF_COUNTED pressure_stencil<double, S_RESID64><<<stencil_grid<double>(g), NT, 0, st>>>(g, a, stencil_cz(g));
       ESF_LAUNCH_CHECK();
-      PcrState ho;
+      PcrState& ho = w->hst[4];
       ESF_CUDA(cudaMemcpyAsync(&ho, w->st, sizeof ho, cudaMemcpyDeviceToHost, st));
       ESF_CUDA(cudaStreamSynchronize(st));
       resid2 = ho.resid2;
@@ -1731,13 +1746,11 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
       hi.rebase = 1;
       hi.eps = predicted(resid2);
       memset(hi.ticket, 0, sizeof hi.ticket);
-      ESF_CUDA(cudaMemcpyAsync(w->st32, &hi, sizeof hi, cudaMemcpyHostToDevice, st));
-      ESF_CUDA(cudaStreamSynchronize(st));
+      ESF_COUNTED put_state<<<1, 1, 0, st>>>(w->st32, hi);
       kx.iteration(st);  // rebase pass
       ESF_LAUNCH_CHECK();
     }
   } else {
-    ESF_CUDA(cudaMemsetAsync(w->x32, 0, g.R * 4, st));
     {
       PcrState h;
       memset(&h, 0, sizeof h);
@@ -1745,11 +1758,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
       h.maxIt = maxIt;
       h.setup = 1;
       h.inner = 1;
-      ESF_CUDA(cudaMemcpyAsync(w->st32, &h, sizeof h, cudaMemcpyHostToDevice, st));
-      ESF_CUDA(cudaStreamSynchronize(st));
-    }
-    {
-      esf_status e = inner_setup();
+      esf_status e = inner_setup(h, true);
       if (e) return e;
     }
     const bool trace = getenv("ESF_TRACE") != nullptr;
@@ -1773,8 +1782,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
         break;
       }
       // refinement: fold the FP32 partial solution into x, recompute r
-      ESF_COUNTED add_correction<<<vec_blocks(g.R), VT, 0, st>>>(g.R, x, w->x32);
-      ESF_CUDA(cudaMemsetAsync(w->x32, 0, g.R * 4, st));
+      ESF_COUNTED fold_correction<<<vec_blocks(g.R), VT, 0, st>>>(g.R, x, w->x32);
       e = true_residual(&resid2, &bnorm2);
       if (e) return e;
       rel = bnorm > 0 ? sqrt(resid2) / bnorm : sqrt(resid2);
@@ -1798,9 +1806,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
       hi.setup = 1;
       hi.eps = trigger(resid2);
       memset(hi.ticket, 0, sizeof hi.ticket);
-      ESF_CUDA(cudaMemcpyAsync(w->st32, &hi, sizeof hi, cudaMemcpyHostToDevice, st));
-      ESF_CUDA(cudaStreamSynchronize(st));
-      e = inner_setup();
+      e = inner_setup(hi, false);
       if (e) return e;
     }
   }
