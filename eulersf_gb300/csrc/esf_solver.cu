@@ -559,7 +559,7 @@ __global__ void convert_vec(long long n, const A* in, B* out) {
 }
 // Node m^-1 in FP32 with rows padded to `pitch` floats (a multiple of 4, as
 // TMA wants 16-byte row strides); boundary nodes (no unknown) and padding 0.
-__global__ void convert_minv_padded(GridDev g, const double* in, float* out, int pitch) {
+__device__ __forceinline__ void minv_padded(const GridDev& g, const double* in, float* out, int pitch) {
   const long long n = (long long)pitch * g.Y * g.Z;
   for (long long i = blockIdx.x * (long long)VT + threadIdx.x; i < n; i += (long long)gridDim.x * VT) {
     const int x = (int)(i % pitch);
@@ -569,6 +569,31 @@ __global__ void convert_minv_padded(GridDev g, const double* in, float* out, int
     if (x > 0 && x < g.X - 1 && y > 0 && y < g.Y - 1 && z > 0 && z < g.Z - 1)
       v = (float)in[x + (long long)y * g.X + (long long)z * g.slab];
     out[i] = v;
+  }
+}
+__global__ void convert_minv_padded(GridDev g, const double* in, float* out, int pitch) {
+  minv_padded(g, in, out, pitch);
+}
+// What a mixed solve starts from, in one launch (a small one's time is its
+// launches, and a batch's threads take turns at them): 1/diag in FP64 and FP32,
+// the padded m^-1 (minvp not null), ||b||^2 in vec_norm2's order, and the state.
+__global__ void __launch_bounds__(VT) mixed_prepare(GridDev g, const double* diag, const double* minv, const double* b,
+                                                    double* invd, float* invd32, float* minvp, int pitch,
+                                                    double* partial, PcrState* st, const __grid_constant__ PcrState h) {
+  double acc = 0;
+  for (long long i = blockIdx.x * (long long)VT + threadIdx.x; i < g.R; i += (long long)gridDim.x * VT) {
+    const double v = 1.0 / diag[i];
+    invd[i] = v;
+    invd32[i] = (float)v;
+    acc += (double)b[i] * (double)b[i];
+  }
+  if (minvp) minv_padded(g, minv, minvp, pitch);
+  const double bs = block_sum<VT>(acc);
+  double total;
+  if (last_block_sum<VT>(bs, partial, &st->ticket[3], gridDim.x, &total) && threadIdx.x == 0) {
+    PcrState L = h;
+    L.bnorm2 = total;
+    *st = L;
   }
 }
 __global__ void inv_vec(long long n, const double* in, double* out64, float* out32) {
@@ -1143,21 +1168,28 @@ static bool loop_fits(const GridDev& g) {
   return cz <= FL_L && (long long)gr.x * gr.y * gr.z <= slots;
 }
 
+// Whether the TMA kernels take a grid's rows (and are not asked away).
+static bool tma_rows(const GridDev& g) {
+  const char* pick = getenv("ESF_PRESSURE_KERNEL");
+  return g.cX % 4 == 0 && !(pick && strcmp(pick, "register") == 0);
+}
+
 // Chooses the FP32 kernels for the mixed path. The TMA kernels need cell
 // rows that are a multiple of 4 floats (16-byte row strides); with them the
 // one-pass iteration is the default, and ESF_PRESSURE_KERNEL=tma or
 // =register selects the two-kernel split with the TMA-staged or the
 // register-prefetch update kernel (those two give the same bits; both kept
-// for comparison). Converts m^-1 into the padded layout and builds the maps
-// once per work.
+// for comparison). Converts m^-1 (not null) into the padded layout and builds the
+// maps once per work.
 static esf_status prepare_tma(PressureWork* w, const GridDev& g, const double* minv64,
                               cudaStream_t st, const TmaMaps** out, int* path = nullptr) {
   *out = nullptr;
   if (path) *path = P32_REGISTER;
   const char* pick = getenv("ESF_PRESSURE_KERNEL");
-  if (g.cX % 4 != 0 || (pick && strcmp(pick, "register") == 0)) return ESF_OK;
-  ESF_COUNTED convert_minv_padded<<<vec_blocks((long long)w->mpitch * g.Y * g.Z), VT, 0, st>>>(
-      g, minv64, w->minv32p, w->mpitch);
+  if (!tma_rows(g)) return ESF_OK;
+  if (minv64)
+    ESF_COUNTED convert_minv_padded<<<vec_blocks((long long)w->mpitch * g.Y * g.Z), VT, 0, st>>>(
+        g, minv64, w->minv32p, w->mpitch);
   ESF_LAUNCH_CHECK();
   if (!w->tmaOk) {
     static const cudaError_t attr = cudaFuncSetAttribute(
@@ -1510,7 +1542,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     dim3 gr = stencil_grid<double>(g);
     if ((long long)gr.x * gr.y * gr.z > ESF_MAX_PARTIALS) return ESF_ERR_UNSUPPORTED;
   }
-  ESF_COUNTED inv_vec<<<vec_blocks(g.R), VT, 0, st>>>(g.R, diag64, w->invd, w->invd32);
+  if (precision == ESF_FP64) ESF_COUNTED inv_vec<<<vec_blocks(g.R), VT, 0, st>>>(g.R, diag64, w->invd, w->invd32);
   ESF_LAUNCH_CHECK();
   // FP64 PCR from the warm start x (the reference's solvePCR): two kernels
   // per iteration replayed as graphs, true-residual check every 5th.
@@ -1584,7 +1616,16 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
   const TmaMaps* tma = nullptr;
   int path = P32_REGISTER;
   {
-    esf_status e = prepare_tma(w, g, minv64, st, &tma, &path);
+    PcrState h;
+    memset(&h, 0, sizeof h);
+    h.eps = eps;
+    h.maxIt = maxIt;
+    h.setup = 1;
+    ESF_COUNTED mixed_prepare<<<vec_blocks(g.R), VT, 0, st>>>(g, diag64, minv64, b, w->invd, w->invd32,
+                                                              tma_rows(g) ? w->minv32p : nullptr, w->mpitch,
+                                                              w->partial + ESF_MAX_PARTIALS / 2, w->st, h);
+    ESF_LAUNCH_CHECK();
+    esf_status e = prepare_tma(w, g, nullptr, st, &tma, &path);
     if (e) return e;
   }
   if (path != P32_FUSED)  // (the one-pass kernels read the padded copy)
@@ -1617,14 +1658,6 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     ESF_LAUNCH_CHECK();
     return ESF_OK;
   };
-  // ||b||
-  {
-    esf_status e = init_state(w->st, eps, maxIt, st);
-    if (e) return e;
-  }
-  ESF_COUNTED vec_norm2<double><<<vec_blocks(g.R), VT, 0, st>>>(g.R, b, w->partial + ESF_MAX_PARTIALS / 2,
-                                                    &w->st->ticket[3], &w->st->bnorm2);
-  ESF_LAUNCH_CHECK();
   // r64 = b - A x (FP64), r32 = (b - A x)/diag in FP32, ||r64||^2
   auto true_residual = [&](double* resid2, double* bnorm2) -> esf_status {
     StencilArgs<double> a;
