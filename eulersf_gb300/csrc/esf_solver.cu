@@ -871,8 +871,9 @@ esf_status pressure_apply(const GridDev& g, const T* minv, const T* in, T* out, 
   a.minv = minv;
   a.out = out;
   if constexpr (std::is_same<T, double>::value) {
-    if (fixed_pays(g)) {
-      launch_fixed<S_APPLY>(g, a, st);
+    FixedShape shape;
+    if (fixed_pays(g, &shape)) {
+      launch_fixed<S_APPLY>(g, a, shape, st);
       ESF_LAUNCH_CHECK();
       return ESF_OK;
     }
@@ -1332,7 +1333,8 @@ struct PressureKernels {
   double* partial;
   PcrState* st;
   const TmaMaps* tma = nullptr;  // FP32 only: TMA-staged update kernel
-  bool fixed = false;            // FP64 only: the stencil on integers
+  bool fixed = false;            // FP64 only: the stencil on integers, and its launch shape
+  FixedShape shape{};
   void setup_warm(cudaStream_t cs) const {  // r = (b - Ax)/diag, ||b||; then s = Ar, delta
     StencilArgs<T> a;
     memset(&a, 0, sizeof a);
@@ -1366,7 +1368,7 @@ struct PressureKernels {
   bool stencil(const StencilArgs<T>& a, cudaStream_t cs) const {
     if constexpr (std::is_same<T, double>::value) {
       if (fixed) {
-        launch_fixed<MODE>(g, a, cs);
+        launch_fixed<MODE>(g, a, shape, cs);
         return true;
       }
     }
@@ -1505,9 +1507,9 @@ static esf_status init_state(PcrState* d, double eps, int maxIt, cudaStream_t st
 // grid for which that pays, and bounds of x and 1/m, which this leaves in the
 // state, far from the ends of the exponent range.
 static esf_status fixed_start(const GridDev& g, const double* minv, const double* x, PcrState* st, cudaStream_t cs,
-                              bool* fixed) {
+                              bool* fixed, FixedShape* shape) {
   *fixed = false;
-  if (!fixed_pays(g)) return ESF_OK;
+  if (!fixed_pays(g, shape)) return ESF_OK;
   ESF_COUNTED fixed_bounds<<<vec_blocks(g.T), 256, 0, cs>>>(g, x, minv, &st->hx, &st->hm);
   ESF_LAUNCH_CHECK();
   unsigned h[2];
@@ -1565,7 +1567,7 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     PressureKernels<double> k{g, pm, w->invd, pb, px, w->r, w->d, w->Ap, w->s, w->partial, w->st};
     {
       esf_status e = init_state(w->st, eps, itCap, st);
-      if (!e) e = fixed_start(g, pm, px, w->st, st, &k.fixed);
+      if (!e) e = fixed_start(g, pm, px, w->st, st, &k.fixed, &k.shape);
       if (e) return e;
     }
     if (w->perCall && !copies)
@@ -3167,7 +3169,7 @@ esf_status pressure_solve_static(void* scratch, const GridDev& g, const double* 
   }
   PressureKernels<double> k{g, minv, invd, b, x, r, d, Ap, s, partial, state};
   {
-    esf_status e = fixed_start(g, minv, x, state, st, &k.fixed);
+    esf_status e = fixed_start(g, minv, x, state, st, &k.fixed, &k.shape);
     if (e) return e;
   }
   k.setup_warm(st);

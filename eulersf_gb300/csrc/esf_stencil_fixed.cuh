@@ -19,9 +19,9 @@
 // Bound: instruction issue (192^3 UPDATE: 127 M warp instructions, half a one a
 // cycle and scheduler, its three warps waiting on their own chains; DRAM at a
 // third). Measured against pressure_stencil<double>, whose bound is the FP64
-// pipe: product 32^3 19.1 -> 8.1 us, 64^3 29.5 -> 17.6, 128^3 159 -> 65,
-// 161x127x190 343 -> 104, 256^3 1154 -> 377; solve iteration (phase A included)
-// 34.7 -> 21, 57.8 -> 36, 260 -> 133, 499 -> 215, 1749 -> 783 us. Error of a
+// pipe: product 32^3 19.1 -> 8.2 us, 64^3 29.5 -> 18.9, 128^3 159 -> 64,
+// 161x127x190 343 -> 106, 256^3 1154 -> 390; solve iteration (phase A included)
+// 34.7 -> 19, 57.8 -> 34, 260 -> 124, 499 -> 212, 1749 -> 746 us. Error of a
 // product against extended precision: 3/4 of the FP64 kernel's (2-norm).
 #pragma once
 
@@ -312,27 +312,45 @@ __global__ void __launch_bounds__(256) fixed_bounds(GridDev g, const double* x, 
   }
 }
 
-// Launch shape: rows a warp, and the z-chunk depth from the warps wanted an SM.
-// More rows share halo rows and conversions, fewer give small grids warps (solve
-// iteration, 2 against 4 rows: 32^3 22 and 26 us, 64^3 50 and 54, 96^3 87 and
-// 85, 256^3 equal, its product 431 and 377). Twelve warps an SM are resident;
-// chunks pay two extra layers each, so small grids take one wave of them and
-// large ones more, for the tail (12, 24, 48 warps: 64^3 54, 60, 60 us, 96^3 85,
-// 92, 99, 128^3 160, 146, 164, 161x127x190 287, 222, 240, 256^3 953, 850, 802).
+// Launch shape: rows a warp and z-chunk depth, the ones of least cost in a model
+// of what was measured. A block marches cz + 2 layers, and half of one is its
+// start and end. An SM holds three blocks, so each of its schedulers one to three
+// of their warps: a warp alone issues every 4.5 cycles, two hardly disturb each
+// other, three share half an issue a cycle (cost of a layer 4.5, 4.7 and 6); more
+// blocks run in waves of three. Four rows a warp are 1.65 times two rows'
+// instructions. Solve iteration, against fixed numbers of warps by size: 80^3 53.3
+// -> 46.3 us, 128^3 130 -> 124, 144^3 178 -> 159, 256^3 781 -> 746, 32x33x300
+// 62.8 -> 46.3, 64^3 the same, 72^3 40.1 -> 42.5.
 struct FixedShape {
   int ry, cz;
   dim3 grid;
 };
 static FixedShape fixed_shape(const GridDev& g) {
-  FixedShape s;
-  const int ry = s.ry = g.R < 600000 ? 2 : 4;
-  const int warps = g.R < 1500000 ? 12 : g.R < 8000000 ? 24 : 48;
-  const long long cols = (long long)((g.cX + FX_COLS - 1) / FX_COLS) * ((g.cY + ry - 1) / ry);
-  int n = (int)((warps * 152 + cols - 1) / cols);
-  n = n < 1 ? 1 : n > g.cZ ? g.cZ : n;
-  s.cz = (g.cZ + n - 1) / n;
-  s.grid = dim3((g.cX + FX_COLS - 1) / FX_COLS, (g.cY + FX_W * ry - 1) / (FX_W * ry), (g.cZ + s.cz - 1) / s.cz);
-  return s;
+  FixedShape best{};
+  double least = 0;
+  const long long gx = (g.cX + FX_COLS - 1) / FX_COLS;
+  for (int ry = 2; ry <= 4; ry += 2) {
+    const long long gy = (g.cY + FX_W * ry - 1) / (FX_W * ry), gxy = gx * gy;
+    // the most chunks that a number of blocks an SM leaves room for
+    const int last = (int)((gxy + 151) / 152 + 2) / 3 * 3 + 12;
+    for (int k = 1; k <= last; k += k < 3 ? 1 : 3) {
+      long long n = 152LL * k / gxy;
+      if (n < 1) continue;
+      if (n > g.cZ) n = g.cZ;
+      const int cz = (int)((g.cZ + n - 1) / n), gz = (g.cZ + cz - 1) / cz;
+      const int per = (int)((gxy * gz + 151) / 152);
+      const double rest[3] = {0.0, 4.5, 4.7};
+      const double cost = (cz + 2.5) * ((per / 3) * 6.0 + rest[per % 3]) * (ry == 2 ? 1.0 : 1.65);
+      if (!best.ry || cost < least) {
+        least = cost;
+        best.ry = ry;
+        best.cz = cz;
+        best.grid = dim3((unsigned)gx, (unsigned)gy, (unsigned)gz);
+      }
+      if (n == g.cZ) break;
+    }
+  }
+  return best;
 }
 template <int MODE, int RY>
 static void launch_fixed_rows(const GridDev& g, const StencilArgs<double>& a, const FixedShape& s, cudaStream_t st) {
@@ -343,8 +361,7 @@ static void launch_fixed_rows(const GridDev& g, const StencilArgs<double>& a, co
   ESF_COUNTED pressure_stencil_fixed<MODE, RY><<<s.grid, FX_T, smem, st>>>(g, a, s.cz);
 }
 template <int MODE>
-static void launch_fixed(const GridDev& g, const StencilArgs<double>& a, cudaStream_t st) {
-  const FixedShape s = fixed_shape(g);
+static void launch_fixed(const GridDev& g, const StencilArgs<double>& a, const FixedShape& s, cudaStream_t st) {
   if (s.ry == 2) launch_fixed_rows<MODE, 2>(g, a, s, st);
   else launch_fixed_rows<MODE, 4>(g, a, s, st);
 }
@@ -354,8 +371,8 @@ static void launch_fixed(const GridDev& g, const StencilArgs<double>& a, cudaStr
 // 8192 cells, where a step is its launches, FP64 in pressure_stencil's order
 // stays, whose results to the last bit whole steps on such grids are compared
 // by. More blocks than the sums have room for stay too.
-static bool fixed_pays(const GridDev& g) {
+static bool fixed_pays(const GridDev& g, FixedShape* s) {
   if (g.R < 8192) return false;
-  const FixedShape s = fixed_shape(g);
-  return (long long)s.grid.x * s.grid.y * s.grid.z <= FX_MAX_BLOCKS && s.grid.y <= 65535 && s.grid.z <= 65535;
+  *s = fixed_shape(g);
+  return (long long)s->grid.x * s->grid.y * s->grid.z <= FX_MAX_BLOCKS && s->grid.y <= 65535 && s->grid.z <= 65535;
 }
