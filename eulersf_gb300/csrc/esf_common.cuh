@@ -116,6 +116,7 @@ struct PcrState {
   // fixed-point FP64 stencil: bounds as high words (fixed_mag) of x, 1/m, the
   // stencil's input r - alpha Ap/diag, and what phase A collects for that
   unsigned int hx, hm, hv, hr, hq;
+  double limit;  // one-pass FP32 iteration: eps^2 delta0, below which it stops
 };
 
 // Solid system layout ("sliced"): the 27 neighbour 3x3 blocks of solid node a,

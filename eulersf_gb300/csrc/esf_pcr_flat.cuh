@@ -11,16 +11,20 @@
 //    to the next; r, t and q go through memory, because the neighbours read them,
 //    and come back in three copies (one box a vector), which are on their way
 //    while the sums are folded: they need no scalar of the new pass;
-//  * a grid barrier, after which every block folds the sums for itself.
+//  * a grid barrier, after which every block folds the sums for itself, a warp a
+//    sum.
 //
 //   (a) group by layer: r' at tile and halo into V; own layers: x, d, q, r
 //   (b) group by own layer: the two node layers around it, their sums A, B, C
 //   (c) s', t' of the own layer, and what the sums are formed from
 //   (d) group by sum: over the layers in fused_pass's order
 // Bound: latencies (128 blocks at 64^3, one an SM; its 12 words a row are 2 us of
-// L2). An iteration against a launch of fused_pass each: 12.4 -> 7.9 us at 32^3,
-// 12.4 -> 8.2 at 64^3, in double-float 14.3 -> 9.5 and 15.1 -> 10.0. fused_pass
-// itself in a loop gave 12.0 at 64^3, 21.2 for 19.0 at 96^3, 26.7 for 24.7 at
+// L2). An iteration against a launch of fused_pass each: 12.4 -> 7.1 us at 32^3,
+// 12.4 -> 7.7 at 64^3, in double-float 14.3 -> 8.4 and 15.1 -> 9.4 (8.2 at 64^3
+// with the sums by eight warps in turn; 8.1 with one thread for barrier and
+// copies). At 64^3 it is some 16000 cycles: (a) to (d) a third, block sums, folds
+// and scalars, whose FP64 instructions take 63 cycles each, two fifths, the
+// barrier a fifth. fused_pass itself in a loop gave 12.0 at 64^3, 21.2 for 19.0 at 96^3, 26.7 for 24.7 at
 // 128^3: the launches in a graph cost a microsecond, the barrier as much.
 #pragma once
 
@@ -36,19 +40,18 @@ struct FlatMaps {
 constexpr int FL_RB = FL_H * TMA_HALO_BYTES, FL_MB = (FL_L + 1) * TMA_NODE_BYTES;
 constexpr int FL_VP = TW_PP * HY;        // V of a layer, laid out as sP
 constexpr int FL_NP = TW_NP * NYN;
+constexpr int FL_SP = 8 * 33 + 4;        // a sum's values, warp w's at 33 w
 constexpr int FL_OFF_R = 0, FL_OFF_M = 3 * FL_RB, FL_OFF_V = FL_OFF_M + (FL_MB + 127) / 128 * 128,
               FL_OFF_K = FL_OFF_V + FL_H * FL_VP * 4, FL_OFF_S = FL_OFF_K + 10 * NT * FL_L * 4,
-              FL_OFF_RED = FL_OFF_S + FU_SUMS * NT * 4, FL_OFF_BAR = FL_OFF_RED + 32 * 8, FL_SMEM = FL_OFF_BAR + 16;
+              FL_OFF_T = FL_OFF_S + FU_SUMS * FL_SP * 4, FL_OFF_BAR = FL_OFF_T + FU_SUMS * 8, FL_SMEM = FL_OFF_BAR + 16;
 static_assert(FL_RB % 128 == 0 && FL_OFF_M % 128 == 0 && FL_OFF_V % 16 == 0 && FL_OFF_K % 16 == 0 &&
-                  FL_OFF_RED % 16 == 0, "layout");
+                  FL_OFF_T % 16 == 0, "layout");
 // (b) writes A, B, C over r, t and q, which (a) is done with
 static_assert(FL_L * 3 * FL_NP * 4 <= FL_OFF_M, "overlay");
 
-// Arrival of all blocks at the next pass: a release add on a counter, then
-// acquire loads, bounded; by thread 0.
-__device__ __forceinline__ bool flat_barrier(PcrState* st, unsigned target) {
+// Arrival of all blocks at the next pass: polls of the counter they add to, bounded.
+__device__ __forceinline__ bool flat_wait(PcrState* st, unsigned target) {
   unsigned cur, it = 0, bad = 0;
-  asm volatile("red.add.release.gpu.global.u32 [%0], 1;" ::"l"(&st->ticket[2]) : "memory");
   do {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(&st->ticket[2]) : "memory");
     if ((++it & 1023u) == 0) {
@@ -58,6 +61,23 @@ __device__ __forceinline__ bool flat_barrier(PcrState* st, unsigned target) {
   } while ((int)(cur - target) < 0 && !bad);
   return !bad;
 }
+// block_sum's tree over 256 values by one warp: value(w, i) is lane i's of warp w.
+template <typename F>
+__device__ __forceinline__ double flat_tree(F value) {
+  const int lane = threadIdx.x & 31, w = lane & 7, i = lane >> 3;
+  double t[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) t[k] = value(w, i + 4 * k);
+#pragma unroll
+  for (int h = 4; h > 0; h /= 2)
+#pragma unroll
+    for (int k = 0; k < h; k++) t[k] += t[k + h];
+  double r = t[0];
+  for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return r;
+}
+// the first four warps, one on each of the SM's schedulers
+__device__ __forceinline__ void flat_sync4() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 template <bool X64>
 __global__ void __launch_bounds__(FL_G* NT, 1)
@@ -65,13 +85,13 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
                   float* ddf, double* partial, PcrState* st, int cz, int budget) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ PcrState L;
-  __shared__ int go;
+  __shared__ int go, arrived;
   static_assert(FL_G == FL_L && FL_G == FU_SUMS, "a group for each own layer and each sum");
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + FL_OFF_BAR);
-  double* sred = reinterpret_cast<double*>(smem + FL_OFF_RED);
   float* sV = reinterpret_cast<float*>(smem + FL_OFF_V);
   float* sK = reinterpret_cast<float*>(smem + FL_OFF_K);  // [layer][10][NT]
-  float* sS = reinterpret_cast<float*>(smem + FL_OFF_S);  // [sum][NT]
+  float* sS = reinterpret_cast<float*>(smem + FL_OFF_S);  // [sum][FL_SP]
+  double* sT = reinterpret_cast<double*>(smem + FL_OFF_T);  // [sum]
   float* sN = reinterpret_cast<float*>(smem + FL_OFF_R);  // [layer][A, B, C]
   const int nb = gridDim.x * gridDim.y * gridDim.z;
   const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
@@ -90,7 +110,7 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
   __syncthreads();
   if (L.done) return;
   const unsigned base = L.ticket[0];
-  auto fetch = [&](int set) {  // by thread 0
+  auto fetch = [&](int set) {  // by one thread
     asm volatile("fence.proxy.async;" ::: "memory");  // (what the blocks wrote before the barrier)
     mbar_expect_tx(&bar[0], 3 * FL_RB);
     tma_load_3d(smem + FL_OFF_R, set ? &tm.r[1] : &tm.r[0], x0 - 4, y0 - 1, z0 - 1, &bar[0]);
@@ -154,16 +174,17 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
     float* tOut = pout ? p.t[1] : p.t[0];
     // (a) r' = r - alpha (t + beta q)
     float2 vo = make_float2(0.f, 0.f), qo = vo;
-    auto layer_in = [&](int h, bool mine) {
+    auto layer_in = [&](int h, bool mine, bool tile, bool ring) {
       const float* R = reinterpret_cast<const float*>(smem + FL_OFF_R + h * TMA_HALO_BYTES);
       const float *Tt = R + FL_RB / 4, *Qq = R + 2 * (FL_RB / 4);
+      if (ring && hasE) sV[h * FL_VP + pE] = __fmaf_rn(-alpha, __fmaf_rn(beta, Qq[bE], Tt[bE]), R[bE]);
+      if (!tile) return;
       const float2 r2 = *reinterpret_cast<const float2*>(R + bM);
       const float2 t2 = *reinterpret_cast<const float2*>(Tt + bM);
       const float2 q2 = *reinterpret_cast<const float2*>(Qq + bM);
       const float qn0 = rb ? q2.x : __fmaf_rn(beta, q2.x, t2.x), qn1 = rb ? q2.y : __fmaf_rn(beta, q2.y, t2.y);
       const float v0 = __fmaf_rn(-alpha, qn0, r2.x), v1 = __fmaf_rn(-alpha, qn1, r2.y);
       *reinterpret_cast<float2*>(sV + h * FL_VP + pM) = make_float2(v0, v1);
-      if (hasE) sV[h * FL_VP + pE] = __fmaf_rn(-alpha, __fmaf_rn(beta, Qq[bE], Tt[bE]), R[bE]);
       if (!mine) return;
       if constexpr (X64) {
         const float2 dn0 = rb ? make_float2(ds.x, ds.y) : df_axpy(beta, make_float2(ds.x, ds.y), r2.x);
@@ -183,9 +204,9 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
       vo = make_float2(v0, v1);
       qo = make_float2(qn0, qn1);
     };
-    if (grp < layers) layer_in(grp + 1, own);
-    if (grp == FL_G - 1) layer_in(0, false);
-    if (grp == FL_G - 2) layer_in(layers + 1, false);
+    if (grp < layers) layer_in(grp + 1, own, true, true);
+    // the layers around: tile and ring to a group each
+    layer_in(grp < 2 ? 0 : layers + 1, false, grp & 1, !(grp & 1));
     if (__syncthreads_or(!ok)) break;
 
     // (b) J^T r' scaled by m^-1 on the node layers below and above the own layer
@@ -290,51 +311,66 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
       float* q = sK + grp * 10 * NT + tid;
       q[0] = vo.x;
       q[NT] = vo.y;
-      q[2 * NT] = o0;
-      q[3 * NT] = o1;
-      q[4 * NT] = t0;
-      q[5 * NT] = t1;
-      q[6 * NT] = qo.x;
-      q[7 * NT] = qo.y;
-      q[8 * NT] = iv.x;
-      q[9 * NT] = iv.y;
+      q[2 * NT] = t0;
+      q[3 * NT] = t1;
+      q[4 * NT] = qo.x;
+      q[5 * NT] = qo.y;
+      q[6 * NT] = iv.x;
+      q[7 * NT] = iv.y;
+      q[8 * NT] = o0;
+      q[9 * NT] = o1;
     }
     __syncthreads();
 
     // (d) (r', s'), (s', t'), (s', q), (Ap, q)
     float sum = 0;
     if (cin) {
-      const float* q = sK + tid;
-      const int a = grp == 0 ? 0 : grp == 1 ? 4 : 6;  // r', t', q of the first three
+      const float* q = sK + 2 * grp * NT + tid;
       for (int l = 0; l < layers; l++, q += 10 * NT) {
+        const float a0 = q[0], a1 = q[NT];
         if (grp == 3) {
-          const float q0 = q[6 * NT], q1 = q[7 * NT], iv0 = q[8 * NT], iv1 = q[9 * NT];
-          if (iv0 > 0.0f) sum += __fdividef(q0 * q0, iv0);
-          if (iv1 > 0.0f) sum += __fdividef(q1 * q1, iv1);
+          // (quotients in the expressions that fused_pass has: formed earlier they
+          // round differently)
+          const float q0 = q[-2 * NT], q1 = q[-NT];
+          if (a0 > 0.0f) sum += __fdividef(q0 * q0, a0);
+          if (a1 > 0.0f) sum += __fdividef(q1 * q1, a1);
         } else {
-          const float a0 = q[a * NT], a1 = q[(a + 1) * NT], o0 = q[2 * NT], o1 = q[3 * NT];
-          sum += a0 * o0 + a1 * o1;
+          const float* o = sK + (10 * l + 8) * NT + tid;
+          sum += a0 * o[0] + a1 * o[NT];
         }
       }
     }
-    sS[grp * NT + tid] = sum;
+    sS[grp * FL_SP + w * 33 + lane] = sum;
     __syncthreads();
-    double* part = partial + (pass & 1) * FU_SUMS * nb;  // (a block can be a pass ahead of another's fold)
-    const float sums[FU_SUMS] = {sS[tid], sS[NT + tid], sS[2 * NT + tid], sS[3 * NT + tid]};
-    put4(sums, part, nb, bid, sred);
-    if (threadIdx.x == 0) {
-      go = flat_barrier(st, base + (unsigned)(pass + 1) * nb);
-      if (go) fetch(pout);
+    // a warp a sum, on schedulers of their own; a fifth fetches
+    const unsigned target = base + (unsigned)(pass + 1) * nb;
+    if (threadIdx.x < 128) {
+      const int h = threadIdx.x >> 5;
+      // (a block can be a pass ahead of another's fold)
+      double* part = partial + ((pass & 1) * FU_SUMS + h) * nb;
+      const float* mine = sS + h * FL_SP;
+      const double ps = flat_tree([&](int a, int i) { return widen(mine[a * 33 + i]); });
+      if (lane == 0) __stcg(part + bid, ps);
+      flat_sync4();
+      if (threadIdx.x == 0) {
+        asm volatile("red.add.release.gpu.global.u32 [%0], 1;" ::"l"(&st->ticket[2]) : "memory");
+        go = flat_wait(st, target);  // (one poller: four in each block were slower)
+      }
+      flat_sync4();
+      const double total =
+          flat_tree([&](int a, int i) { return a * 32 + i < nb ? __ldcg(part + a * 32 + i) : 0.0; });
+      if (lane == 0) sT[h] = total;
+      flat_sync4();
+      if (threadIdx.x == 0) finish_fused(&L, sT[0], sT[1], sT[2], sT[3]);
+    } else if (threadIdx.x == 128) {
+      arrived = flat_wait(st, target);
+      if (arrived) fetch(pout);
     }
     __syncthreads();
-    if (!go) break;
-    const double total = fold4(part, nb, sred);
-    if (threadIdx.x < 32) {
-      const double tMu = __shfl_sync(0xffffffffu, total, 8), tNu = __shfl_sync(0xffffffffu, total, 16),
-                   tOm = __shfl_sync(0xffffffffu, total, 24);
-      if (threadIdx.x == 0) finish_fused(&L, total, tMu, tNu, tOm);
+    if (!go || !arrived) {
+      if (arrived) mbar_wait(&bar[0], (pass + 1) & 1);
+      break;
     }
-    __syncthreads();
   }
   // a block that gave up on a copy or on the others: an error, and they give up too
   const bool stopped = pass == budget || L.done || L.iter >= L.maxIt;

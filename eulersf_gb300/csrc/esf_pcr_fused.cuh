@@ -67,6 +67,10 @@ constexpr int FU_SUMS = 4;                    // delta, mu, nu, omega
 __device__ __forceinline__ bool is_nan(double v) {
   return (unsigned)(__double2hiint(v) & 0x7fffffff) + (__double2loint(v) != 0) > 0x7ff00000u;
 }
+__device__ __forceinline__ bool at_most(double v, double limit) {  // (limit not negative)
+  const long long a = __double_as_longlong(v), b = __double_as_longlong(limit);
+  return !is_nan(v) && !is_nan(limit) && (a < 0 || a <= b);
+}
 __device__ __forceinline__ bool is_positive(double v) {
   return __double_as_longlong(v) > 0 && !is_nan(v);
 }
@@ -85,6 +89,7 @@ __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu,
     st->alpha = is_positive(den) ? dl / den : 0.0;
     st->delta = dl;
     st->delta0 = dl;
+    st->limit = st->eps * st->eps * dl;
     st->rebase = 0;
     st->iter++;
     st->iter0 = st->iter;
@@ -95,6 +100,7 @@ __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu,
   } else if (st->setup) {
     st->delta = dl;
     st->delta0 = dl;
+    st->limit = st->eps * st->eps * dl;
     st->beta = 0.0;
     st->alpha = (mu > 0.0) ? dl / mu : 0.0;  // first direction is r: (Ap, Ap/diag) = mu
     st->setup = 0;
@@ -112,7 +118,7 @@ __device__ __forceinline__ void finish_fused(PcrState* st, double dl, double mu,
     st->deltaPrev = st->delta;
     st->delta = dl;
     st->iter++;
-    if (dl <= st->eps * st->eps * st->delta0 || (st->cap > 0 && st->iter - st->iter0 >= st->cap)) {
+    if (at_most(dl, st->limit) || (st->cap > 0 && st->iter - st->iter0 >= st->cap)) {
       st->converged = 1;
       st->done = 1;
     }
