@@ -1146,7 +1146,7 @@ enum Fp32Path {
 // Whether a grid's iterations run in loops (pcr_loop_flat): chunks of FL_L layers
 // at most, and one block an SM for a pass (64^3 cells and less), the first
 // condition for the kernel's shared memory, the second for its barrier. Where
-// both hold it is the faster one (8.2 against 12.4 us an iteration at 64^3).
+// both hold it is the faster one (7.7 against 12.4 us an iteration at 64^3).
 // ESF_PRESSURE_KERNEL=pass takes a launch an iteration everywhere (for
 // comparison; same bits).
 static bool loop_fits(const GridDev& g) {
@@ -2632,6 +2632,7 @@ struct InnerBatcher {
   int slotRefs[kSlots] = {};
   std::map<Shape, Lane> lanes;
   std::map<std::array<int, 3>, int> attached;  // works attached, by grid shape (cells per axis)
+  std::map<std::array<int, 3>, std::chrono::steady_clock::time_point> left;  // when one was last detached
   std::mutex m;
   std::condition_variable cv, doneCv;
   std::deque<Job*> pending;
@@ -2965,6 +2966,7 @@ esf_status pressure_work_set_batcher(PressureWork* w, InnerBatcher* b) {
   if (w->batcher) {
     std::lock_guard<std::mutex> g(w->batcher->m);
     w->batcher->attached[shape]--;
+    w->batcher->left[shape] = std::chrono::steady_clock::now();
   }
   w->batcher = b;
   if (b) {
@@ -2980,7 +2982,9 @@ esf_status pressure_work_set_batcher(PressureWork* w, InnerBatcher* b) {
 // on the 48^3-160^3 serving mix: 6.9 scene-steps/s batching every shape
 // against 7.6 unbatched), and only while another work of the same grid shape
 // is attached (a task alone in its lane gains nothing over the scene's own
-// captured graphs).
+// launches) or was within the last second: requests of a shape come one after
+// another, and a scene that is through between two others is not a reason to
+// leave the lane.
 static bool batching_pays(PressureWork* w) {
   if (!w->batcher) return false;
   static const int slots = [] {
@@ -2996,8 +3000,11 @@ static bool batching_pays(PressureWork* w) {
   const dim3 gr = tma_grid(w->g, fused_cz(w->g));
   if ((long long)gr.x * gr.y * gr.z * 4 > slots) return false;
   std::lock_guard<std::mutex> g(w->batcher->m);
-  auto it = w->batcher->attached.find({w->g.cX, w->g.cY, w->g.cZ});
-  return it != w->batcher->attached.end() && it->second >= 2;
+  const std::array<int, 3> shape = {w->g.cX, w->g.cY, w->g.cZ};
+  auto it = w->batcher->attached.find(shape);
+  if (it != w->batcher->attached.end() && it->second >= 2) return true;
+  auto gone = w->batcher->left.find(shape);
+  return gone != w->batcher->left.end() && std::chrono::steady_clock::now() - gone->second < std::chrono::seconds(1);
 }
 
 // One inner solve of a scene through the batcher: the set-up pass has been
