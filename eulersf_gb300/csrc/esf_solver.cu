@@ -872,7 +872,7 @@ esf_status pressure_apply(const GridDev& g, const T* minv, const T* in, T* out, 
   a.out = out;
   if constexpr (std::is_same<T, double>::value) {
     FixedShape shape;
-    if (fixed_pays(g, &shape)) {
+    if (fixed_pays(g, false, &shape)) {
       launch_fixed<S_APPLY>(g, a, shape, st);
       ESF_LAUNCH_CHECK();
       return ESF_OK;
@@ -1509,7 +1509,7 @@ static esf_status init_state(PcrState* d, double eps, int maxIt, cudaStream_t st
 static esf_status fixed_start(const GridDev& g, const double* minv, const double* x, PcrState* st, cudaStream_t cs,
                               bool* fixed, FixedShape* shape) {
   *fixed = false;
-  if (!fixed_pays(g, shape)) return ESF_OK;
+  if (!fixed_pays(g, true, shape)) return ESF_OK;
   ESF_COUNTED fixed_bounds<<<vec_blocks(g.T), 256, 0, cs>>>(g, x, minv, &st->hx, &st->hm);
   ESF_LAUNCH_CHECK();
   unsigned h[2];

@@ -21,7 +21,7 @@
 // third). Measured against pressure_stencil<double>, whose bound is the FP64
 // pipe: product 32^3 19.1 -> 8.2 us, 64^3 29.5 -> 18.9, 128^3 159 -> 64,
 // 161x127x190 343 -> 106, 256^3 1154 -> 390; solve iteration (phase A included)
-// 34.7 -> 19, 57.8 -> 34, 260 -> 124, 499 -> 212, 1749 -> 746 us. Error of a
+// 34.7 -> 19, 57.8 -> 34, 260 -> 121, 499 -> 201, 1749 -> 733 us. Error of a
 // product against extended precision: 3/4 of the FP64 kernel's (2-norm).
 #pragma once
 
@@ -97,8 +97,11 @@ __device__ __forceinline__ unsigned fixed_bound(unsigned hr, unsigned hq, double
   const double b = from_words(hr, ~0u) + fabs(alpha) * from_words(hq, ~0u);
   return fixed_mag(b * 1.0000001);
 }
+// blocks an SM holds: the products' scan wants the registers, the solves' modes fit four
+template <int MODE>
+constexpr int FX_RESIDENT = MODE == S_APPLY ? 3 : 4;
 template <int MODE, int RY>
-__global__ void __launch_bounds__(FX_T, 3) pressure_stencil_fixed(GridDev g, StencilArgs<double> a, int cz) {
+__global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixed(GridDev g, StencilArgs<double> a, int cz) {
   extern __shared__ double ring[];  // [2][slots][FX_T]
   if (MODE != S_APPLY && a.st->done) return;
   constexpr int SLOTS = fx_slots<MODE, RY>();
@@ -314,33 +317,36 @@ __global__ void __launch_bounds__(256) fixed_bounds(GridDev g, const double* x, 
 
 // Launch shape: rows a warp and z-chunk depth, the ones of least cost in a model
 // of what was measured. A block marches cz + 2 layers, and half of one is its
-// start and end. An SM holds three blocks, so each of its schedulers one to three
-// of their warps: a warp alone issues every 4.5 cycles, two hardly disturb each
-// other, three share half an issue a cycle (cost of a layer 4.5, 4.7 and 6); more
-// blocks run in waves of three. Four rows a warp are 1.65 times two rows'
-// instructions. Solve iteration, against fixed numbers of warps by size: 80^3 53.3
-// -> 46.3 us, 128^3 130 -> 124, 144^3 178 -> 159, 256^3 781 -> 746, 32x33x300
-// 62.8 -> 46.3, 64^3 the same, 72^3 40.1 -> 42.5.
+// start and end. An SM holds three blocks of a product's kernel, four of a
+// solve's, so each of its schedulers as many of their warps: a warp alone issues
+// every 4.5 cycles, two hardly disturb each other, three share half an issue a
+// cycle (cost of a layer 4.5, 4.7, 6 and 7.5); more blocks run in waves. Products
+// take two rows a warp or four (1.65 times the instructions of two), solves two:
+// with four an iteration took 65 us for 61 at 96^3, 212 for 201 at 161x127x190,
+// 745 for 733 at 256^3. Against fixed numbers of warps by size, an iteration takes
+// 41 for 53 us at 80^3, 121 for 130 at 128^3, 44 for 63 at 32x33x300; 64^3 the same.
 struct FixedShape {
   int ry, cz;
   dim3 grid;
 };
-static FixedShape fixed_shape(const GridDev& g) {
+static FixedShape fixed_shape(const GridDev& g, bool solve) {
   FixedShape best{};
   double least = 0;
   const long long gx = (g.cX + FX_COLS - 1) / FX_COLS;
-  for (int ry = 2; ry <= 4; ry += 2) {
+  const int resident = solve ? FX_RESIDENT<S_UPDATE> : FX_RESIDENT<S_APPLY>;
+  const double layer[5] = {0.0, 4.5, 4.7, 6.0, 7.5};
+  for (int ry = 2; ry <= (solve ? 2 : 4); ry += 2) {
     const long long gy = (g.cY + FX_W * ry - 1) / (FX_W * ry), gxy = gx * gy;
     // the most chunks that a number of blocks an SM leaves room for
-    const int last = (int)((gxy + 151) / 152 + 2) / 3 * 3 + 12;
-    for (int k = 1; k <= last; k += k < 3 ? 1 : 3) {
+    const int last = (int)((gxy + 151) / 152) + 5 * resident;
+    for (int k = 1; k <= last; k += k < resident ? 1 : resident) {
       long long n = 152LL * k / gxy;
-      if (n < 1) continue;
+      if (n < 1) n = 1;
       if (n > g.cZ) n = g.cZ;
       const int cz = (int)((g.cZ + n - 1) / n), gz = (g.cZ + cz - 1) / cz;
       const int per = (int)((gxy * gz + 151) / 152);
-      const double rest[3] = {0.0, 4.5, 4.7};
-      const double cost = (cz + 2.5) * ((per / 3) * 6.0 + rest[per % 3]) * (ry == 2 ? 1.0 : 1.65);
+      const double cost = (cz + 2.5) * ((per / resident) * layer[resident] + layer[per % resident]) *
+                          (ry == 2 ? 1.0 : 1.65);
       if (!best.ry || cost < least) {
         least = cost;
         best.ry = ry;
@@ -362,8 +368,13 @@ static void launch_fixed_rows(const GridDev& g, const StencilArgs<double>& a, co
 }
 template <int MODE>
 static void launch_fixed(const GridDev& g, const StencilArgs<double>& a, const FixedShape& s, cudaStream_t st) {
-  if (s.ry == 2) launch_fixed_rows<MODE, 2>(g, a, s, st);
-  else launch_fixed_rows<MODE, 4>(g, a, s, st);
+  if constexpr (MODE == S_APPLY) {
+    if (s.ry == 4) {
+      launch_fixed_rows<MODE, 4>(g, a, s, st);
+      return;
+    }
+  }
+  launch_fixed_rows<MODE, 2>(g, a, s, st);
 }
 // Whether a grid's FP64 products and solves use it. It is the faster one at
 // every size and shape measured: 8^3 8.1 against 19.2 us a product, 20 against
@@ -371,8 +382,8 @@ static void launch_fixed(const GridDev& g, const StencilArgs<double>& a, const F
 // 8192 cells, where a step is its launches, FP64 in pressure_stencil's order
 // stays, whose results to the last bit whole steps on such grids are compared
 // by. More blocks than the sums have room for stay too.
-static bool fixed_pays(const GridDev& g, FixedShape* s) {
+static bool fixed_pays(const GridDev& g, bool solve, FixedShape* s) {
   if (g.R < 8192) return false;
-  *s = fixed_shape(g);
+  *s = fixed_shape(g, solve);
   return (long long)s->grid.x * s->grid.y * s->grid.z <= FX_MAX_BLOCKS && s->grid.y <= 65535 && s->grid.z <= 65535;
 }

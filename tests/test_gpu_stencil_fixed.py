@@ -126,7 +126,7 @@ def _gpu_apply(lib, minv, v):
 
 
 # node counts z, y, x. The integers start at 8192 cells; warps of 30
-# columns and 2 rows, 4 from 600 thousand cells on; two layers, rows and columns
+# columns and 2 rows, products of larger grids 4; two layers, rows and columns
 SHAPES = [(17, 17, 33), (18, 17, 32), (33, 33, 33), (34, 35, 31), (41, 34, 32), (33, 36, 62), (3, 132, 128), (128, 3, 132),
           (132, 128, 3), (70, 95, 97), (151, 90, 47)]
 
