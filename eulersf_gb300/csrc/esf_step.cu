@@ -669,7 +669,12 @@ static esf_status compute_solid_mass(esf_scene* sc, Solid* d, int usesdf) {
   const double subDh = sc->p.mass_sample_dh;
   const int res = (int)(G.dh / subDh);
   ESF_COUNTED k_det_finv<<<kblocks(nc), KT, 0, st>>>(G, x, cells);
-  ESF_COUNTED k_mass_subsample<<<kblocks(nc, 128), 128, 0, st>>>(G, x, cells, usesdf, subDh, res);
+  const int per = res < MASS_T ? MASS_T / res : 1;  // cells a block
+  const size_t smem = (size_t)per * (3 * (size_t)res * sizeof(MassPlace) + 8 * (sizeof(int) + sizeof(double)));
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_mass_subsample, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  ESF_CUDA(attr);
+  ESF_COUNTED k_mass_subsample<<<kblocks(nc, per), MASS_T, smem, st>>>(G, x, cells, usesdf, subDh, res, per);
   ESF_COUNTED k_mass_gather<<<kblocks(boxn(nodes)), KT, 0, st>>>(G, x, cells, nodes);
   ESF_LAUNCH_CHECK();
   return ESF_OK;
@@ -1400,8 +1405,12 @@ extern "C" esf_status esf_step(esf_scene* sc, esf_step_report* rep) {
       nb.vel = o->d.vel;
       nb.sdf = o->sdf;
     }
-    if (d->np > 0)
-      ESF_COUNTED k_grid_to_particle<<<kblocks(d->np), KT, 0, st>>>(G, d->d, d->np, d->part.as<double>(), cp, cs);
+    if (d->np > 0) {
+      // (tmp3 is scratch until finalizeSolution)
+      ESF_COUNTED k_velocity_change<<<kblocks(3 * G.T), KT, 0, st>>>(G, d->d.vel, d->d.vws, d->d.tmp3);
+      ESF_COUNTED k_grid_to_particle<<<kblocks(d->np), KT, 0, st>>>(G, d->d, d->np, d->part.as<double>(), d->d.tmp3,
+                                                        cp, cs);
+    }
   }
   ESF_CUDA(cudaEventRecord(sc->ph[7], st));
   for (int i = 0; i < sc->ns; i++) {  // particleToGrid
