@@ -142,13 +142,27 @@ __global__ void __launch_bounds__(VT, std::is_same<T, float>::value ? 2 : 1) sol
   const int lane = tid & 31, warp = tid >> 5;
   // body(i, accumulator) for each element of the vectors, in the graph
   // kernels' virtual blocks, and their sums to `sums` (may be null)
+  // (four virtual blocks at a time, a warp for each one's sum: a block that had
+  // three of them one after another, 1000 cycles a sum, kept all others waiting)
   auto for_vec = [&](double* sums, auto zero, auto&& body) {
-    for (int v = blockIdx.x; v < a.vb; v += G) {
-      auto acc = zero;
-      for (long long i = v * (long long)VT + tid; i < n; i += (long long)a.vb * VT) body(i, acc);
-      if (sums) {
-        const double bs = block_sum<VT>((double)acc);
-        if (tid == 0) sums[v] = bs;
+    typedef BlockTree<VT> B;
+    __shared__ double values[4][B::WORDS];
+    for (int v0 = blockIdx.x; v0 < a.vb; v0 += 4 * G) {
+      if (sums) __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int v = v0 + k * G;
+        if (v >= a.vb) break;
+        auto acc = zero;
+        for (long long i = v * (long long)VT + tid; i < n; i += (long long)a.vb * VT) body(i, acc);
+        if (sums) B::put(values[k], (double)acc);
+      }
+      if (!sums) continue;
+      __syncthreads();
+      const int v = v0 + warp * G;
+      if (warp < 4 && v < a.vb) {
+        const double bs = B::sum(values[warp]);
+        if (lane == 0) sums[v] = bs;
       }
     }
   };

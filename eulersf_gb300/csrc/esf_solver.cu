@@ -45,16 +45,16 @@ namespace esf {
 // of the FP64 solve takes 19.0 for 21.6 us at 32^3, 33.7 for 36.4 at 64^3, 130
 // for 133 at 128^3, and the mixed solid solve of a step at 128^3 2.72 for 2.90 ms.
 template <int NT>
-__device__ __forceinline__ double block_sum(double v) {
-  constexpr int NW = NT / 32, STEP = 32 / NW, PITCH = 36;
+struct BlockTree {
+  static constexpr int NW = NT / 32, STEP = 32 / NW, PITCH = 36, WORDS = NW * PITCH;
   static_assert(NW == 4 || NW == 8, "a lane for each warp and step");
-  __shared__ double values[NW * PITCH];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __syncthreads();
-  values[w * PITCH + lane] = v;
-  __syncthreads();
-  double r = 0;
-  if (threadIdx.x < 32) {
+  // every thread's value to its place
+  static __device__ __forceinline__ void put(double* values, double v) {
+    values[(threadIdx.x >> 5) * PITCH + (threadIdx.x & 31)] = v;
+  }
+  // the sum of the places, by a warp
+  static __device__ __forceinline__ double sum(const double* values) {
+    const int lane = threadIdx.x & 31;
     const double* q = values + (lane % NW) * PITCH + lane / NW;
     double t[NW];
 #pragma unroll
@@ -63,11 +63,19 @@ __device__ __forceinline__ double block_sum(double v) {
     for (int h = NW / 2; h > 0; h /= 2)
 #pragma unroll
       for (int k = 0; k < h; k++) t[k] += t[k + h];
-    r = t[0];
+    double r = t[0];
     for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    if (__double_as_longlong(r) == (long long)0x8000000000000000ull) r = 0.0;  // (never -0)
+    return __double_as_longlong(r) == (long long)0x8000000000000000ull ? 0.0 : r;  // (never -0)
   }
-  return r;
+};
+template <int NT>
+__device__ __forceinline__ double block_sum(double v) {
+  typedef BlockTree<NT> B;
+  __shared__ double values[B::WORDS];
+  __syncthreads();
+  B::put(values, v);
+  __syncthreads();
+  return threadIdx.x < 32 ? B::sum(values) : 0.0;
 }
 
 // The largest of a block's words into *out, by thread 0 (whose fence in

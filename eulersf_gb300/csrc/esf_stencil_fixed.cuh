@@ -22,7 +22,8 @@
 // pipe: product 32^3 19.1 -> 8.2 us, 64^3 29.5 -> 18.9, 128^3 159 -> 64,
 // 161x127x190 343 -> 106, 256^3 1154 -> 390; solve iteration (phase A included)
 // 34.7 -> 19, 57.8 -> 34, 260 -> 121, 499 -> 201, 1749 -> 733 us. Error of a
-// product against extended precision: 3/4 of the FP64 kernel's (2-norm).
+// product against extended precision 4.7e-17 of the norm, the rounding of the
+// result; a plain FP64 evaluation has 1.7e-16.
 #pragma once
 
 constexpr int FX_T = 128;              // threads a block: four warps, stacked along y
