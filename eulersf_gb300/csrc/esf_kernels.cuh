@@ -668,7 +668,7 @@ __global__ void k_grid_to_particle(GridDev g, SolidDev s, long long np, double* 
 // P2G binning: key = stencil base node shifted by +3 per axis on an
 // (X+3)(Y+3)(Z+3) lattice; particles whose stencil misses the grid get the
 // key `nkeys` (sorted last, never gathered).
-// Keys, stencil weights and the particles' index box (reduced per warp and
+// Keys and the particles' index box (reduced per warp and
 // block, one atomic per block and bound; the box words start at
 // +/- 2^30 on the host).
 __global__ void __launch_bounds__(256) k_p2g_keys(GridDev g, long long np, const double* part, unsigned int* keys,

@@ -6,9 +6,11 @@
 //    CONJUGATE_RESIDUAL::solvePCR (CONJUGATE_RESIDUAL.inl:109-276) as two
 //    kernels per iteration (axpy+norm, update+SpMV+dot) plus a residual check
 //    every 5th iteration, with all scalars kept on the device and the
-//    iteration chunks replayed as CUDA graphs;
+//    iteration chunks replayed as CUDA graphs (FP64: the stencil on integers,
+//    esf_stencil_fixed.cuh);
 //  * FP32 inner solves inside FP64 iterative refinement (ESF_MIXED), one
-//    TMA-staged kernel per inner iteration (esf_pcr_fused.cuh);
+//    TMA-staged kernel per inner iteration (esf_pcr_fused.cuh), small grids'
+//    iterations in cooperative loops (esf_pcr_flat.cuh);
 //  * the solid system (M + dt^2 K) in 27-neighbour 3x3 block rows.
 #include <stdio.h>
 #include <stdlib.h>

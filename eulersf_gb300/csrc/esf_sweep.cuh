@@ -44,14 +44,13 @@ __device__ __forceinline__ double third(double x) {
   return __fma_rn(__fma_rn(-3.0, q, x), y, q);
 }
 
-// a < b of numbers (no NaN) by their bits, 40 cycles where an FP64 comparison and
-// a select on it take 104; zeros of either sign order by their sign, which no
-// caller can tell.
-__device__ __forceinline__ long long order_key(double a) {
-  const int hi = __double2hiint(a), m = hi >> 31;
-  return ((long long)(hi ^ (m & 0x7fffffff)) << 32) | (unsigned)(__double2loint(a) ^ m);
+// a < b by their bits, for numbers (no NaN) that are not both negative unless they
+// are the same: phi is -1/2 at nodes with mass and positive elsewhere, as the root
+// of sum over ds_i < t of (t - ds_i)^2 = 1 lies at least 1/sqrt(3) above the least
+// ds_i. 15 cycles, where an FP64 comparison and a select on it take 104.
+__device__ __forceinline__ bool less_bits(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
 }
-__device__ __forceinline__ bool less_bits(double a, double b) { return order_key(a) < order_key(b); }
 // x to 24 bits, towards zero, as a float, 0 below 2^-126, by its bits (a conversion is an FP64
 // operation); for numbers below 2^128.
 __device__ __forceinline__ float near_float(double x) {
@@ -71,7 +70,7 @@ __device__ __forceinline__ double root(double x) {
 // The same update, with the FP64 work that cannot change its outcome left
 // out. GB300 takes an FP64 instruction from a warp every 63 cycles, so their
 // number is most of a node's time (27 here at first with sqrt() and the quotient
-// by FMAs, 2740 cycles a node of a lone chain; 20 now, 2200), so:
+// by FMAs, 2740 cycles a node of a lone chain; 20 now, 2150), so:
 //  * a node whose value v already lies below the new distance keeps it. The
 //    new distance is the root of sum over ds_i < t of (t - ds_i)^2 = 1, whose
 //    left side grows with t: where it is below `skipBelow` (0.99) at t = v,
@@ -90,7 +89,7 @@ __device__ __forceinline__ double root(double x) {
 __device__ __forceinline__ bool solve_distance_fast(double p, double q, double r, double& v, float fp, float fq,
                                                     float fr, float fv, float skipBelow) {
   const float tp = fmaxf(fv - fp, 0.0f), tq = fmaxf(fv - fq, 0.0f), tr = fmaxf(fv - fr, 0.0f);
-  if (tp * tp + tq * tq + tr * tr < skipBelow) return false;
+  if (__fmaf_rn(tp, tp, __fmaf_rn(tq, tq, tr * tr)) < skipBelow) return false;
   const bool rq = less_bits(r, q);
   const double mqr = rq ? r : q, Mqr = rq ? q : r;  // (equal ones are the same)
   const double ds0 = less_bits(mqr, p) ? mqr : p, ds2 = less_bits(p, Mqr) ? Mqr : p;
@@ -98,8 +97,8 @@ __device__ __forceinline__ bool solve_distance_fast(double p, double q, double r
   const float lo = fminf(fminf(fp, fq), fr), hi = fmaxf(fmaxf(fp, fq), fr), mid = fp + fq + fr - lo - hi;
   const float e1 = mid - lo, e2 = hi - lo, e21 = hi - mid;
   int i = 2;
-  if (skipBelow > 0.0f && e2 * e2 + e21 * e21 > 1.01f)
-    i = (e1 * e1 > 1.01f && fabsf(e1 * e1 - 2.0f) > 0.02f) ? 0 : 1;
+  if (skipBelow > 0.0f && __fmaf_rn(e2, e2, e21 * e21) > 1.01f)
+    i = (e1 * e1 > 1.01f && fabsf(__fmaf_rn(e1, e1, -2.0f)) > 0.02f) ? 0 : 1;
   const double c0 = ds0 * ds0 - 1.0;
   const double b1 = ds1 + ds0, c1 = ds1 * ds1 + c0;
   const double b2 = ds2 + b1, c2 = ds2 * ds2 + c1;
@@ -481,9 +480,9 @@ __global__ void __launch_bounds__(EXTEND_THREADS) k_extend_field(GridDev g, doub
 // (MARCH_WAIT_LIMIT polls): a warp that gives up sets *err and stops waiting,
 // as does every warp that sees *err, so the launch ends; the host reports it.
 // Measured (mesh, SDF and particle phase of a step, GB300): 11.3 ms with the
-// wave and 6.5 with the march at 64^3, 16.1 and 9.5 at 128^3; 5.2 and 7.7 with
+// wave and 6.5 with the march at 64^3, 16.1 and 9.5 at 128^3; 5.1 and 7.6 with
 // comparisons on the numbers' bits and the root and the third of esf_root.cuh.
-// What is left is the chain of FP64 instructions, 2200 cycles a step where lanes
+// What is left is the chain of FP64 instructions, 2150 cycles a step where lanes
 // update. A version with progress counters (release and acquire every batch) took 8.3,
 // and one that loaded mailboxes step by step 8.0 ms a step's passes at 64^3.
 constexpr int MARCH_B = 8, MARCH_C = 4, MARCH_BATCH = 4;
