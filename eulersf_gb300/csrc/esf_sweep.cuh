@@ -469,7 +469,9 @@ __global__ void __launch_bounds__(EXTEND_THREADS) k_extend_field(GridDev g, doub
 // leave a patch at its downwind faces go through mailboxes in global memory
 // which the host fills with SWEEP_EMPTY before the pass: a value is its own
 // arrival flag, so neither side fences, and the reader loads a batch of
-// MARCH_BATCH steps ahead and polls again only where it came too early.
+// MARCH_BATCH steps ahead and polls again only where it came too early. (A patch
+// trails its neighbour by a batch and the value's way: batches of 4, 3, 2 and 1
+// gave 5.1, 4.65, 4.35 and 4.0 ms a phase at 64^3, 7.6, 6.9, 6.4 and 5.9 at 128^3.)
 // What bounds a pass is the chain of steps: a patch trails its b neighbour by
 // 8 steps and its c neighbour by 4, plus the ~1 us a value takes through L2,
 // and then has n of its own. The warps are spread over all SMs, one or a few
@@ -481,11 +483,11 @@ __global__ void __launch_bounds__(EXTEND_THREADS) k_extend_field(GridDev g, doub
 // as does every warp that sees *err, so the launch ends; the host reports it.
 // Measured (mesh, SDF and particle phase of a step, GB300): 11.3 ms with the
 // wave and 6.5 with the march at 64^3, 16.1 and 9.5 at 128^3; 5.1 and 7.6 with
-// comparisons on the numbers' bits and the root and the third of esf_root.cuh.
-// What is left is the chain of FP64 instructions, 2150 cycles a step where lanes
-// update. A version with progress counters (release and acquire every batch) took 8.3,
-// and one that loaded mailboxes step by step 8.0 ms a step's passes at 64^3.
-constexpr int MARCH_B = 8, MARCH_C = 4, MARCH_BATCH = 4;
+// comparisons on the numbers' bits and the root and the third of esf_root.cuh, 4.0
+// and 5.9 in batches of one step. What is left is the chain of FP64 instructions,
+// 2150 cycles a step where lanes update, and the mailboxes' way. A version with
+// progress counters (release and acquire every batch of 4) took 8.3 ms at 64^3.
+constexpr int MARCH_B = 8, MARCH_C = 4, MARCH_BATCH = 1;
 constexpr int MARCH_SKEW = (MARCH_B - 1) + (MARCH_C - 1);
 constexpr unsigned MARCH_WAIT_LIMIT = 1u << 22;
 constexpr unsigned long long SWEEP_EMPTY = ~0ull;  // a NaN no arithmetic gives
