@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(KT) k_sweep_vec_scan(SweepLists L) {
 // octant's (b, c) columns (one plane for even levels, one for odd). Entries
 // are loaded two levels ahead and a copy's value one, so the chain of a level
 // is three shared-memory reads, the blend and the barrier.
-// What bounds it is the FP64 pipe of one SM (five instructions an entry at
+// What bounds it is the FP64 pipe of one SM (three instructions an entry at
 // two lanes a cycle) and that chain, about 0.3 us a level: so entries are
 // packed: one thread to a column, idle lanes included, took 134 us a pass
 // against 118 us for lists read through L2 and 85 us here, at 64^3. Measured a
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(EXTEND_THREADS) k_extend_field(GridDev g, doub
 // What bounds a pass is the chain of steps: a patch trails its b neighbour by
 // 8 steps and its c neighbour by 4, plus the ~1 us a value takes through L2,
 // and then has n of its own. The warps are spread over all SMs, one or a few
-// each, so their FP64 instructions (16 cycles each a warp) do not queue. Warps
+// each, so their FP64 instructions (63 cycles each a warp) do not queue. Warps
 // claim patches from a ticket counter in an order in which each patch comes
 // after those it reads from, so a pass makes progress with any number of
 // warps resident and needs no cooperative launch. Waits are bounded
