@@ -114,8 +114,9 @@ struct PcrState {
   unsigned int ticket[4];
   double deltaPrev;  // one-pass double-float run: r.s of the iterate before the current one
   // fixed-point FP64 stencil: bounds as high words (fixed_mag) of x, 1/m, the
-  // stencil's input r - alpha Ap/diag, and what phase A collects for that
-  unsigned int hx, hm, hv, hr, hq;
+  // stencil's input r - alpha Ap/diag, and what phase A collects for that; and of
+  // the least 1/m (fixed_bounds)
+  unsigned int hx, hm, hv, hr, hq, lm;
   double limit;  // one-pass FP32 iteration: eps^2 delta0, below which it stops
 };
 

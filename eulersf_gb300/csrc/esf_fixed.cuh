@@ -14,10 +14,9 @@
 // mantissa and an exponent of their own. Sums of eight values (J^T v), their
 // products with 1/m and sums of 24 of those fit the limbs; sums are exact, and
 // the products drop what lies below 2^-77 of the largest. A double has 53 bits,
-// so the result is nearer to the exact one than FP64 arithmetic's wherever the
-// values around a cell are above 2^-22 of the largest value the scale was
-// chosen for, and everywhere its error is below 2^-70 of that (FP64's is about
-// 2^-52 of the values around the cell).
+// so a cell's result is nearer to the exact one than FP64 arithmetic's where its
+// largest product of a value and a factor lies less than 2^21 below the scales'
+// (FIX_SPARE); callers use FP64 for the others (fixed_loses).
 //
 // Where fixed_ok says no (a bound that is not finite, a negative 1/m, scales
 // near the top of the exponent range) callers use FP64, in which NaN and
@@ -89,6 +88,18 @@ ESF_HD bool fixed_low(unsigned hv, unsigned hm) {
 ESF_HD bool fixed_ok(unsigned hv, unsigned hm) {
   return hv < 0x7ff00000u && hm < 0x7ff00000u && fixed_scale(hv, hm) + fixed_exp(hm) < 900;
 }
+
+// Where a value or factor stands: |x| < 2^fixed_place(x), at least half of that
+// where x is normal; of zero, far below all others.
+constexpr int FIX_NOWHERE = -100000;
+ESF_HD int fixed_place(double x) { return fixed_mag1(x) ? fixed_exp(fixed_mag(x)) : FIX_NOWHERE; }
+// How far below the scales' product, in places, a cell's largest product of a
+// value and a factor may lie. A cell's error is some 11 units of 2^(Ev + Em - 77)
+// in the mean square. Against the sum of a cell's terms without their signs, by
+// how far it lies below (in brackets an FP64 evaluation's): at the scale 8.5e-18
+// (3.5e-17), 21 places 1.2e-17 (3.5e-17), 22 places 3.8e-17 (3.6e-17), 24 places
+// 1.6e-16, 45 places 6e-10.
+constexpr int FIX_SPARE = 21;
 
 // x 2^(77 - Ev) towards zero, for |x| < 2^Ev, Ev at least -880
 ESF_HD Fix fixed_from(double x, int Ev) {

@@ -1520,7 +1520,7 @@ static esf_status fixed_start(const GridDev& g, const double* minv, const double
                               bool* fixed, FixedShape* shape) {
   *fixed = false;
   if (!fixed_pays(g, true, shape)) return ESF_OK;
-  ESF_COUNTED fixed_bounds<<<vec_blocks(g.T), 256, 0, cs>>>(g, x, minv, &st->hx, &st->hm);
+  ESF_COUNTED fixed_bounds<<<vec_blocks(g.T), 256, 0, cs>>>(g, x, minv, &st->hx, &st->hm, &st->lm);
   ESF_LAUNCH_CHECK();
   unsigned h[2];
   ESF_CUDA(cudaMemcpyAsync(h, &st->hx, sizeof h, cudaMemcpyDeviceToHost, cs));

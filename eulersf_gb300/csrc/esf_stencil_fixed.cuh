@@ -20,8 +20,8 @@
 // cycle and scheduler, its three warps waiting on their own chains; DRAM at a
 // third). Measured against pressure_stencil<double>, whose bound is the FP64
 // pipe: product 32^3 19.1 -> 8.2 us, 64^3 29.5 -> 18.9, 128^3 159 -> 64,
-// 161x127x190 343 -> 106, 256^3 1154 -> 390; solve iteration (phase A included)
-// 34.7 -> 19, 57.8 -> 34, 260 -> 121, 499 -> 201, 1749 -> 733 us. Error of a
+// 161x127x190 343 -> 106, 256^3 1154 -> 400; solve iteration (phase A included)
+// 34.7 -> 19, 57.8 -> 35, 260 -> 121, 499 -> 207, 1749 -> 733 us. Error of a
 // product against extended precision 4.7e-17 of the norm, the rounding of the
 // result; a plain FP64 evaluation has 1.7e-16.
 #pragma once
@@ -55,41 +55,162 @@ __device__ __forceinline__ Fix shfl_up(Fix a) {
              __shfl_up_sync(0xffffffffu, a.l2, 1)};
 }
 
-// (J diag(1/m) J^T v) of one cell in FP64, in pressure_stencil's order, from
-// memory: the warps whose values do not fit a scale (NaN, infinities, negative
-// 1/m, the ends of the exponent range).
-__device__ double stencil_cell_direct(const GridDev& g, const double* v, const double* minv, int x, int y, int z) {
-  auto at = [&](int i, int j, int k) {
-    return i >= 0 && j >= 0 && k >= 0 && i < g.cX && j < g.cY && k < g.cZ
-               ? v[i + (long long)j * g.cX + (long long)k * g.cslab] : 0.0;
-  };
-  double m[2][2][2][3];
-  for (int dz = 0; dz < 2; dz++)
-    for (int dy = 0; dy < 2; dy++)
-      for (int dx = 0; dx < 2; dx++) {
-        const int i = x + dx, j = y + dy, k = z + dz;  // node; its cells are i-1..i, j-1..j, k-1..k
-        double p[2][2], q[2][2];
-        for (int b = 0; b < 2; b++)
-          for (int a = 0; a < 2; a++) {
-            const double lo = at(i - 1 + a, j - 1 + b, k - 1), hi = at(i - 1 + a, j - 1 + b, k);
-            p[b][a] = lo + hi;
-            q[b][a] = lo - hi;
-          }
-        const bool inside = i > 0 && j > 0 && k > 0 && i < g.X - 1 && j < g.Y - 1 && k < g.Z - 1;
-        const double mi = inside ? minv[i + (long long)j * g.X + (long long)k * g.slab] : 0.0;
-        m[dz][dy][dx][0] = ((p[0][0] + p[1][0]) - (p[0][1] + p[1][1])) * mi;
-        m[dz][dy][dx][1] = ((p[0][0] + p[0][1]) - (p[1][0] + p[1][1])) * mi;
-        m[dz][dy][dx][2] = ((q[0][0] + q[0][1]) + (q[1][0] + q[1][1])) * mi;
-      }
-  double A[2][2], B[2][2], C[2][2];
-  for (int dy = 0; dy < 2; dy++)
-    for (int dx = 0; dx < 2; dx++) {
-      A[dy][dx] = m[0][dy][dx][0] + m[1][dy][dx][0];
-      B[dy][dx] = m[0][dy][dx][1] + m[1][dy][dx][1];
-      C[dy][dx] = m[1][dy][dx][2] - m[0][dy][dx][2];
+__device__ __forceinline__ double shfl_down(double a) { return __shfl_down_sync(0xffffffffu, a, 1); }
+__device__ __forceinline__ double shfl_up(double a) { return __shfl_up_sync(0xffffffffu, a, 1); }
+
+// A warp's layer as fixed_finish reads it: the rows' values, the node rows' 1/m.
+template <int MODE, int RY>
+struct FixedLayer {
+  double v[RY + 2], m[RY + 1];
+  __device__ __forceinline__ void load(const GridDev& g, const StencilArgs<double>& a, double alpha, int cx, int y0,
+                                       int kk, int last) {
+    const bool layer = kk >= 0 && kk < g.cZ && kk <= last, col = cx >= 0 && cx < g.cX;
+#pragma unroll
+    for (int j = 0; j < RY + 2; j++) {
+      const int y = y0 - 1 + j;
+      const long long c = cx + (long long)y * g.cX + (long long)kk * g.cslab;
+      v[j] = 0.0;
+      if (layer && col && y >= 0 && y < g.cY)
+        v[j] = MODE == S_UPDATE ? upd_r(a.r[c], alpha, a.Ap[c], a.invd[c]) : a.in[c];
     }
-  return ((A[0][1] + A[1][1]) - (A[0][0] + A[1][0])) + ((B[1][0] + B[1][1]) - (B[0][0] + B[0][1])) +
-         ((C[0][0] + C[0][1]) + (C[1][0] + C[1][1]));
+#pragma unroll
+    for (int j = 0; j < RY + 1; j++) {
+      const int y = y0 + j;
+      const bool in = col && cx < g.cX - 1 && y > 0 && y < g.Y - 1 && kk > 0 && kk < g.Z - 1 && kk <= last;
+      m[j] = in ? a.minv[cx + 1 + (long long)y * g.X + (long long)kk * g.slab] : 0.0;
+    }
+  }
+};
+// Which of a warp's cells lose bits on integers that FP64 keeps: those whose
+// largest product of a value and a factor lies below 2^(top - FIX_SPARE).
+template <int RY>
+struct FixedReach {
+  int ev[RY + 2], en[RY + 1];  // of the layer before: values' places, products'
+  __device__ __forceinline__ FixedReach() {
+#pragma unroll
+    for (int j = 0; j < RY + 2; j++) ev[j] = FIX_NOWHERE;
+#pragma unroll
+    for (int j = 0; j < RY + 1; j++) en[j] = FIX_NOWHERE;
+  }
+  // the next layer; bit j: this lane's cell of row j, layer kk - 1
+  template <int MODE>
+  __device__ __forceinline__ unsigned next(const FixedLayer<MODE, RY>& l, int top) {
+    int pair = FIX_NOWHERE, pn = FIX_NOWHERE;  // of the row before
+    unsigned loses = 0;
+#pragma unroll
+    for (int j = 0; j < RY + 2; j++) {
+      const int e = fixed_place(l.v[j]), two = max(ev[j], e);
+      ev[j] = e;
+      int at = max(pair, two);
+      pair = two;
+      if (j == 0) continue;
+      at = max(at, __shfl_down_sync(0xffffffffu, at, 1)) + fixed_place(l.m[j - 1]);
+      const int nodes = max(en[j - 1], at);
+      en[j - 1] = at;
+      int best = max(pn, nodes);
+      pn = nodes;
+      if (j == 1) continue;
+      best = max(best, __shfl_up_sync(0xffffffffu, best, 1));
+      if (best > FIX_NOWHERE / 2 && best < top - FIX_SPARE) loses |= 1u << (j - 2);
+    }
+    return loses;
+  }
+};
+// The warp's cells again in FP64: those that lose bits on integers (FixedReach),
+// or `all`, for values that fit no scale (NaN, infinities, negative 1/m, the ends
+// of the exponent range). The others' results stay, as do their shares of acc, but
+// for CHECK, whose whole sum it forms. Apart from the kernel, whose registers it
+// would cost; the march on integers only watches whether any warp needs it, which
+// is 3 % of a product or an iteration (256^3 400 -> 411 us, 161x127x190 202 -> 207,
+// 64^3 34.2 -> 35.1). A product of 256^3 cells takes 412 us, 1107 with values of
+// 1e-12 around a one in every 16^3 cells, 563 with values that fall by e^40 along
+// z, 686 with a NaN in every 16^3 cells (pressure_stencil<double> 1160 each); an
+// iteration at 161x127x190 from a right-hand side of one cell 485 (499).
+template <int MODE, int RY>
+__device__ __noinline__ double fixed_finish(const GridDev& g, const StencilArgs<double>& a, double alpha, int top,
+                                            bool all, int y0, int z0, int z1, double acc, unsigned* hx) {
+  const int lane = threadIdx.x & 31, cx = blockIdx.x * FX_COLS + lane - 1;
+  const bool own = cx >= 0 && cx < g.cX && lane >= 1 && lane <= FX_COLS;
+  unsigned mine = 0;  // own rows
+#pragma unroll
+  for (int j = 0; j < RY; j++) mine |= own && y0 + j < g.cY ? 1u << j : 0u;
+  FixedLayer<MODE, RY> l, n;
+  if (MODE == S_APPLY && !all) {  // the layers that have any (a solve's reads cost more than the march saves)
+    FixedReach<RY> reach;
+    int first = INT_MAX, last = -1;
+    n.load(g, a, alpha, cx, y0, z0 - 1, z1);
+    for (int kk = z0 - 1; kk <= z1; kk++) {
+      l = n;
+      n.load(g, a, alpha, cx, y0, kk + 1, z1);
+      if (reach.next(l, top) & mine && kk > z0) {
+        first = min(first, kk - 1);
+        last = kk - 1;
+      }
+    }
+    z0 = __reduce_min_sync(0xffffffffu, first);
+    z1 = __reduce_max_sync(0xffffffffu, last) + 1;
+    if (z0 >= z1) return acc;
+  }
+  if (MODE == S_CHECK) acc = 0.0;
+  FixedReach<RY> reach;
+  double own_value[RY] = {};  // of the layer before
+  double prev[RY + 2] = {}, mpx[RY + 1] = {}, mpy[RY + 1] = {}, mpz[RY + 1] = {};
+  n.load(g, a, alpha, cx, y0, z0 - 1, z1);
+  for (int kk = z0 - 1; kk <= z1; kk++) {
+    l = n;
+    n.load(g, a, alpha, cx, y0, kk + 1, z1);
+    const unsigned loses = (all ? ~0u : reach.next(l, top)) & mine;
+    double dp, xp, xq, vp = 0.0;  // as in the march on integers
+#pragma unroll
+    for (int j = 0; j < RY + 2; j++) {
+      const double old = prev[j], P = old + l.v[j], Q = old - l.v[j];
+      prev[j] = l.v[j];
+      if (kk < z0) continue;
+      const double pn = shfl_down(P), qn = shfl_down(Q);
+      const double dp1 = P - pn, xp1 = P + pn, xq1 = Q + qn;
+      if (j > 0) {
+        const double m = l.m[j - 1];
+        const double mx = (dp + dp1) * m, my = (xp - xp1) * m, mz = (xq + xq1) * m;
+        if (kk > z0) {
+          const double A = mpx[j - 1] + mx, B = mpy[j - 1] + my, C = mz - mpz[j - 1];
+          const double CA = C - A, AC = A + C;
+          const double up = shfl_up(CA + B), um = shfl_up(CA - B);
+          if (j > 1) {
+            const double o = (vp + up) + (AC + B);
+            const long long c = cx + (long long)(y0 + j - 2) * g.cX + (long long)(kk - 1) * g.cslab;
+            const bool it = loses >> (j - 2) & 1u;
+            if (MODE == S_APPLY) {
+              if (it) a.out[c] = o;
+            } else if (MODE == S_UPDATE) {
+              if (it) {
+                acc += own_value[j - 2] * (o - a.out[c]);
+                a.out[c] = o;
+              }
+            } else if (MODE == S_CHECK) {
+              const double e = mine >> (j - 2) & 1u ? o - a.b[c] : 0.0;
+              acc += e * e;
+            } else if (MODE == S_RESID_INIT) {
+              if (it) {
+                const double rn = (a.b[c] - o) * a.invd[c];
+                a.r[c] = rn;
+                *hx = max(*hx, fixed_mag(rn));
+              }
+            }
+          }
+          vp = (AC - B) + um;
+        }
+        mpx[j - 1] = mx;
+        mpy[j - 1] = my;
+        mpz[j - 1] = mz;
+      }
+      dp = dp1;
+      xp = xp1;
+      xq = xq1;
+    }
+#pragma unroll
+    for (int j = 0; j < RY; j++) own_value[j] = l.v[j + 1];
+  }
+  return acc;
 }
 
 // The bound of v = r - alpha Ap/diag from the largest |r| and |Ap/diag|, as a
@@ -102,7 +223,9 @@ __device__ __forceinline__ unsigned fixed_bound(unsigned hr, unsigned hq, double
 template <int MODE>
 constexpr int FX_RESIDENT = MODE == S_APPLY ? 3 : 4;
 template <int MODE, int RY>
-__global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixed(GridDev g, StencilArgs<double> a, int cz) {
+__global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixed(const __grid_constant__ GridDev g,
+                                                                                      const __grid_constant__ StencilArgs<double> a,
+                                                                                      int cz) {
   extern __shared__ double ring[];  // [2][slots][FX_T]
   if (MODE != S_APPLY && a.st->done) return;
   constexpr int SLOTS = fx_slots<MODE, RY>();
@@ -116,12 +239,18 @@ __global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixe
   const double alpha = MODE == S_UPDATE ? a.st->alpha : 0.0;
   double acc = 0.0;
   unsigned hx = 0;  // UPDATE: largest new x; RESID_INIT: largest r
+  // how far down the values reach: the least over the cells of the largest in the
+  // three rows around it (high words less one; all zero: none). A cell that loses
+  // bits has small ones only around it, in its own column or one beside it.
+  unsigned least = ~0u;
+  const int rows = min(RY, g.cY - y0);
   auto cell = [&](int y, int z) { return cx + (long long)y * g.cX + (long long)z * g.cslab; };
   auto node = [&](int y, int z) { return cx + 1 + (long long)y * g.X + (long long)z * g.slab; };
   if (y0 < g.cY) {
-    unsigned hv, hm;
+    unsigned hv, hm, lm;  // bounds of v and 1/m; the least 1/m's high word less one
     if (MODE == S_APPLY) {  // this warp's own values
       hv = hm = 0;
+      lm = ~0u;
       // (four layers' loads in flight: one layer at a time the scan took as long
       // as the march)
       for (int z = z0 - 1; z <= z1; z += 4) {
@@ -138,22 +267,28 @@ __global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixe
         for (int k = 0; k < 4; k++)
 #pragma unroll
           for (int j = 0; j < RY + 2; j++) {
-            hv = max(hv, fixed_mag1(v[k][j]));
-            if (j > 0) hm = max(hm, hi_word(m[k][j - 1]) | (lo_word(m[k][j - 1]) ? 1u : 0u));
+            const unsigned h = fixed_mag1(v[k][j]);
+            hv = max(hv, h);
+            if (j > 0) {
+              if (j > 1 && j - 2 < rows) least = min(least, max(max(h, fixed_mag1(v[k][j - 1])), fixed_mag1(v[k][j - 2])) - 1u);
+              const unsigned w = hi_word(m[k][j - 1]) | (lo_word(m[k][j - 1]) ? 1u : 0u);
+              hm = max(hm, w);
+              lm = min(lm, w - 1u);
+            }
           }
       }
       hv = __reduce_max_sync(0xffffffffu, hv);
       hm = __reduce_max_sync(0xffffffffu, hm);
+      lm = __reduce_min_sync(0xffffffffu, lm);
     } else {
       hm = a.st->hm;
+      lm = ~a.st->lm;
       hv = MODE == S_UPDATE ? a.st->hv : a.st->hx;
     }
     const int Em = fixed_exp(hm), Ev = fixed_scale(hv, hm);
     const bool ok = fixed_ok(hv, hm);
     if (MODE == S_APPLY && (!ok || fixed_low(hv, hm))) {
-      for (int z = z0; z < z1; z++)
-        for (int j = 0; j < RY; j++)
-          if (own && y0 + j < g.cY) a.out[cell(y0 + j, z)] = stencil_cell_direct(g, a.in, a.minv, cx, y0 + j, z);
+      fixed_finish<MODE, RY>(g, a, alpha, 0, true, y0, z0, z1, 0.0, nullptr);
       return;
     }
     // (in a solve, a scale that does not fit is a value on its way to infinity,
@@ -216,6 +351,10 @@ __global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixe
         v[j] = MODE == S_UPDATE
                    ? upd_r(q[FX_T * (3 * j)], alpha, q[FX_T * (3 * j + 1)], q[FX_T * (3 * j + 2)])
                    : q[FX_T * j];
+      if (MODE != S_APPLY)
+#pragma unroll
+        for (int j = 2; j < RY + 2; j++)
+          if (j - 2 < rows) least = min(least, max(max(fixed_mag(v[j - 2]), fixed_mag(v[j - 1])), fixed_mag(v[j])) - 1u);
       if (MODE == S_UPDATE && kk >= z0 && kk < z1) {
 #pragma unroll
         for (int j = 0; j < RY; j++)
@@ -275,6 +414,12 @@ __global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixe
 #pragma unroll
         for (int j = 0; j < RY; j++) vo[j] = v[j + 1];
     }
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (ok && least != ~0u && Ev - fixed_exp(least + 1u) + (Em - fixed_exp(lm + 1u)) > FIX_SPARE) {
+      unsigned h = hx;
+      acc = fixed_finish<MODE, RY>(g, a, alpha, Ev + Em, false, y0, z0, z1, acc, &h);
+      hx = h;
+    }
   }
   if (MODE == S_APPLY) return;
   if (MODE == S_UPDATE || MODE == S_RESID_INIT) block_max(hx, MODE == S_UPDATE ? &a.st->hx : &a.st->hr);
@@ -297,22 +442,29 @@ __global__ void __launch_bounds__(FX_T, FX_RESIDENT<MODE>) pressure_stencil_fixe
 }
 
 // Bounds a fixed-point solve starts from: the largest |x|, and the largest 1/m
-// of the interior nodes (a negative one's sign bit makes it the largest). The
-// words are zero before.
+// of the interior nodes (a negative one's sign bit makes it the largest); and the
+// complement of their least 1/m's word less one (0: all are zero). The words are
+// zero before.
 __global__ void __launch_bounds__(256) fixed_bounds(GridDev g, const double* x, const double* minv, unsigned* hx,
-                                                    unsigned* hm) {
-  unsigned mx = 0, mm = 0;
+                                                    unsigned* hm, unsigned* lm) {
+  unsigned mx = 0, mm = 0, ml = 0;
   const long long stride = (long long)gridDim.x * 256;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < g.R; i += stride) mx = max(mx, fixed_mag(x[i]));
   for (long long n = blockIdx.x * 256LL + threadIdx.x; n < g.T; n += stride) {
     const int i = (int)(n % g.X), j = (int)((n / g.X) % g.Y), k = (int)(n / g.slab);
-    if (i > 0 && j > 0 && k > 0 && i < g.X - 1 && j < g.Y - 1 && k < g.Z - 1) mm = max(mm, hi_word(minv[n]));
+    if (i > 0 && j > 0 && k > 0 && i < g.X - 1 && j < g.Y - 1 && k < g.Z - 1) {
+      const unsigned w = hi_word(minv[n]) | (lo_word(minv[n]) ? 1u : 0u);
+      mm = max(mm, w);
+      ml = max(ml, ~(w - 1u));
+    }
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
   mm = __reduce_max_sync(0xffffffffu, mm);
+  ml = __reduce_max_sync(0xffffffffu, ml);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(hx, mx);
     atomicMax(hm, mm);
+    atomicMax(lm, ml);
   }
 }
 
