@@ -681,17 +681,18 @@ static esf_status compute_solid_mass(esf_scene* sc, Solid* d, int usesdf) {
 }
 
 // The Gauss-Seidel sweeps: sweepPhi as a systolic march of warps
-// (k_sweep_march), the velocity extension over level lists (k_extend_field);
-// ESF_SWEEP=wave runs both as cooperative hyperplane waves (k_sweep_wave)
-// instead, for comparison. Either gives the bits of the sequential loops. A
+// (k_sweep_march), the velocity extension over level lists (k_extend_field) or,
+// for large octants, tiles (k_sweep_vec_tile); for comparison, ESF_SWEEP=tiles
+// takes tiles for any octant, ESF_SWEEP=wave runs both kinds of sweep as cooperative
+// hyperplane waves (k_sweep_wave). All give the bits of the sequential loops. A
 // wait that ran out raises the scene's sweep error word (dInts[42]), checked
 // when the step or init ends.
 constexpr int kSweepBar = 40, kSweepErr = 42;
 constexpr int kFallbackCount = 44;  // mixed: cells of the FP32 stiffness evaluated again in FP64 (one per solid)
 constexpr int kOverlap = 52;        // broad phase: two solids' meshes overlap
-static bool sweep_wave_asked() {
+static bool sweep_asked(const char* schedule) {
   const char* pick = getenv("ESF_SWEEP");
-  return pick && strcmp(pick, "wave") == 0;
+  return pick && strcmp(pick, schedule) == 0;
 }
 // direction `dir` of the reference's eight loops over the box, which leave
 // out `margin` nodes of each axis
@@ -745,7 +746,7 @@ static esf_status sweep_wave(esf_scene* sc, Solid* d, const Sweep& w, const unsi
 static esf_status sweep_phi(esf_scene* sc, Solid* d, const Box& ex) {
   const Sweep shape = sweep_of(ex, 0, 1);
   if (shape.ni <= 0 || shape.nj <= 0 || shape.nk <= 0) return ESF_OK;
-  if (sweep_wave_asked()) {
+  if (sweep_asked("wave")) {
     for (int pass = 0; pass < 16; pass++) TRY(sweep_wave<false>(sc, d, sweep_of(ex, pass % 8, 1), nullptr));
     return ESF_OK;
   }
@@ -811,18 +812,26 @@ static esf_status extend_velocity(esf_scene* sc, Solid* d) {
   ESF_LAUNCH_CHECK();
   ESF_CUDA(cudaMemcpyAsync(h, dims, 56 * sizeof(int), cudaMemcpyDeviceToHost, st));
   ESF_CUDA(cudaStreamSynchronize(st));
-  // columns of the largest octant's plane, and all entries
-  long long cols = 1, entries = 0;
+  // columns of the largest octant's plane, all entries, and what a round of passes
+  // takes (us) by lists and by tiles: 0.2 a level and 2.2 a thousand entries (three
+  // blocks), 15.4 a launch of tiles. Measured a step, lists and tiles: a ball of 36
+  // nodes across 5.9 and 9.6 ms, 77 15.5 and 15.6, 92 21.1 and 18.1, 102 25.9 and
+  // 19.9; of 154 x 154 x 30 nodes 26.9 and 27.9, of 51 x 51 x 179 17.4 and 20.2.
+  // (The model is off by up to a sixth, hence lists up to 1.2 times.)
+  long long cols = 1, entries = 0, tileLaunches = 0, octantLevels = 0;
   for (int dir = 0; dir < 8; dir++) {
     const int* q = h + 6 * dir;
     if (q[1] < 0) continue;
     cols = std::max(cols, (long long)(q[3] - q[2] + 2) * (q[5] - q[4] + 2));
     entries += h[48 + dir];
+    tileLaunches += sweep_tile_launches(q);
+    octantLevels += (q[1] - q[0]) + (q[3] - q[2]) + (q[5] - q[4]) + 2;
   }
-  // two planes and the levels in shared memory: octants up to 115 x 115
-  // columns (a solid that spans more than 200 nodes); beyond that the wave
+  // lists need two planes and the levels in shared memory
   const long long smem = 16 * cols + 32LL * (L.levels + 1);
-  if (!sweep_wave_asked() && smem <= 220 * 1024) {
+  const bool wave = sweep_asked("wave");
+  const bool lists = smem <= 220 * 1024 && 0.2 * octantLevels + 2.2e-3 * entries <= 1.2 * 15.4 * tileLaunches;
+  if (lists && !wave && !sweep_asked("tiles")) {
     TRY(sc->sweepList.ensure((size_t)entries * sizeof(SweepEntry)));
     L.entry = sc->sweepList.as<SweepEntry>();
     static const cudaError_t attr =
@@ -835,7 +844,28 @@ static esf_status extend_velocity(esf_scene* sc, Solid* d) {
     return ESF_OK;
   }
   for (int round = 0; round < 4; round++) {
-    for (int dir = 0; dir < 8; dir++) TRY(sweep_wave<true>(sc, d, all.d[dir], ranks + 3 * dir));
+    for (int dir = 0; dir < 8; dir++) {
+      Sweep w = all.d[dir];
+      if (wave) {
+        TRY(sweep_wave<true>(sc, d, w, ranks + 3 * dir));
+        continue;
+      }
+      const int* q = h + 6 * dir;
+      if (q[1] < 0) continue;
+      const int ni = w.ni;
+      const long long nij = (long long)w.ni * w.nj;
+      const double2* weights = wt + dir * total;
+      const long long first = q[0] + (long long)q[2] * ni + q[4] * nij;
+      w.i0 += q[0] * w.di;
+      w.j0 += q[2] * w.dj;
+      w.k0 += q[4] * w.dk;
+      w.ni = q[1] - q[0] + 1;
+      w.nj = q[3] - q[2] + 1;
+      w.nk = q[5] - q[4] + 1;
+      const int blocks = (w.ni + ST - 1) / ST * ((w.nj + ST - 1) / ST);
+      for (int P = 0; P < sweep_tile_launches(q); P++)
+        ESF_COUNTED k_sweep_vec_tile<<<blocks, TILE_THREADS, 0, st>>>(G, d->d.vel, w, weights, first, ni, nij, P);
+    }
     for (int axis = 2; axis >= 0; axis--)
       ESF_COUNTED k_extend_faces<<<kblocks(boxn(ex) / (ex.hi[axis] - ex.lo[axis])), KT, 0, st>>>(
           G, d->d.vel, d->d.mass, ex, axis);

@@ -460,6 +460,67 @@ __global__ void __launch_bounds__(EXTEND_THREADS) k_extend_field(GridDev g, doub
   }
 }
 
+// The passes of larger octants as a wavefront of tiles: the octant's nodes (w is
+// its sweep: its first node and its sides) are cut into tiles of ST^3, and launch
+// P runs every tile (I, J, K) with I + J + K = P, whose three upwind tiles ran in
+// launch P - 1: some 15 us, 22 planes of a chain of shared-memory reads each. At
+// 256^3 a step of it took 22 ms for a ball of 113 nodes across, 31 for 154, 49 for
+// 215 (the wave 57, 80 and 117, tiles over the whole box 31, 44 and 70). A block copies its tile and the upwind layer of each axis into
+// shared memory and walks the tile's planes a' + b' + c' = q there, a barrier a
+// plane. Weights in loop order: the octant's node (0, 0, 0) at wt[first], rows of
+// ni, planes of nij.
+constexpr int ST = 8, SP = ST + 1;  // tile edge; with the upwind layer
+constexpr int TILE_THREADS = ST * ST * ST;
+// launches of a pass over the octant of these bounds (k_sweep_vec_weights)
+inline int sweep_tile_launches(const int* q) {
+  return (q[1] - q[0]) / ST + (q[3] - q[2]) / ST + (q[5] - q[4]) / ST + 1;
+}
+__global__ void __launch_bounds__(TILE_THREADS) k_sweep_vec_tile(GridDev g, double* f, Sweep w, const double2* wt,
+                                                                 long long first, int ni, long long nij, int P) {
+  __shared__ double sv[3 * SP * SP * SP];
+  __shared__ double2 sw[TILE_THREADS];
+  const int nti = (w.ni + ST - 1) / ST, ntj = (w.nj + ST - 1) / ST, ntk = (w.nk + ST - 1) / ST;
+  const int I = blockIdx.x % nti, J = blockIdx.x / nti, K = P - I - J;
+  if (J >= ntj || K < 0 || K >= ntk) return;
+  const int a0 = I * ST, b0 = J * ST, c0 = K * ST;
+  const int na = min(ST, w.ni - a0), nb = min(ST, w.nj - b0), nc = min(ST, w.nk - c0);
+  // local -1 .. n-1 on each axis (local -1 of the first tile is the node before
+  // the octant's first, inside the box)
+  for (int t = threadIdx.x; t < SP * SP * SP; t += TILE_THREADS) {
+    const int la = t % SP - 1, lb = (t / SP) % SP - 1, lc = t / (SP * SP) - 1;
+    if (la >= na || lb >= nb || lc >= nc) continue;
+    const long long n = nidx(g, w.i0 + (a0 + la) * w.di, w.j0 + (b0 + lb) * w.dj, w.k0 + (c0 + lc) * w.dk);
+#pragma unroll
+    for (int q = 0; q < 3; q++) sv[3 * t + q] = f[3 * n + q];
+  }
+  const int ta = threadIdx.x % ST, tb = (threadIdx.x / ST) % ST, tc = threadIdx.x / (ST * ST);
+  const bool in = ta < na && tb < nb && tc < nc;
+  sw[threadIdx.x] = in ? wt[first + (a0 + ta) + (long long)(b0 + tb) * ni + (c0 + tc) * nij]
+                       : make_double2(__longlong_as_double((long long)SWEEP_KEEP), 0.0);
+  auto keeps = [&](int u) { return (unsigned long long)__double_as_longlong(sw[u].x) == SWEEP_KEEP; };
+  __syncthreads();
+  for (int q = 0; q <= (na - 1) + (nb - 1) + (nc - 1); q++) {
+    const int lc = q - ta - tb;  // (the first ST^2 threads)
+    if (threadIdx.x < ST * ST && lc >= 0 && lc < ST) {
+      const int u = ta + tb * ST + lc * ST * ST;
+      if (!keeps(u)) {
+        const int s = (ta + 1) + (tb + 1) * SP + (lc + 1) * SP * SP;
+        const int sa = s - 1, sb = s - SP, sc = s - SP * SP;  // upwind in a, b, c
+        const double alpha = sw[u].x, beta = sw[u].y;
+#pragma unroll
+        for (int e = 0; e < 3; e++)
+          sv[3 * s + e] = (alpha * sv[3 * sa + e] + beta * sv[3 * sb + e]) + (1 - alpha - beta) * sv[3 * sc + e];
+      }
+    }
+    __syncthreads();
+  }
+  if (!in || keeps(threadIdx.x)) return;
+  const int s = (ta + 1) + (tb + 1) * SP + (tc + 1) * SP * SP;
+  const long long n = nidx(g, w.i0 + (a0 + ta) * w.di, w.j0 + (b0 + tb) * w.dj, w.k0 + (c0 + tc) * w.dk);
+#pragma unroll
+  for (int e = 0; e < 3; e++) f[3 * n + e] = sv[3 * s + e];
+}
+
 // ------------------------------------------------------------- the march
 // A pass as a systolic march of warps. The pass's (b, c) columns (y and z in
 // sweep order) are cut into patches of 8 x 4; one warp owns a patch and
