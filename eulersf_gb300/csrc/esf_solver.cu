@@ -1159,24 +1159,35 @@ enum Fp32Path {
 // both hold it is the faster one (7.7 against 12.4 us an iteration at 64^3).
 // ESF_PRESSURE_KERNEL=pass takes a launch an iteration everywhere (for
 // comparison; same bits).
+// The kernels' opt-in to FL_SMEM. It belongs to a device's context, which another
+// may follow in the process: asked for before the launches of each solve, not once.
+static esf_status allow_loops() {
+  ESF_CUDA(cudaFuncSetAttribute(pcr_loop_flat<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FL_SMEM));
+  ESF_CUDA(cudaFuncSetAttribute(pcr_loop_flat<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FL_SMEM));
+  return ESF_OK;
+}
+// blocks of the loops that the current device holds at once
+static long long loop_slots() {
+  static std::atomic<long long> known[64];  // one more than the number; 0: not looked up
+  int dev = 0, sms = 0, coop = 0, a = 0, b = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev < 64 && known[dev].load()) return known[dev].load() - 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  auto fits = [](auto* kernel, int* per) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, kernel, FL_G * NT, FL_SMEM) == cudaSuccess;
+  };
+  const bool ok = coop && allow_loops() == ESF_OK && fits(pcr_loop_flat<false>, &a) && fits(pcr_loop_flat<true>, &b);
+  const long long slots = ok ? (long long)sms * (a < b ? a : b) : 0;
+  if (dev < 64) known[dev].store(slots + 1);
+  return slots;
+}
 static bool loop_fits(const GridDev& g) {
-  static const long long slots = [] {
-    int dev = 0, sms = 0, coop = 0, a = 0, b = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    auto fits = [](auto* kernel, int* per) {
-      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FL_SMEM) == cudaSuccess &&
-             cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, kernel, FL_G * NT, FL_SMEM) == cudaSuccess;
-    };
-    if (!coop || !fits(pcr_loop_flat<false>, &a) || !fits(pcr_loop_flat<true>, &b)) return 0LL;
-    return (long long)sms * (a < b ? a : b);
-  }();
   const char* pick = getenv("ESF_PRESSURE_KERNEL");
   if (pick && strcmp(pick, "pass") == 0) return false;
   const int cz = fused_cz(g);
   const dim3 gr = tma_grid(g, cz);
-  return cz <= FL_L && (long long)gr.x * gr.y * gr.z <= slots;
+  return cz <= FL_L && (long long)gr.x * gr.y * gr.z <= loop_slots();
 }
 
 // Whether the TMA kernels take a grid's rows (and are not asked away).
@@ -1498,6 +1509,8 @@ static esf_status run_graph_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst,
 static esf_status run_fused(PressureWork* w, const FusedKernels& k, cudaGraphExec_t graph, unsigned long long kernels,
                             int maxIt, cudaStream_t st, PcrState* out) {
   if (!k.loops()) return run_graph_solve(w->hst, w->ev, k.st, nullptr, graph, 0, kernels, maxIt, st, out);
+  esf_status e = allow_loops();
+  if (e) return e;
   return run_solve(w->hst, w->ev, k.st, maxIt, st, out, [&](bool) { return k.loop(st, FL_CHUNK); }, FL_CHUNK);
 }
 

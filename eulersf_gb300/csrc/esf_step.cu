@@ -671,9 +671,8 @@ static esf_status compute_solid_mass(esf_scene* sc, Solid* d, int usesdf) {
   ESF_COUNTED k_det_finv<<<kblocks(nc), KT, 0, st>>>(G, x, cells);
   const int per = res < MASS_T ? MASS_T / res : 1;  // cells a block
   const size_t smem = (size_t)per * (3 * (size_t)res * sizeof(MassPlace) + 8 * (sizeof(int) + sizeof(double)));
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_mass_subsample, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-  ESF_CUDA(attr);
+  // (of the context, so before each launch, not once a process)
+  ESF_CUDA(cudaFuncSetAttribute(k_mass_subsample, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
   ESF_COUNTED k_mass_subsample<<<kblocks(nc, per), MASS_T, smem, st>>>(G, x, cells, usesdf, subDh, res, per);
   ESF_COUNTED k_mass_gather<<<kblocks(boxn(nodes)), KT, 0, st>>>(G, x, cells, nodes);
   ESF_LAUNCH_CHECK();
@@ -834,9 +833,7 @@ static esf_status extend_velocity(esf_scene* sc, Solid* d) {
   if (lists && !wave && !sweep_asked("tiles")) {
     TRY(sc->sweepList.ensure((size_t)entries * sizeof(SweepEntry)));
     L.entry = sc->sweepList.as<SweepEntry>();
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_extend_field, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    ESF_CUDA(attr);
+    ESF_CUDA(cudaFuncSetAttribute(k_extend_field, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     ESF_COUNTED k_sweep_vec_list<false><<<grid, KT, 0, st>>>(G, all, wt, dims, L);
     ESF_COUNTED k_extend_field<<<3, EXTEND_THREADS, (size_t)smem, st>>>(G, d->d.vel, d->d.mass, ex, all, dims, L,
                                                                         (int)cols);
