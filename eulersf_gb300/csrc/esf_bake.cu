@@ -407,9 +407,9 @@ extern "C" esf_status esf_rasterize_solid(const double* vertices, int num_vertic
   unsigned long long* dCount = nullptr;
   unsigned char* scratch = nullptr;
   esf_status e = ESF_OK;
-  if (cudaMalloc(&dTri, tri.size() * 4) != cudaSuccess || cudaMalloc(&dMass, total * 8) != cudaSuccess ||
-      cudaMalloc(&dCount, 8) != cudaSuccess ||
-      (cubes && cudaMalloc(&scratch, size.bytes + total) != cudaSuccess)) {
+  if (device_alloc(&dTri, tri.size() * 4) != cudaSuccess || device_alloc(&dMass, total * 8) != cudaSuccess ||
+      device_alloc(&dCount, 8) != cudaSuccess ||
+      (cubes && device_alloc(&scratch, size.bytes + total) != cudaSuccess)) {
     set_error("esf_rasterize_solid: device allocation failed");
     e = ESF_ERR_OOM;
   }

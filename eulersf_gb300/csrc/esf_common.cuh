@@ -178,6 +178,13 @@ esf_status pressure_work_take(PressureWork** w, const GridDev& g, int mixed);
 void pressure_work_give(PressureWork* w, bool idle);
 // frees those waiting for a next call on the device (-1: on all); whether any were
 bool pressure_work_release_idle(int device);
+// cudaMalloc, a second time after freeing those where the device's memory is out:
+// all device memory of the library comes from here (or is mapped, vec_alloc)
+cudaError_t device_alloc_bytes(void** p, size_t bytes);
+template <typename T>
+inline cudaError_t device_alloc(T** p, size_t bytes) {
+  return device_alloc_bytes(reinterpret_cast<void**>(p), bytes);
+}
 // a non-blocking stream of the work's own
 cudaStream_t pressure_work_stream(PressureWork* w);
 // Full pressure solve; x is the warm start / result. minv64 per node.

@@ -796,7 +796,7 @@ static esf_status vec_alloc(MappedSet* w, float** out, size_t bytes) {
   const unsigned char comp =
       (mode && strcmp(mode, "none") == 0) ? CU_MEM_ALLOCATION_COMP_NONE : CU_MEM_ALLOCATION_COMP_GENERIC;
   if (!malloc_only && vec_map(w, out, bytes, comp)) return ESF_OK;
-  ESF_CUDA(cudaMalloc(out, bytes));
+  ESF_CUDA(device_alloc(out, bytes));
   return ESF_OK;
 }
 static void vec_free(MappedSet* w, float* p) {
@@ -899,11 +899,11 @@ template esf_status pressure_apply<float>(const GridDev&, const float*, const fl
 
 static esf_status work_buffers(PressureWork* w, const GridDev& g, int mixed) {
   const size_t R = g.R;
-  ESF_CUDA(cudaMalloc(&w->r, R * 8));
-  ESF_CUDA(cudaMalloc(&w->d, R * 8));
-  ESF_CUDA(cudaMalloc(&w->Ap, R * 8));
-  ESF_CUDA(cudaMalloc(&w->s, R * 8));
-  ESF_CUDA(cudaMalloc(&w->invd, R * 8));
+  ESF_CUDA(device_alloc(&w->r, R * 8));
+  ESF_CUDA(device_alloc(&w->d, R * 8));
+  ESF_CUDA(device_alloc(&w->Ap, R * 8));
+  ESF_CUDA(device_alloc(&w->s, R * 8));
+  ESF_CUDA(device_alloc(&w->invd, R * 8));
   if (mixed) {
     w->mpitch = (g.X + 3) / 4 * 4;
     // (mapping eleven vectors takes 2 ms; below 2 MB, the granularity, a work
@@ -911,7 +911,7 @@ static esf_status work_buffers(PressureWork* w, const GridDev& g, int mixed) {
     const bool map = !w->perCall || R * 4 >= (2u << 20);
     auto vec = [&](float** v, size_t bytes) -> esf_status {
       if (map) return vec_alloc(&w->mapped, v, bytes);
-      ESF_CUDA(cudaMalloc(v, bytes));
+      ESF_CUDA(device_alloc(v, bytes));
       return ESF_OK;
     };
     float** vecs[] = {&w->x32, &w->r32, &w->d32, &w->Ap32, &w->s32, &w->invd32,
@@ -922,12 +922,12 @@ static esf_status work_buffers(PressureWork* w, const GridDev& g, int mixed) {
     }
     esf_status e = vec(&w->minv32p, (size_t)w->mpitch * g.Y * g.Z * 4);
     if (e) return e;
-    ESF_CUDA(cudaMalloc(&w->minv32, g.T * 4));
+    ESF_CUDA(device_alloc(&w->minv32, g.T * 4));
   }
-  ESF_CUDA(cudaMalloc(&w->partial, ESF_MAX_PARTIALS * 8));
-  ESF_CUDA(cudaMalloc(&w->st, sizeof(PcrState)));
-  ESF_CUDA(cudaMalloc(&w->st32, sizeof(PcrState)));
-  ESF_CUDA(cudaMalloc(&w->stT, sizeof(PcrState)));
+  ESF_CUDA(device_alloc(&w->partial, ESF_MAX_PARTIALS * 8));
+  ESF_CUDA(device_alloc(&w->st, sizeof(PcrState)));
+  ESF_CUDA(device_alloc(&w->st32, sizeof(PcrState)));
+  ESF_CUDA(device_alloc(&w->stT, sizeof(PcrState)));
   ESF_CUDA(cudaMemset(w->st, 0, sizeof(PcrState)));
   ESF_CUDA(cudaMemset(w->st32, 0, sizeof(PcrState)));
   ESF_CUDA(cudaMallocHost(&w->hst, 8 * sizeof(PcrState)));
@@ -1046,6 +1046,16 @@ bool pressure_work_release_idle(int device) {
   return n > 0;
 }
 
+cudaError_t device_alloc_bytes(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  int dev = 0;
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess && pressure_work_release_idle(dev)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 esf_status pressure_work_take(PressureWork** out, const GridDev& g, int mixed) {
   IdleWorks& P = idle_works();
   int dev = 0;
@@ -1065,10 +1075,6 @@ esf_status pressure_work_take(PressureWork** out, const GridDev& g, int mixed) {
     }
   }
   esf_status e = work_alloc(out, g, mixed, true);
-  if (e && pressure_work_release_idle(dev)) {
-    cudaGetLastError();
-    e = work_alloc(out, g, mixed, true);
-  }
   if (!e) {
     (*out)->device = dev;
     (*out)->ctx = known ? id : 0;  // 0: not kept
@@ -1578,9 +1584,9 @@ esf_status pressure_solve(PressureWork* w, const GridDev& g, const double* minv6
     constexpr long long kCopyCells = 1 << 21;
     const bool copies = w->perCall && g.R <= kCopyCells;
     if (copies) {
-      if (!w->m64) ESF_CUDA(cudaMalloc(&w->m64, g.T * 8));
-      if (!w->b64) ESF_CUDA(cudaMalloc(&w->b64, g.R * 8));
-      if (!w->x64) ESF_CUDA(cudaMalloc(&w->x64, g.R * 8));
+      if (!w->m64) ESF_CUDA(device_alloc(&w->m64, g.T * 8));
+      if (!w->b64) ESF_CUDA(device_alloc(&w->b64, g.R * 8));
+      if (!w->x64) ESF_CUDA(device_alloc(&w->x64, g.R * 8));
       ESF_CUDA(cudaMemcpyAsync(w->m64, minv64, g.T * 8, cudaMemcpyDeviceToDevice, st));
       ESF_CUDA(cudaMemcpyAsync(w->b64, b, g.R * 8, cudaMemcpyDeviceToDevice, st));
       ESF_CUDA(cudaMemcpyAsync(w->x64, x, g.R * 8, cudaMemcpyDeviceToDevice, st));
@@ -1939,8 +1945,8 @@ static esf_status time_kernels_t(PressureWork* w, const GridDev& g, const T* min
 // The double-float correction and direction of ESF_MIXED_X64 (8 bytes a
 // row each), allocated on first use.
 static esf_status df_buffers(PressureWork* w, const GridDev& g) {
-  if (!w->edf) ESF_CUDA(cudaMalloc(&w->edf, g.R * 8));
-  if (!w->ddf) ESF_CUDA(cudaMalloc(&w->ddf, g.R * 8));
+  if (!w->edf) ESF_CUDA(device_alloc(&w->edf, g.R * 8));
+  if (!w->ddf) ESF_CUDA(device_alloc(&w->ddf, g.R * 8));
   return ESF_OK;
 }
 
@@ -2020,7 +2026,7 @@ esf_status pressure_time_kernels(PressureWork* w, const GridDev& g, const double
   }
   // FP64: x scratch is w->s's neighbour; use the FP64 work arrays only
   double* xs = nullptr;
-  ESF_CUDA(cudaMalloc(&xs, g.R * 8));
+  ESF_CUDA(device_alloc(&xs, g.R * 8));
   esf_status e = time_kernels_t<double>(w, g, minv64, w->invd, b, xs, w->r, w->d, w->Ap, w->s, reps,
                                         update_ms, axpy_ms, st);
   cudaStreamSynchronize(st);
@@ -2290,15 +2296,15 @@ esf_status solid_work_alloc(SolidWork** out, long long S, int mixed) {
   w->S = S;
   w->cap = S > 0 ? S : 1;
   size_t n = 3 * w->cap;
-  ESF_CUDA(cudaMalloc(&w->r, n * 8));
-  ESF_CUDA(cudaMalloc(&w->d, n * 8));
-  ESF_CUDA(cudaMalloc(&w->Ap, n * 8));
-  ESF_CUDA(cudaMalloc(&w->s, n * 8));
-  ESF_CUDA(cudaMalloc(&w->invd, n * 8));
-  ESF_CUDA(cudaMalloc(&w->partial, ESF_MAX_PARTIALS * 8));
-  ESF_CUDA(cudaMalloc(&w->st, sizeof(PcrState)));
-  ESF_CUDA(cudaMalloc(&w->st32, sizeof(PcrState)));
-  ESF_CUDA(cudaMalloc(&w->bar, 2 * sizeof(unsigned)));
+  ESF_CUDA(device_alloc(&w->r, n * 8));
+  ESF_CUDA(device_alloc(&w->d, n * 8));
+  ESF_CUDA(device_alloc(&w->Ap, n * 8));
+  ESF_CUDA(device_alloc(&w->s, n * 8));
+  ESF_CUDA(device_alloc(&w->invd, n * 8));
+  ESF_CUDA(device_alloc(&w->partial, ESF_MAX_PARTIALS * 8));
+  ESF_CUDA(device_alloc(&w->st, sizeof(PcrState)));
+  ESF_CUDA(device_alloc(&w->st32, sizeof(PcrState)));
+  ESF_CUDA(device_alloc(&w->bar, 2 * sizeof(unsigned)));
   ESF_CUDA(cudaMallocHost(&w->hst, 4 * sizeof(PcrState)));
   for (int i = 0; i < 4; i++) ESF_CUDA(cudaEventCreateWithFlags(&w->ev[i], cudaEventDisableTiming));
   ESF_CUDA(cudaStreamCreateWithFlags(&w->capStream, cudaStreamNonBlocking));
@@ -2307,13 +2313,13 @@ esf_status solid_work_alloc(SolidWork** out, long long S, int mixed) {
     // solves per 256^3 step with cudaMalloc
     esf_status e = vec_alloc(&w->mapped, &w->blocks32, rows32(w->cap) * 243 * 4);
     if (e) return e;
-    ESF_CUDA(cudaMalloc(&w->x32, n * 4));
-    ESF_CUDA(cudaMalloc(&w->r32, n * 4));
-    ESF_CUDA(cudaMalloc(&w->d32, n * 4));
-    ESF_CUDA(cudaMalloc(&w->Ap32, n * 4));
-    ESF_CUDA(cudaMalloc(&w->s32, n * 4));
-    ESF_CUDA(cudaMalloc(&w->invd32, n * 4));
-    ESF_CUDA(cudaMalloc(&w->b32, n * 4));
+    ESF_CUDA(device_alloc(&w->x32, n * 4));
+    ESF_CUDA(device_alloc(&w->r32, n * 4));
+    ESF_CUDA(device_alloc(&w->d32, n * 4));
+    ESF_CUDA(device_alloc(&w->Ap32, n * 4));
+    ESF_CUDA(device_alloc(&w->s32, n * 4));
+    ESF_CUDA(device_alloc(&w->invd32, n * 4));
+    ESF_CUDA(device_alloc(&w->b32, n * 4));
   }
   *out = w;
   return ESF_OK;
@@ -2351,10 +2357,10 @@ esf_status solid_work_set_matrix_free(SolidWork* w, const GridDev& g, long long 
     cudaFree(w->mfShare);
     w->mfShare = nullptr;
     w->mfShareCap = 0;
-    ESF_CUDA(cudaMalloc(&w->mfShare, (size_t)24 * (nc + nc / 4 + 16) * 4));
+    ESF_CUDA(device_alloc(&w->mfShare, (size_t)24 * (nc + nc / 4 + 16) * 4));
     w->mfShareCap = nc + nc / 4 + 16;
   }
-  if (!w->damped32) ESF_CUDA(cudaMalloc(&w->damped32, (size_t)3 * w->cap * 4));
+  if (!w->damped32) ESF_CUDA(device_alloc(&w->damped32, (size_t)3 * w->cap * 4));
   w->mf.g = g;
   w->mf.nc = nc;
   w->mf.cell = cell;
@@ -2672,7 +2678,7 @@ struct InnerBatcher {
   esf_status init(int dev) {
     device = dev;
     cudaSetDevice(dev);
-    ESF_CUDA(cudaMalloc(&dTasks, sizeof(FusedTask) * kSlots));
+    ESF_CUDA(device_alloc(&dTasks, sizeof(FusedTask) * kSlots));
     ESF_CUDA(cudaMallocHost(&hTasks, sizeof(FusedTask) * kSlots));
     static const cudaError_t attr = cudaFuncSetAttribute(
         pcr_iteration_fused_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, FU_SMEM);
@@ -2691,7 +2697,7 @@ struct InnerBatcher {
       ESF_CUDA(cudaEventCreate(&L.t0[i]));
       ESF_CUDA(cudaEventCreate(&L.t1[i]));
     }
-    ESF_CUDA(cudaMalloc(&L.dStates, sizeof(PcrState) * kSlots * kRing));
+    ESF_CUDA(device_alloc(&L.dStates, sizeof(PcrState) * kSlots * kRing));
     ESF_CUDA(cudaMallocHost(&L.hStates, sizeof(PcrState) * kSlots * kRing));
     return ESF_OK;
   }

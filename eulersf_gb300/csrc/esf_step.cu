@@ -78,7 +78,7 @@ struct DBuf {
     p = nullptr;
     bytes = 0;
     size_t nb = b + b / 4 + 256;
-    cudaError_t e = cudaMalloc(&p, nb);
+    cudaError_t e = device_alloc(&p, nb);
     if (e != cudaSuccess) {
       set_error("cudaMalloc(%zu): %s", nb, cudaGetErrorString(e));
       return ESF_ERR_OOM;
@@ -221,12 +221,7 @@ esf_status esf_params_default(const esf_grid* g, esf_params* p) {
 }  // extern "C"
 
 static esf_status dalloc(void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes ? bytes : 8);
-  int dev = 0;
-  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess && pressure_work_release_idle(dev)) {
-    cudaGetLastError();
-    e = cudaMalloc(p, bytes ? bytes : 8);
-  }
+  cudaError_t e = device_alloc(p, bytes ? bytes : 8);
   if (e != cudaSuccess) {
     set_error("cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
     return ESF_ERR_OOM;
@@ -336,10 +331,6 @@ extern "C" esf_status esf_create(const esf_grid* g, const esf_params* p, void* s
     cudaMemsetAsync(s->rhs, 0, R * 8, s->stream);
     cudaMemsetAsync(s->b1, 0, R * 8, s->stream);
     e = pressure_work_alloc(&s->pw, G, p->precision != ESF_FP64);
-    if (e == ESF_ERR_OOM && pressure_work_release_idle(s->device)) {
-      cudaGetLastError();
-      e = pressure_work_alloc(&s->pw, G, p->precision != ESF_FP64);
-    }
   }
   if (!e && cudaEventCreate(&s->e0) != cudaSuccess) e = ESF_ERR_CUDA;
   if (!e && cudaEventCreate(&s->e1) != cudaSuccess) e = ESF_ERR_CUDA;
@@ -1908,7 +1899,7 @@ extern "C" esf_status esf_selftest_bounded_wait(int kind, int* gave_up, double* 
     return ESF_ERR_INVALID_ARG;
   }
   int* d = nullptr;
-  ESF_CUDA(cudaMalloc(&d, 16));
+  ESF_CUDA(device_alloc(&d, 16));
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   esf_status e = ESF_OK;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) e = ESF_ERR_CUDA;
