@@ -408,10 +408,15 @@ extern "C" esf_status esf_rasterize_solid(const double* vertices, int num_vertic
   unsigned char* scratch = nullptr;
   esf_status e = ESF_OK;
   if (device_alloc(&dTri, tri.size() * 4) != cudaSuccess || device_alloc(&dMass, total * 8) != cudaSuccess ||
-      device_alloc(&dCount, 8) != cudaSuccess ||
-      (cubes && device_alloc(&scratch, size.bytes + total) != cudaSuccess)) {
+      device_alloc(&dCount, 8) != cudaSuccess) {
     set_error("esf_rasterize_solid: device allocation failed");
     e = ESF_ERR_OOM;
+  }
+  // (no memory for the cubes: the kernel that needs none)
+  if (!e && cubes && device_alloc(&scratch, size.bytes + total) != cudaSuccess) {
+    cudaGetLastError();
+    scratch = nullptr;
+    cubes = false;
   }
   if (!e && (cudaMemcpy(dTri, tri.data(), tri.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
              cudaMemset(dCount, 0, 8) != cudaSuccess ||

@@ -135,3 +135,33 @@ def test_kept_workspaces_are_given_back(gpu_lib, tmp_path):
     for k, (_, refused) in out.items():
         if k.split()[0] in ("solve", "batch", "bake", "create") or k.endswith(" 0"):
             assert refused > 0, k
+
+
+_BAKE = textwrap.dedent("""
+    import ctypes as C, json, sys
+    sys.path[:0] = [{root!r}]
+    import numpy as np
+    import torch
+    import eulersf_gb300 as E
+    from eulersf_gb300 import abi
+    from eulersf_gb300.bake import rasterize_solid
+    from eulersf_gb300.scene import icosphere
+    shim = C.CDLL(None)
+    lib = E.load()
+    verts, faces = icosphere(3, 0.1)
+    grid = rasterize_solid(verts, faces, 0.1 / 40, 1000.0)
+    assert np.prod(grid[0]) * len(faces) >= 2e8  # by cubes
+    lib.esf_release_workspaces()
+    shim.esf_test_refuse_after(3)
+    try:
+        again = rasterize_solid(verts, faces, 0.1 / 40, 1000.0)
+        print(json.dumps([shim.esf_test_refused(), bool(np.array_equal(grid[3], again[3]) and grid[4] == again[4])]))
+    except abi.EsfError as e:
+        print(json.dumps([shim.esf_test_refused(), str(e)]))
+""")
+
+
+def test_baking_without_memory_for_cubes(gpu_lib, tmp_path):
+    """The cubes' lists refused, and nothing kept to give back: every node
+    against every triangle, the same masses."""
+    assert child(_BAKE, tmp_path) == [1, True]
