@@ -26,7 +26,7 @@ EXPORTS = [
     "esf_pressure_solve", "esf_pressure_solve_batch", "esf_pressure_solve_static", "esf_write_frame", "esf_read_frame", "esf_write_frame_async", "esf_frame_wait", "esf_kernel_launches",
     "esf_time_pressure_kernels", "esf_scene_footprint", "esf_server_create", "esf_server_submit",
     "esf_server_poll", "esf_server_wait", "esf_server_get_field", "esf_server_release",
-    "esf_server_destroy", "esf_server_batch_stats", "esf_selftest_bounded_wait", "esf_rasterize_solid",
+    "esf_server_destroy", "esf_server_batch_stats", "esf_selftest_bounded_wait", "esf_selftest_loop_wait", "esf_rasterize_solid",
     "esf_solid_load_rest_sdf", "esf_rest_sdf_query", "esf_svol_read", "esf_release_workspaces",
 ]
 

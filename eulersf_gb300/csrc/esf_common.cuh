@@ -106,6 +106,9 @@ struct PcrState {
   int setup;         // 1: next phase-B reduction initialises delta
   int status;        // 0 ok, 6 numeric (NaN met)
   int inner;         // 1: inner solve of a refinement, stops on delta/delta0
+  // loops of the one-pass iteration: a block gave up on a copy or on the others.
+  // Set by that block alone, left out where block 0 writes the rest
+  unsigned int failed;
   double delta0;     // delta after set-up or after the last residual replacement
   int rebase;        // 1: next update reduction replaces the residual (keeps d)
   int iter0;         // iteration of the last replacement
@@ -119,6 +122,7 @@ struct PcrState {
   unsigned int hx, hm, hv, hr, hq, lm;
   double limit;  // one-pass FP32 iteration: eps^2 delta0, below which it stops
 };
+static_assert(sizeof(PcrState) == 160, "five sectors: a pass's last block reads and writes it in its tail");
 
 // Solid system layout ("sliced"): the 27 neighbour 3x3 blocks of solid node a,
 // entry je = 9 j + e, live at ((a / 32) * 243 + je) * 32 + a % 32, and the
@@ -203,6 +207,8 @@ void batcher_stats(InnerBatcher* b, esf_batch_stats* out);
 esf_status pressure_work_set_batcher(PressureWork* w, InnerBatcher* b);
 // self-test of the TMA kernels' bounded mbarrier wait (esf_solver.cu)
 esf_status selftest_mbar_wait(int* gaveUp, cudaStream_t st);
+// ... and of a wait that runs out in the cooperative loops of the FP32 iteration
+esf_status selftest_loop_wait(bool x64, int maxIt);
 // allocation-free FP64 solve on the module's static scratch (esf_solver.cu)
 esf_status static_scratch_address(void** out);
 esf_status pressure_solve_static(void* scratch, const GridDev& g, const double* minv,

@@ -55,8 +55,8 @@ __device__ __forceinline__ bool flat_wait(PcrState* st, unsigned target) {
   do {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(&st->ticket[2]) : "memory");
     if ((++it & 1023u) == 0) {
-      bad = *(volatile unsigned*)&st->ticket[3];
-      if (it >= FU_LOOP_WAIT) bad = *(volatile unsigned*)&st->ticket[3] = 1;
+      bad = *(volatile unsigned*)&st->failed;
+      if (it >= FU_LOOP_WAIT) bad = *(volatile unsigned*)&st->failed = 1;
     }
   } while ((int)(cur - target) < 0 && !bad);
   return !bad;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
 
   if (threadIdx.x == 0) L = *st;
   __syncthreads();
-  if (L.done) return;
+  if (L.done || L.failed) return;
   const unsigned base = L.ticket[0];
   auto fetch = [&](int set) {  // by one thread
     asm volatile("fence.proxy.async;" ::: "memory");  // (what the blocks wrote before the barrier)
@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
   const int aN = cx + w * TW_NP;
 
   int pass = 0;
+  bool failed = false;  // (the same in all threads)
   for (;; pass++) {
     const bool stop = pass == budget || L.done || L.iter >= L.maxIt;  // the same in every block
     ok = mbar_wait(&bar[0], pass & 1) && ok;
@@ -207,7 +208,8 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
     if (grp < layers) layer_in(grp + 1, own, true, true);
     // the layers around: tile and ring to a group each
     layer_in(grp < 2 ? 0 : layers + 1, false, grp & 1, !(grp & 1));
-    if (__syncthreads_or(!ok)) break;
+    failed = __syncthreads_or(!ok);
+    if (failed) break;
 
     // (b) J^T r' scaled by m^-1 on the node layers below and above the own layer
     if (grp < layers) {
@@ -357,11 +359,13 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
         go = flat_wait(st, target);  // (one poller: four in each block were slower)
       }
       flat_sync4();
-      const double total =
-          flat_tree([&](int a, int i) { return a * 32 + i < nb ? __ldcg(part + a * 32 + i) : 0.0; });
-      if (lane == 0) sT[h] = total;
-      flat_sync4();
-      if (threadIdx.x == 0) finish_fused(&L, sT[0], sT[1], sT[2], sT[3]);
+      if (go) {  // (all sums are there)
+        const double total =
+            flat_tree([&](int a, int i) { return a * 32 + i < nb ? __ldcg(part + a * 32 + i) : 0.0; });
+        if (lane == 0) sT[h] = total;
+        flat_sync4();
+        if (threadIdx.x == 0) finish_fused(&L, sT[0], sT[1], sT[2], sT[3]);
+      }
     } else if (threadIdx.x == 128) {
       arrived = flat_wait(st, target);
       if (arrived) fetch(pout);
@@ -369,17 +373,14 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
     __syncthreads();
     if (!go || !arrived) {
       if (arrived) mbar_wait(&bar[0], (pass + 1) & 1);
+      failed = true;
       break;
     }
   }
-  // a block that gave up on a copy or on the others: an error, and they give up too
-  const bool stopped = pass == budget || L.done || L.iter >= L.maxIt;
-  if (!stopped || __syncthreads_or(!ok)) {
-    if (threadIdx.x == 0) {
-      *(volatile unsigned*)&st->ticket[3] = 1;
-      st->status = ESF_ERR_CUDA;
-      st->done = 1;
-    }
+  // a block that gave up on a copy or on the others has no x and d to store: the
+  // solve has failed, whatever the others' sums say, and they give up too
+  if (__syncthreads_or(failed || !ok)) {
+    if (threadIdx.x == 0) *(volatile unsigned*)&st->failed = 1;
     return;
   }
   if (own) {
@@ -394,6 +395,8 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
   if (bid == 0 && threadIdx.x == 0) {
     if (L.iter >= L.maxIt) L.done = 1;
     L.ticket[0] = L.ticket[2] = base + (unsigned)pass * nb;
-    *st = L;
+    for (unsigned k = 0; k < sizeof(PcrState) / 4; k++)
+      if (k != offsetof(PcrState, failed) / 4)
+        reinterpret_cast<unsigned*>(st)[k] = reinterpret_cast<const unsigned*>(&L)[k];
   }
 }

@@ -1273,7 +1273,12 @@ static esf_status prepare_tma(PressureWork* w, const GridDev& g, const double* m
     w->fmaps = m;
     w->fusedOk = true;
   }
-  if (!w->flatOk && loop_fits(g)) {
+  const bool loops = loop_fits(g);
+  if (loops) {
+    esf_status e = allow_loops();
+    if (e) return e;
+  }
+  if (!w->flatOk && loops) {
     FlatMaps m;
     esf_status e;
     float* rs[2] = {w->r32, w->r32b};
@@ -1485,7 +1490,7 @@ static esf_status run_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst, int m
       ESF_CUDA(cudaEventSynchronize(ev[waited % 4]));
       PcrState h = hst[waited % 4];
       waited++;
-      if (h.done) {
+      if (h.done || h.failed) {
         done = true;
         *out = h;
       } else if (waited >= maxChunks) {
@@ -1515,9 +1520,10 @@ static esf_status run_graph_solve(PcrState* hst, cudaEvent_t* ev, PcrState* dst,
 static esf_status run_fused(PressureWork* w, const FusedKernels& k, cudaGraphExec_t graph, unsigned long long kernels,
                             int maxIt, cudaStream_t st, PcrState* out) {
   if (!k.loops()) return run_graph_solve(w->hst, w->ev, k.st, nullptr, graph, 0, kernels, maxIt, st, out);
-  esf_status e = allow_loops();
-  if (e) return e;
-  return run_solve(w->hst, w->ev, k.st, maxIt, st, out, [&](bool) { return k.loop(st, FL_CHUNK); }, FL_CHUNK);
+  esf_status e = run_solve(w->hst, w->ev, k.st, maxIt, st, out, [&](bool) { return k.loop(st, FL_CHUNK); }, FL_CHUNK);
+  if (e || !out->failed) return e;
+  set_error("pressure solve: a wait of the iteration's blocks for a copy or for one another ran out");
+  return ESF_ERR_CUDA;
 }
 
 static esf_status init_state(PcrState* d, double eps, int maxIt, cudaStream_t st, int inner = 0) {
@@ -3086,6 +3092,60 @@ esf_status selftest_mbar_wait(int* gaveUp, cudaStream_t st) {
   ESF_COUNTED k_selftest_mbar_wait<<<1, 32, 0, st>>>(gaveUp);
   ESF_LAUNCH_CHECK();
   return ESF_OK;
+}
+
+// A loop of the one-pass iteration on a grid of zeros whose blocks wait for more
+// arrivals than there are blocks: the first pass's wait runs out.
+esf_status selftest_loop_wait(bool x64, int maxIt) {
+  GridDev g;
+  memset(&g, 0, sizeof g);
+  g.X = g.Y = g.Z = 33;
+  g.cX = g.cY = g.cZ = 32;
+  g.slab = 33 * 33;
+  g.T = 33 * 33 * 33;
+  g.cslab = 32 * 32;
+  g.R = 32 * 32 * 32;
+  PressureWork* w = nullptr;
+  esf_status e = work_alloc(&w, g, 1, true);
+  if (e) return e;
+  auto run = [&]() -> esf_status {
+    const TmaMaps* tma = nullptr;
+    int path = P32_REGISTER;
+    esf_status s = prepare_tma(w, g, nullptr, w->capStream, &tma, &path);
+    if (!s && x64) s = df_buffers(w, g);
+    if (s) return s;
+    FusedKernels k = fused_kernels(w, g, w->st32);
+    if (x64) {
+      k.edf = w->edf;
+      k.ddf = w->ddf;
+    }
+    if (path != P32_FUSED || !k.loops()) {
+      set_error("esf_selftest_loop_wait: no loops on this device");
+      return ESF_ERR_UNSUPPORTED;
+    }
+    for (float* v : {w->x32, w->r32, w->d32, w->Ap32, w->s32, w->invd32, w->b32, w->r32b, w->s32b, w->Ap32b})
+      ESF_CUDA(cudaMemsetAsync(v, 0, g.R * 4, w->capStream));
+    ESF_CUDA(cudaMemsetAsync(w->minv32p, 0, (size_t)w->mpitch * g.Y * g.Z * 4, w->capStream));
+    for (float* v : {w->edf, w->ddf})
+      if (v) ESF_CUDA(cudaMemsetAsync(v, 0, g.R * 8, w->capStream));
+    PcrState h, out;
+    memset(&h, 0, sizeof h);
+    h.maxIt = maxIt;
+    h.setup = 1;
+    h.inner = 1;
+    h.ticket[0] = 1;  // arrivals before the first pass, of which there were none
+    ESF_COUNTED put_state<<<1, 1, 0, w->capStream>>>(w->st32, h);
+    ESF_LAUNCH_CHECK();
+    return run_fused(w, k, nullptr, 0, maxIt, w->capStream, &out);
+  };
+  e = run();
+  const cudaError_t idle = cudaStreamSynchronize(w->capStream);
+  pressure_work_free(w);
+  if (idle != cudaSuccess) {
+    set_error("esf_selftest_loop_wait: %s", cudaGetErrorString(idle));
+    return ESF_ERR_STATE;
+  }
+  return e;
 }
 
 // ------------------------------------ allocation-free FP64 pressure solve

@@ -1927,6 +1927,14 @@ extern "C" esf_status esf_selftest_bounded_wait(int kind, int* gave_up, double* 
   return e;
 }
 
+extern "C" esf_status esf_selftest_loop_wait(int precision, int max_iterations) {
+  if ((precision != ESF_MIXED && precision != ESF_MIXED_X64) || max_iterations < 1) {
+    set_error("esf_selftest_loop_wait: precision must be ESF_MIXED or ESF_MIXED_X64, max_iterations positive");
+    return ESF_ERR_INVALID_ARG;
+  }
+  return selftest_loop_wait(precision == ESF_MIXED_X64, max_iterations);
+}
+
 // COUPLED_INTEGRATOR_3D::writeFrame (COUPLED_INTEGRATOR_3D.cpp:997-1012) with
 // DEFOR_SOLID_3D::writeFrame (DEFOR_SOLID_3D.cpp:1362-1370): per solid i
 // "frame.NNNN.solid.i" + .displacement/.velocity/.phi (every 10th frame or

@@ -343,6 +343,14 @@ esf_status esf_pressure_solve_static(const esf_grid* grid, const double* mass_in
  * NULL) is the kernel's device time. The context stays usable afterwards. */
 esf_status esf_selftest_bounded_wait(int kind, int* gave_up, double* elapsed_ms);
 
+/* Self-test of a solve whose blocks wait for one another and for more arrivals
+ * than there are blocks: an FP32 iteration in cooperative loops (ESF_MIXED or
+ * ESF_MIXED_X64) of at most max_iterations on a grid of zeros. The wait runs out
+ * after a second or two, and the call returns what a solve returns then,
+ * ESF_ERR_CUDA with a message (ESF_ERR_UNSUPPORTED on a device without such
+ * loops). The context stays usable. */
+esf_status esf_selftest_loop_wait(int precision, int max_iterations);
+
 /* Offline mass baking (projects/rasterizeSolid/main.cpp:20-80, the
  * reference's rasterizeSolid tool) on the GPU: the rest-pose mass grid of a
  * solid from its closed triangle mesh (num_vertices x 3 doubles,
