@@ -196,7 +196,7 @@ extern "C" size_t esf_scene_footprint(const esf_grid* g, const esf_params* p, in
   const double R = (double)(g->xRes - 1) * (g->yRes - 1) * (g->zRes - 1);
   // integrator and per-solid node fields, pressure vectors (FP64 + FP32);
   // coefficients fitted to scenes measured on GB300 at 48^3, 96^3 and 160^3
-  // (estimate / measured = 1.07, 1.00, 0.99 for a 0.2-radius ball), plus
+  // (estimate / measured = 1.07, 1.01, 1.00 for a 0.2-radius ball, mixed), plus
   // the one-pass FP32 iteration's second set of r, t, q (12 bytes a row)
   double bytes = T * (520.0 + 240.0 * ns) + R * 192.0;
   // ESF_MIXED_X64: the double-float correction and direction (8 bytes each a row)
@@ -215,11 +215,20 @@ extern "C" size_t esf_scene_footprint(const esf_grid* g, const esf_params* p, in
         lo[q] = std::min(lo[q], c);
         hi[q] = std::max(hi[q], c);
       }
-    double cells = 1.0;
-    for (int q = 0; q < 3; q++) cells *= std::max(0.0, (hi[q] - lo[q]) / g->dh + 2.0);
+    double cells = 1.0, box = 1.0;  // box: the sweeps', with the extrapolated cells
+    const int res[3] = {g->xRes, g->yRes, g->zRes};
+    for (int q = 0; q < 3; q++) {
+      const double n = std::max(0.0, (hi[q] - lo[q]) / g->dh + 2.0);
+      cells *= n;
+      box *= std::min(n + 2.0 * std::max(0, p->extrapolation_cells), (double)res[q]);
+    }
     const double solidNodes = 0.55 * cells;  // sphere / box volume, plus a margin
-    // (a particle: its state, and 96 bytes more in its P2G record than the fit had)
-    bytes += solidNodes * (27 * 9 * 8 * 1.5 + 27 * 4 + 400) + solidNodes * p->particles_per_cell * 160.0;
+    const double np = solidNodes * p->particles_per_cell;
+    bytes += solidNodes * (27 * 9 * 8 * 1.5 + 27 * 4 + 400) + np * 80.0;
+    // since that fit: particle records of 192 bytes for weights of 96, in one buffer
+    // with the velocity extension's weights (128 bytes a node of the box), and its
+    // level lists (an entry of 32 bytes to a node); buffers have a quarter to spare
+    bytes += 1.25 * (std::max(192.0 * np, 128.0 * box) - 96.0 * np + 32.0 * box);
   }
   return (size_t)(bytes * 1.1) + (140u << 20);
 }
