@@ -205,6 +205,10 @@ esf_status batcher_create(int device, InnerBatcher** out, bool autotune);
 void batcher_destroy(InnerBatcher* b);
 void batcher_stats(InnerBatcher* b, esf_batch_stats* out);
 esf_status pressure_work_set_batcher(PressureWork* w, InnerBatcher* b);
+// a scene or system of this grid shape (cells) is under way, and no longer: inner
+// solves are batched while there are two
+void batcher_join(InnerBatcher* b, int cX, int cY, int cZ);
+void batcher_leave(InnerBatcher* b, int cX, int cY, int cZ);
 // self-test of the TMA kernels' bounded mbarrier wait (esf_solver.cu)
 esf_status selftest_mbar_wait(int* gaveUp, cudaStream_t st);
 // ... and of a wait that runs out in the cooperative loops of the FP32 iteration

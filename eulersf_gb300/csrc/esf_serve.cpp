@@ -33,6 +33,8 @@ esf_status batcher_create(int device, InnerBatcher** out, bool autotune);
 void batcher_destroy(InnerBatcher* b);
 void batcher_stats(InnerBatcher* b, esf_batch_stats* out);
 esf_status scene_set_batcher(esf_scene* s, InnerBatcher* b);
+void batcher_join(InnerBatcher* b, int cX, int cY, int cZ);
+void batcher_leave(InnerBatcher* b, int cX, int cY, int cZ);
 }
 
 namespace {
@@ -171,7 +173,11 @@ struct esf_server {
         r->st.state = ESF_REQ_RUNNING;
         r->st.queued_ms = ms_since(r->submitted, Clock::now());
       }
+      const bool joins = batcher && r->params.precision == ESF_MIXED;
+      const esf_grid& g = r->grid;
+      if (joins) esf::batcher_join(batcher, g.xRes - 1, g.yRes - 1, g.zRes - 1);
       const esf_status e = run(r);
+      if (joins) esf::batcher_leave(batcher, g.xRes - 1, g.yRes - 1, g.zRes - 1);
       {
         std::lock_guard<std::mutex> g(m);
         active--;

@@ -2666,8 +2666,7 @@ struct InnerBatcher {
   bool slotUsed[kSlots] = {};
   int slotRefs[kSlots] = {};
   std::map<Shape, Lane> lanes;
-  std::map<std::array<int, 3>, int> attached;  // works attached, by grid shape (cells per axis)
-  std::map<std::array<int, 3>, std::chrono::steady_clock::time_point> left;  // when one was last detached
+  std::map<std::array<int, 3>, int> running;  // scenes or systems under way, by grid shape (cells per axis)
   std::mutex m;
   std::condition_variable cv, doneCv;
   std::deque<Job*> pending;
@@ -2997,29 +2996,29 @@ esf_status pressure_work_set_batcher(PressureWork* w, InnerBatcher* b) {
     ESF_CUDA(cudaEventCreateWithFlags(&w->batchReady, cudaEventDisableTiming));
     ESF_CUDA(cudaEventCreateWithFlags(&w->batchDone, cudaEventDisableTiming));
   }
-  const std::array<int, 3> shape = {w->g.cX, w->g.cY, w->g.cZ};
-  if (w->batcher) {
-    std::lock_guard<std::mutex> g(w->batcher->m);
-    w->batcher->attached[shape]--;
-    w->batcher->left[shape] = std::chrono::steady_clock::now();
-  }
   w->batcher = b;
-  if (b) {
-    std::lock_guard<std::mutex> g(b->m);
-    b->attached[shape]++;
-  }
   return ESF_OK;
+}
+void batcher_join(InnerBatcher* b, int cX, int cY, int cZ) {
+  std::lock_guard<std::mutex> g(b->m);
+  b->running[{cX, cY, cZ}]++;
+}
+void batcher_leave(InnerBatcher* b, int cX, int cY, int cZ) {
+  std::lock_guard<std::mutex> g(b->m);
+  auto it = b->running.find({cX, cY, cZ});
+  if (it != b->running.end() && --it->second == 0) b->running.erase(it);
 }
 // Whether a scene's inner solves go through its batcher: only for a grid
 // whose own pass fills at most a quarter of the GPU's resident blocks (a
 // larger one already keeps the GPU busy alone, and the batcher's
 // one-launch-at-a-time host loop and its kernel's spills only cost; measured
 // on the 48^3-160^3 serving mix: 6.9 scene-steps/s batching every shape
-// against 7.6 unbatched), and only while another work of the same grid shape
-// is attached (a task alone in its lane gains nothing over the scene's own
-// launches) or was within the last second: requests of a shape come one after
-// another, and a scene that is through between two others is not a reason to
-// leave the lane.
+// against 7.6 unbatched), and only while another scene or system of the same grid
+// shape is under way, from before it is built to its last step: a task alone in
+// its lane takes twice as long as by the scene's own loops. (Batched for a second
+// more after a scene had left, the next one alone took 255 ms for 141 at 64^3 and
+// 80 for 48 at 32^3, and the serving benchmark 6.75 scene-steps/s for 6.81, 61.1
+// for 62.4 with scenes of 32^3 and 48^3.)
 static bool batching_pays(PressureWork* w) {
   if (!w->batcher) return false;
   static const int slots = [] {
@@ -3035,11 +3034,8 @@ static bool batching_pays(PressureWork* w) {
   const dim3 gr = tma_grid(w->g, fused_cz(w->g));
   if ((long long)gr.x * gr.y * gr.z * 4 > slots) return false;
   std::lock_guard<std::mutex> g(w->batcher->m);
-  const std::array<int, 3> shape = {w->g.cX, w->g.cY, w->g.cZ};
-  auto it = w->batcher->attached.find(shape);
-  if (it != w->batcher->attached.end() && it->second >= 2) return true;
-  auto gone = w->batcher->left.find(shape);
-  return gone != w->batcher->left.end() && std::chrono::steady_clock::now() - gone->second < std::chrono::seconds(1);
+  auto it = w->batcher->running.find({w->g.cX, w->g.cY, w->g.cZ});
+  return it != w->batcher->running.end() && it->second >= 2;
 }
 
 // One inner solve of a scene through the batcher: the set-up pass has been

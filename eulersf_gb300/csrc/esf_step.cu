@@ -1826,6 +1826,7 @@ extern "C" esf_status esf_pressure_solve_batch(int n, const esf_grid* grids, con
       e = ESF_ERR_CUDA;
     }
     if (!e && batcher) e = pressure_work_set_batcher(works[i], batcher);
+    if (!e && batcher) batcher_join(batcher, grids[i].xRes - 1, grids[i].yRes - 1, grids[i].zRes - 1);
   }
   if (!e) {
     // one host thread per system drives its FP64 refinement loop on its own
