@@ -351,12 +351,9 @@ static long long persist_rows() {
 
 template <typename T>
 static esf_status solid_pcr_persist(SolidPersist<T> p, bool mf, PcrState* hst, cudaStream_t st, PcrState* out) {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-  }();
+  int dev = 0, sms = 0;
+  ESF_CUDA(cudaGetDevice(&dev));
+  ESF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const void* kernel = (const void*)solid_pcr_persistent<T, false>;
   if constexpr (std::is_same<T, float>::value)
     if (mf) kernel = (const void*)solid_pcr_persistent<float, true>;
