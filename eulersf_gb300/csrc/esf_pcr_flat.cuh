@@ -354,18 +354,18 @@ __global__ void __launch_bounds__(FL_G* NT, 1)
       const double ps = flat_tree([&](int a, int i) { return widen(mine[a * 33 + i]); });
       if (lane == 0) __stcg(part + bid, ps);
       flat_sync4();
+      bool here = false;  // thread 0's: all sums are there
       if (threadIdx.x == 0) {
         asm volatile("red.add.release.gpu.global.u32 [%0], 1;" ::"l"(&st->ticket[2]) : "memory");
-        go = flat_wait(st, target);  // (one poller: four in each block were slower)
+        here = flat_wait(st, target);  // (one poller: four in each block were slower)
+        go = here;
       }
       flat_sync4();
-      if (go) {  // (all sums are there)
-        const double total =
-            flat_tree([&](int a, int i) { return a * 32 + i < nb ? __ldcg(part + a * 32 + i) : 0.0; });
-        if (lane == 0) sT[h] = total;
-        flat_sync4();
-        if (threadIdx.x == 0) finish_fused(&L, sT[0], sT[1], sT[2], sT[3]);
-      }
+      const double total =
+          flat_tree([&](int a, int i) { return a * 32 + i < nb ? __ldcg(part + a * 32 + i) : 0.0; });
+      if (lane == 0) sT[h] = total;
+      flat_sync4();
+      if (threadIdx.x == 0 && here) finish_fused(&L, sT[0], sT[1], sT[2], sT[3]);  // (not of sums that may be missing)
     } else if (threadIdx.x == 128) {
       arrived = flat_wait(st, target);
       if (arrived) fetch(pout);
