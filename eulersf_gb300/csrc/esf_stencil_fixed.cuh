@@ -16,12 +16,12 @@
 //   cell:      (A + C - B) + (C - A - B)' of the lower node row plus
 //              (A + C + B) + (C - A + B)' of the upper (' of the column before)
 //
-// Bound: instruction issue (192^3 UPDATE: 127 M warp instructions, half a one a
-// cycle and scheduler, its three warps waiting on their own chains; DRAM at a
-// third). Measured against pressure_stencil<double>, whose bound is the FP64
-// pipe: product 32^3 19.1 -> 8.2 us, 64^3 29.5 -> 18.9, 128^3 159 -> 64,
-// 161x127x190 343 -> 106, 256^3 1154 -> 400; solve iteration (phase A included)
-// 34.7 -> 19, 57.8 -> 35, 260 -> 121, 499 -> 207, 1749 -> 733 us. Error of a
+// Bound: instruction issue (161x127x190 UPDATE: 89 M warp instructions, 0.61 a
+// cycle and scheduler, its three or four warps waiting on their own chains; DRAM
+// at a fifth). Measured against pressure_stencil<double>, whose bound is the FP64
+// pipe: product 32^3 18.6 -> 8.5 us, 64^3 28.8 -> 18.7, 128^3 158 -> 66,
+// 161x127x190 343 -> 109, 256^3 1154 -> 404; solve iteration (phase A included)
+// 33 -> 20, 53 -> 36, 254 -> 125, 499 -> 207, 1748 -> 755 us. Error of a
 // product against extended precision 4.7e-17 of the norm, the rounding of the
 // result; a plain FP64 evaluation has 1.7e-16.
 #pragma once
@@ -476,8 +476,9 @@ __global__ void __launch_bounds__(256) fixed_bounds(GridDev g, const double* x, 
 // cycle (cost of a layer 4.5, 4.7, 6 and 7.5); more blocks run in waves. Products
 // take two rows a warp or four (1.65 times the instructions of two), solves two:
 // with four an iteration took 65 us for 61 at 96^3, 212 for 201 at 161x127x190,
-// 745 for 733 at 256^3. Against fixed numbers of warps by size, an iteration takes
-// 41 for 53 us at 80^3, 121 for 130 at 128^3, 44 for 63 at 32x33x300; 64^3 the same.
+// 745 for 733 at 256^3. Against fixed numbers of warps by size, an iteration took
+// 41 for 53 us at 80^3, 121 for 130 at 128^3, 44 for 63 at 32x33x300; 64^3 the same
+// (these before the watch for cells that lose bits, which costs each 3 %).
 struct FixedShape {
   int ry, cz;
   dim3 grid;
@@ -530,8 +531,10 @@ static void launch_fixed(const GridDev& g, const StencilArgs<double>& a, const F
   launch_fixed_rows<MODE, 2>(g, a, s, st);
 }
 // Whether a grid's FP64 products and solves use it. It is the faster one at
-// every size and shape measured: 8^3 8.1 against 19.2 us a product, 20 against
-// 34 a solve iteration; 3x200x200 cells 9.5 and 19; 32x33x300 37 and 41. Below
+// every size and shape measured, a product and a solve iteration in us: 8^3 7.5
+// and 17 against 18.1 and 31, 20^3 7.5 and 19 against 18.6 and 33; 3x200x200 cells
+// (x y z) 37 and 60 against 107 and 156, 200x3x200 17 and 32 against 35 and 61,
+// 200x200x3 14 and 28 against 23 and 42; 32x33x300 29 and 45 against 41 and 83. Below
 // 8192 cells, where a step is its launches, FP64 in pressure_stencil's order
 // stays, whose results to the last bit whole steps on such grids are compared
 // by. More blocks than the sums have room for stay too.

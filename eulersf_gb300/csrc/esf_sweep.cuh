@@ -372,11 +372,12 @@ __global__ void __launch_bounds__(KT) k_sweep_vec_scan(SweepLists L) {
 // octant's (b, c) columns (one plane for even levels, one for odd). Entries
 // are loaded two levels ahead and a copy's value one, so the chain of a level
 // is three shared-memory reads, the blend and the barrier.
-// What bounds it is the FP64 pipe of one SM (three instructions an entry at
-// two lanes a cycle) and that chain, about 0.3 us a level: so entries are
-// packed: one thread to a column, idle lanes included, took 134 us a pass
-// against 118 us for lists read through L2 and 85 us here, at 64^3. Measured a
-// step: tile launches 9.8 ms at 64^3 and 13.2 at 128^3, this 2.7 and 5.6.
+// What bounds it is the FP64 pipe of one SM (five instructions an entry, three
+// products and two sums, at two lanes a cycle) and that chain, about 0.3 us a
+// level: so entries are packed: one thread to a column, idle lanes included, took
+// 134 us a pass against 118 us for lists read through L2 and 85 us here, at 64^3.
+// Measured a step: tiles over the whole box 9.8 ms at 64^3 and 13.2 at 128^3, over
+// the octant 7.0 and 9.6, this 2.7 and 5.6; larger octants: extend_velocity.
 constexpr int EXTEND_THREADS = 1024;
 __global__ void __launch_bounds__(EXTEND_THREADS) k_extend_field(GridDev g, double* f, const double* ms, Box ex,
                                                                  const Sweep8 all, const int* __restrict__ dims,
